@@ -47,7 +47,7 @@ struct FftDesc {
 struct GeomHost {
   int npairs = 0, nphmax = 0, nmax_complex = 0;
   int P = 2;                          // largest Bluestein convolution length (>= 2)
-  int synth_tile = 256;
+  int synth_tile = 256;               // ring pairs per CTA of the FP64 synthesis
   std::vector<int> order, count_m, mlim_sorted;
   std::vector<int2> synth_items, mixed_items;
   std::vector<double> cth, sth, phi0, weight;
@@ -198,6 +198,9 @@ void launch_mixed_anal(const JobDesc &job, const GeomPlan &gp, CoefPlan &cp,
                        cudaStream_t st);
 
 // Kernel launchers (sht_legendre.cu)
+// Ring pairs up to which the spin analysis takes two transforms per pass (above,
+// four rings per thread leave no registers for a second one).
+constexpr int kAnalWidePairs = 512;
 void launch_coef_tables(CoefPlan &cp, cudaStream_t st);
 void launch_legendre_synth(const JobDesc &job, const GeomPlan &gp, const CoefPlan &cp,
                            const double2 *A, int ncA, int comp0, int nt,
@@ -239,9 +242,11 @@ void launch_phase2ring_direct(const JobDesc &job, const GeomPlan &gp, long long 
 void launch_ring2phase_direct(const JobDesc &job, const GeomPlan &gp, long long map_lo,
                               const void *const *maps_dev, int nmapptr, double2 *phase,
                               int ncm, cudaStream_t st);
+// pm: pairs of components (G, C) are stored as (G - iC, G + iC), the basis of
+// the FP64 spin synthesis.
 void launch_stage_alm(const JobDesc &job, const AlmPlan &ap, long long alm_lo,
                       const CoefPlan &cp, const double *norm_l, const void *const *alm_dev,
-                      int nalmptr, double2 *A, int ncA, cudaStream_t st);
+                      int nalmptr, double2 *A, int ncA, bool pm, cudaStream_t st);
 void launch_scatter_alm(const JobDesc &job, const AlmPlan &ap, long long alm_lo,
                         const CoefPlan &cp, const double *norm_l, const double *Aout, int ncA,
                         void *const *alm_dev, int nalmptr, cudaStream_t st);

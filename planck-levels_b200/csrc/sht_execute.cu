@@ -165,6 +165,12 @@ bool ws_bytes(unsigned long long *reserved, unsigned long long *used) {
 GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin) {
   GeomHost h;
   const int np = g->npairs;
+  // FP64 synthesis: ring pairs per CTA of 128 threads.  Few pairs: one ring per
+  // thread, so that more warps share the work (Nside 64, 128, 256: 6.7, 12.8,
+  // 37.4 us at spin 0 and 10.8, 25.0, 92.7 at spin 2, against 8.6, 14.6, 41.3
+  // and 15.8, 28.8, 98.7 with two); many: two, which share the staged a_lm
+  // (Nside 512: 190 and 531 us against 204 and 556)
+  h.synth_tile = np <= 512 ? 128 : 256;
   h.npairs = np;
   h.nphmax = g->nphmax;
   std::vector<int> mlim(np);
@@ -864,10 +870,11 @@ void execute_impl(sharp_jobtype type_in, int spin, void *alm, void *map,
 
   if (!analysis) {
     DevBuf d_A(sizeof(double2) * size_t(cp->total) * ncA, st);
+    const bool mixed = (flags & SHARP_MIXED) && mixed_synth_supported(job);
     launch_stage_alm(job, *ap, alm_lo, *cp, d_norm.as<double>(),
                      reinterpret_cast<void *const *>(d_almptr.p), nalmptr, d_A.as<double2>(), ncA,
-                     st);
-    if ((flags & SHARP_MIXED) && mixed_synth_supported(job)) {
+                     spin > 0 && !deriv && !mixed, st);
+    if (mixed) {
       int *d_err = nullptr;
       tc_error_word(&d_err);
       launch_mixed_synth(job, *gp, *cp, d_A.as<double2>(), ncA, phase, ncm, d_err, st);
@@ -906,8 +913,8 @@ void execute_impl(sharp_jobtype type_in, int spin, void *alm, void *map,
       launch_ring2phase(job, *gp, map_lo, reinterpret_cast<const void *const *>(d_mapptr.p),
                         nmapptr, phase, ncm, st);
     DevBuf d_Aout(sizeof(double2) * size_t(cp->total) * ncA, st);
-    SHT_CUDA(cudaMemsetAsync(d_Aout.p, 0, sizeof(double2) * size_t(cp->total) * ncA, st));
     if ((flags & SHARP_MIXED) && mixed_anal_supported(job)) {
+      SHT_CUDA(cudaMemsetAsync(d_Aout.p, 0, sizeof(double2) * size_t(cp->total) * ncA, st));
       int *d_err = nullptr;
       tc_error_word(&d_err);
       launch_mixed_anal(job, *gp, *cp, phase, ncm, d_Aout.as<double2>(), ncA, d_err, st);
@@ -921,14 +928,11 @@ void execute_impl(sharp_jobtype type_in, int spin, void *alm, void *map,
         }
       };
       int width = ntmax_anal;
-      if (ntrans >= 2 && tuner_on(flags, st)) {
-        // analysis passes accumulate into Aout: cleared again after the timing runs
-        auto clear = [&] {
-          SHT_CUDA(cudaMemsetAsync(d_Aout.p, 0, sizeof(double2) * size_t(cp->total) * ncA, st));
-        };
-        width = tuned_width(TuneKey{gp->hash, job.lmax, mmax, spin, type, ntrans, 1},
-                            spin == 0 ? 4 : 2, ntmax_anal, passes, clear, st);
-      }
+      const int wmax = spin == 0 ? 4 : gp->npairs <= kAnalWidePairs ? 2 : 1;
+      if (ntrans >= 2 && wmax > 1 && tuner_on(flags, st))
+        // analysis passes overwrite Aout likewise
+        width = tuned_width(TuneKey{gp->hash, job.lmax, mmax, spin, type, ntrans, 1}, wmax,
+                            ntmax_anal, passes, [] {}, st);
       passes(width);
     }
     launch_scatter_alm(job, *ap, alm_lo, *cp, d_norm.as<double>(), d_Aout.as<double>(), ncA,

@@ -16,12 +16,21 @@
 //    the recurrence value is below 2^-kSwitchExp it runs scaled (exponent
 //    renormalised once per l-block, nothing accumulated), then switches to
 //    plain IEEE values.  Skipped terms are < 2^-88 of the leading ones;
-//  * analysis reduces over rings with a warp transpose-reduction and a fixed
-//    cross-warp order: no atomics, bitwise repeatable results.
+//  * analysis reduces over rings through shared memory within a warp and in a
+//    fixed order across warps: no atomics, bitwise repeatable results.
+//
+// What bounds it: the FP64 pipe, and in it the register ports.  A DFMA with
+// three distinct register operands issues every 3 cycles per sub-partition, 2/3
+// of the rate of one that repeats an operand of its predecessor or of a DADD
+// (measured on register-only loops: 42.7, 56.9 and 64 lane operations per cycle
+// and SM).  Per l and 32 ring pairs the loops run 4 (spin 0) or 12 (spin s)
+// such operations; everything else (staging, reduction, tests on the scaled
+// regime) is kept out of them.
 #include <cuda_pipeline.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "sht_device.h"
@@ -31,20 +40,35 @@ namespace sht {
 
 namespace {
 
-// Lane i ends up with sum over the warp of v[i] (recursive halving).
-__device__ __forceinline__ double warp_transpose_reduce32(double (&v)[32]) {
+// Sums v[0..15] over the lanes of the warp through 4 KB of shared memory:
+// every lane stores its 16 values as 8 chunks of 16 bytes (chunk c at c ^ (lane
+// & 7), so stores and loads touch all banks once per quarter-warp), lane
+// (q, c) adds chunk c of rows q, q + 4, ..., and two exchanges add the four
+// q.  Lane c < 8 returns the sums of v[2c] and v[2c + 1].
+__device__ __forceinline__ double2 warp_reduce16(const double (&v)[16], double2 *buf) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int s = 16; s >= 1; s >>= 1) {
-    const bool up = (lane & s) != 0;
+  for (int c = 0; c < 8; ++c) buf[lane * 8 + (c ^ (lane & 7))] = make_double2(v[2 * c], v[2 * c + 1]);
+  __syncwarp();
+  const int q = lane >> 3, c = lane & 7;
+  double2 w[8];
 #pragma unroll
-    for (int i = 0; i < s; ++i) {
-      const double send = up ? v[i] : v[i + s];
-      const double keep = up ? v[i + s] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
-    }
+  for (int t = 0; t < 8; ++t) {
+    const int row = q + 4 * t;
+    w[t] = buf[row * 8 + (c ^ (row & 7))];
   }
-  return v[0];
+#pragma unroll
+  for (int n = 4; n >= 1; n >>= 1)
+#pragma unroll
+    for (int t = 0; t < n; ++t) w[t] = make_double2(w[t].x + w[t + n].x, w[t].y + w[t + n].y);
+  double2 a = w[0];
+  __syncwarp();
+#pragma unroll
+  for (int s = 8; s <= 16; s <<= 1) {
+    a.x += __shfl_xor_sync(0xffffffffu, a.x, s);
+    a.y += __shfl_xor_sync(0xffffffffu, a.y, s);
+  }
+  return a;
 }
 
 // ---------------------------------------------------------------------------
@@ -149,6 +173,56 @@ __device__ __forceinline__ void copy16(double2 *dst, const double2 *src) {
 }
 
 // ---------------------------------------------------------------------------
+// State of one warp's rings in the recurrence.  Below 2^-kSwitchExp a ring
+// runs scaled and adds nothing (act false).  Rings that are absent or whose
+// seed vanished carry zeros and stay out of the test, so a warp is in one of
+// three states for each kLBlock steps: every ring scaled (only the recurrence
+// runs), every ring active (no test in the loop), or some of each (analysis
+// takes zero for the scaled ones; synthesis lets them add and clears their sums
+// when they become active).  A warp's rings are consecutive, i.e. neighbours in
+// latitude, so the mixed state is short (5% of the steps at Nside 1024 with 128
+// rings a warp).
+// ---------------------------------------------------------------------------
+enum WarpState { kSkip, kMixed, kFull };
+
+template <int R>
+__device__ __forceinline__ WarpState warp_state(const bool (&act)[R], const bool (&live)[R]) {
+  bool all = true, any = false;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    all = all && (act[r] || !live[r]);
+    any = any || act[r];
+  }
+  if (__all_sync(0xffffffffu, all)) return kFull;
+  return __any_sync(0xffffffffu, any) ? kMixed : kSkip;
+}
+
+// Spin-0 seed of one ring: (-1)^m mfac sin^m(theta) as mantissa and exponent.
+__device__ __forceinline__ void spin0_start(bool valid, double sth, int m, double sgn_mfac,
+                                            double &mu0, double &mu1, int &E, bool &live,
+                                            bool &act) {
+  XD sd = valid ? xd_pow(sth, m) : XD{0.0, 0};
+  sd = xd_norm(sd.v * sgn_mfac, sd.e);
+  mu0 = 0.0;
+  mu1 = sd.v;
+  E = sd.e;
+  live = valid && sd.v != 0.0;
+  act = live && E >= -kSwitchExp;
+  if (act) mu1 = ldexp(mu1, E);
+}
+
+__device__ __forceinline__ void spin0_renorm(bool &live, bool &act, double &mu0, double &mu1,
+                                             int &E) {
+  if (!live || act) return;
+  live = renorm_pair(mu1, mu0, E);
+  if (live && E >= -kSwitchExp) {
+    mu1 = ldexp(mu1, E);
+    mu0 = ldexp(mu0, E);
+    act = true;
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Spin-0 synthesis: phase_m(p) = sum_l lambda_lm(theta_p) a_lm, split into
 // even (p1) and odd (p2) l-m; north = p1+p2, south = p1-p2.
 // ---------------------------------------------------------------------------
@@ -160,12 +234,14 @@ synth_spin0_kernel(const int2 *__restrict__ items, const int *__restrict__ count
                    const double *__restrict__ alpha, const double *__restrict__ mfac,
                    const double2 *__restrict__ A, int ncA, int comp0, int lmax,
                    double2 *__restrict__ phase, int ncm, int pcomp0, int ms) {
-  __shared__ double s_al[kWarps][3][kChunk];
+  __shared__ __align__(16) double s_al[kWarps][3][kChunk];
   __shared__ double2 s_A[kWarps][3][kChunk * NT];
   const int2 it = items[blockIdx.x];
   const int m = it.x;
   const int cnt = count[m];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int p0 = it.y * (128 * R) + w * (32 * R) + lane;   // this lane's first pair
+  if (p0 - lane >= cnt) return;                            // no pair for this warp
   const long long mo = moff[m] - m;  // table index of l is mo + l
   const double *al = alpha + mo;
   const double2 *Am = A + mo * ncA + comp0;
@@ -174,7 +250,8 @@ synth_spin0_kernel(const int2 *__restrict__ items, const int *__restrict__ count
     if (ch < nchunks) {
       const int lc = m + ch * kChunk;
       const int b = ch % 3;
-      for (int t = lane; t < kChunk; t += 32) copy8(&s_al[w][b][t], al + lc + t);
+      copy8(&s_al[w][b][lane], al + lc + lane);
+#pragma unroll
       for (int t = lane; t < kChunk * NT; t += 32)
         copy16(&s_A[w][b][t], Am + (long long)(lc + t / NT) * ncA + t % NT);
     }
@@ -190,72 +267,85 @@ synth_spin0_kernel(const int2 *__restrict__ items, const int *__restrict__ count
   const double sgn_mfac = (m & 1) ? -mfac[m] : mfac[m];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int p = it.y * (128 * R) + r * 128 + threadIdx.x;
+    const int p = p0 + r * 32;
     const bool valid = p < cnt;
     x[r] = valid ? cth[p] : 0.0;
-    XD sd = valid ? xd_pow(sth[p], m) : XD{0.0, 0};
-    sd = xd_norm(sd.v * sgn_mfac, sd.e);
-    mu0[r] = 0.0;
-    mu1[r] = sd.v;
-    E[r] = sd.e;
-    live[r] = valid && sd.v != 0.0;
-    act[r] = live[r] && E[r] >= -kSwitchExp;
-    if (act[r]) mu1[r] = ldexp(mu1[r], E[r]);
+    spin0_start(valid, valid ? sth[p] : 0.0, m, sgn_mfac, mu0[r], mu1[r], E[r], live[r], act[r]);
 #pragma unroll
     for (int j = 0; j < NT; ++j) p1[r][j] = p2[r][j] = make_double2(0.0, 0.0);
   }
+  WarpState state = warp_state(act, live);
 
   for (int ch = 0; ch < nchunks; ++ch) {
     __pipeline_wait_prior(1);
     __syncwarp();
     stage(ch + 2);
-    const double *ca = s_al[w][ch % 3];
+    const double2 *ca = reinterpret_cast<const double2 *>(s_al[w][ch % 3]);
     const double2 *cA = s_A[w][ch % 3];
-#pragma unroll
-    for (int sb = 0; sb < kChunk; sb += kLBlock) {
+    const int nb = min(kChunk, lmax + 1 - (m + ch * kChunk));
+#pragma unroll 1
+    for (int sb = 0; sb < nb; sb += kLBlock) {
+      if (state != kSkip) {
 #pragma unroll 4
-      for (int i = sb; i < sb + kLBlock; i += 2) {
-        const double a0 = ca[i], a1 = ca[i + 1];
+        for (int i = sb; i < sb + kLBlock; i += 2) {
+          const double2 a = ca[i >> 1];
+          double e[R], o[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const double nm = fma(a0 * x[r], mu1[r], -mu0[r]);
-          const double nn = fma(a1 * x[r], nm, -mu1[r]);
-          if (act[r]) {
-#pragma unroll
-            for (int j = 0; j < NT; ++j) {
-              const double2 A0 = cA[i * NT + j], A1 = cA[(i + 1) * NT + j];
-              p1[r][j].x = fma(mu1[r], A0.x, p1[r][j].x);
-              p1[r][j].y = fma(mu1[r], A0.y, p1[r][j].y);
-              p2[r][j].x = fma(nm, A1.x, p2[r][j].x);
-              p2[r][j].y = fma(nm, A1.y, p2[r][j].y);
-            }
+          for (int r = 0; r < R; ++r) {
+            const double nm = fma(a.x * x[r], mu1[r], -mu0[r]);
+            const double nn = fma(a.y * x[r], nm, -mu1[r]);
+            e[r] = mu1[r];
+            o[r] = nm;
+            mu0[r] = nm;
+            mu1[r] = nn;
           }
-          mu0[r] = nm;
-          mu1[r] = nn;
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            const double2 A0 = cA[i * NT + j], A1 = cA[(i + 1) * NT + j];
+#pragma unroll
+            for (int r = 0; r < R; ++r) p1[r][j].x = fma(A0.x, e[r], p1[r][j].x);
+#pragma unroll
+            for (int r = 0; r < R; ++r) p1[r][j].y = fma(A0.y, e[r], p1[r][j].y);
+#pragma unroll
+            for (int r = 0; r < R; ++r) p2[r][j].x = fma(A1.x, o[r], p2[r][j].x);
+#pragma unroll
+            for (int r = 0; r < R; ++r) p2[r][j].y = fma(A1.y, o[r], p2[r][j].y);
+          }
+        }
+        if (state == kFull) continue;
+      } else {
+#pragma unroll 4
+        for (int i = sb; i < sb + kLBlock; i += 2) {
+          const double2 a = ca[i >> 1];
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const double nm = fma(a.x * x[r], mu1[r], -mu0[r]);
+            mu1[r] = fma(a.y * x[r], nm, -mu1[r]);
+            mu0[r] = nm;
+          }
         }
       }
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        if (live[r] && !act[r]) {
-          live[r] = renorm_pair(mu1[r], mu0[r], E[r]);
-          if (live[r] && E[r] >= -kSwitchExp) {
-            mu1[r] = ldexp(mu1[r], E[r]);
-            mu0[r] = ldexp(mu0[r], E[r]);
-            act[r] = true;
-          }
-        }
+        const bool was = act[r];
+        spin0_renorm(live[r], act[r], mu0[r], mu1[r], E[r]);
+        if (act[r] && !was)   // what the scaled steps added
+#pragma unroll
+          for (int j = 0; j < NT; ++j) p1[r][j] = p2[r][j] = make_double2(0.0, 0.0);
       }
+      state = warp_state(act, live);
     }
   }
 
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int p = it.y * (128 * R) + r * 128 + threadIdx.x;
+    const int p = p0 + r * 32;
     if (p >= cnt) continue;
     const bool has_s = nph_ring[2 * p + 1] > 0;
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
       const long long row = phase_row(p, ncm, pcomp0 + j, 0, ms);
+      if (!act[r]) p1[r][j] = p2[r][j] = make_double2(0.0, 0.0);
       phase[row + m] = make_double2(p1[r][j].x + p2[r][j].x, p1[r][j].y + p2[r][j].y);
       if (has_s)
         phase[row + ms + m] = make_double2(p1[r][j].x - p2[r][j].x, p1[r][j].y - p2[r][j].y);
@@ -266,6 +356,21 @@ synth_spin0_kernel(const int2 *__restrict__ items, const int *__restrict__ count
 // ---------------------------------------------------------------------------
 // Spin-s synthesis (DERIV=false: E/B -> Q/U; DERIV=true: a -> d/dtheta,
 // d/dphi with spin-1 functions).  Two recurrences mu+ / mu- share a_l, b_l.
+//
+// In the basis X1 = G - iC, X2 = G + iC (formed when the a_lm are staged) the
+// sums over lw = mu+ + mu-, lx = mu- - mu+ of the definition become
+//   P = sum mu+ X1,  M = sum mu- X2,  P' = sum (-1)^(l-mhi) mu+ X2,
+//   M' = sum (-1)^(l-mhi) mu- X1,
+//   Q_north = P + M, U_north = i (P - M), Q_south = P' + M',
+//   U_south = -i (P' - M')   (south rows times flip),
+// 8 FMAs per l without forming lw and lx.  With C = 0 (DERIV) X1 = X2 = G,
+// and P, P' are the sum and difference of the even and odd partial sums: 4
+// FMAs per l.
+//
+// Nside 1024, lmax 2048, one transform: 3.57 ms (FP64 pipe at 61% of its peak,
+// 67% being the most with three register operands); in terms of lw and lx, with
+// a test per l for the scaled regime, 4.71 ms.  Nside 2048, lmax 4096: 26.2
+// against 34.5 ms.  R = 3 or 4 rings per thread: 3.68, 3.94 ms.
 // ---------------------------------------------------------------------------
 template <int NT, int R, bool DERIV>
 __global__ void __launch_bounds__(128)
@@ -284,6 +389,8 @@ synth_spin_kernel(const int2 *__restrict__ items, const int *__restrict__ count,
   const int2 it = items[blockIdx.x];
   const int m = it.x;
   const int cnt = count[m];
+  const int p0 = it.y * (128 * R) + w * (32 * R) + lane;   // this lane's first pair
+  if (p0 - lane >= cnt) return;                            // no pair for this warp
   const int mhi = max(m, s);
   const long long mo = moff[m] - m;
   const double *aa = ca + mo;
@@ -294,10 +401,9 @@ synth_spin_kernel(const int2 *__restrict__ items, const int *__restrict__ count,
     if (ch < nchunks) {
       const int lc = mhi + ch * kChunk;
       const int b = ch % 3;
-      for (int t = lane; t < 2 * kChunk; t += 32) {
-        double *dst = reinterpret_cast<double *>(&s_ab[w][b][t >> 1]) + (t & 1);
-        copy8(dst, ((t & 1) ? bb : aa) + lc + (t >> 1));
-      }
+      copy8(&s_ab[w][b][lane].x, aa + lc + lane);
+      copy8(&s_ab[w][b][lane].y, bb + lc + lane);
+#pragma unroll
       for (int t = lane; t < kChunk * NC; t += 32)
         copy16(&s_A[w][b][t], Am + (long long)(lc + t / NC) * ncA + t % NC);
     }
@@ -309,18 +415,20 @@ synth_spin_kernel(const int2 *__restrict__ items, const int *__restrict__ count,
   double x[R], mp0[R], mp1[R], mm0[R], mm1[R];
   int Ep[R], Em[R];
   bool act[R], live[R];
-  double2 q1[R][NT], q2[R][NT], u1[R][NT], u2[R][NT];
+  // SP/SM: P and M, or (DERIV) their even parts; TP/TM: P' and M', or the odd parts
+  double2 SP[R][NT], SM[R][NT], TP[R][NT], TM[R][NT];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int p = it.y * (128 * R) + r * 128 + threadIdx.x;
+    const int p = p0 + r * 32;
     const bool valid = p < cnt;
     x[r] = valid ? cth[p] : 0.0;
     live[r] = spin_start(valid, x[r], valid ? sth[p] : 0.0, m, s, pre_v[m], pre_e[m], mp0[r],
                          mp1[r], mm0[r], mm1[r], Ep[r], Em[r], act[r]);
 #pragma unroll
     for (int j = 0; j < NT; ++j)
-      q1[r][j] = q2[r][j] = u1[r][j] = u2[r][j] = make_double2(0.0, 0.0);
+      SP[r][j] = SM[r][j] = TP[r][j] = TM[r][j] = make_double2(0.0, 0.0);
   }
+  WarpState state = warp_state(act, live);
 
   for (int ch = 0; ch < nchunks; ++ch) {
     __pipeline_wait_prior(1);
@@ -328,114 +436,210 @@ synth_spin_kernel(const int2 *__restrict__ items, const int *__restrict__ count,
     stage(ch + 2);
     const double2 *cab = s_ab[w][ch % 3];
     const double2 *cA = s_A[w][ch % 3];
-#pragma unroll
-    for (int sb = 0; sb < kChunk; sb += kLBlock) {
+    const int nb = min(kChunk, lmax + 1 - (mhi + ch * kChunk));
+#pragma unroll 1
+    for (int sb = 0; sb < nb; sb += kLBlock) {
+      if (state != kSkip) {
 #pragma unroll 2
-      for (int i = sb; i < sb + kLBlock; i += 2) {
-        const double2 ab0 = cab[i], ab1 = cab[i + 1];
+        for (int i = sb; i < sb + kLBlock; i += 2) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          // even offset from mhi: px = p1, py = p2
-          if (act[r]) {
-            const double lw = mp1[r] + mm1[r], lx = mm1[r] - mp1[r];
+          for (int odd = 0; odd < 2; ++odd) {
+            const double2 ab = cab[i + odd];
+            double ep[R], em[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              ep[r] = mp1[r];
+              em[r] = mm1[r];
+              const double np = fma(fma(ab.x, x[r], -ab.y), mp1[r], -mp0[r]);
+              const double nm = fma(fma(ab.x, x[r], ab.y), mm1[r], -mm0[r]);
+              mp0[r] = mp1[r];
+              mm0[r] = mm1[r];
+              mp1[r] = np;
+              mm1[r] = nm;
+            }
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
-              const double2 G0 = cA[i * NC + NA * j];
-              q1[r][j].x = fma(G0.x, lw, q1[r][j].x);
-              q1[r][j].y = fma(G0.y, lw, q1[r][j].y);
-              u2[r][j].x = fma(G0.y, lx, u2[r][j].x);
-              u2[r][j].y = fma(-G0.x, lx, u2[r][j].y);
-              if (!DERIV) {
-                const double2 C0 = cA[i * NC + NA * j + 1];
-                u1[r][j].x = fma(C0.x, lw, u1[r][j].x);
-                u1[r][j].y = fma(C0.y, lw, u1[r][j].y);
-                q2[r][j].x = fma(-C0.y, lx, q2[r][j].x);
-                q2[r][j].y = fma(C0.x, lx, q2[r][j].y);
+              if (DERIV) {
+                const double2 G = cA[(i + odd) * NC + j];
+                double2(&sp)[R][NT] = odd ? TP : SP;
+                double2(&sm)[R][NT] = odd ? TM : SM;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  sp[r][j].x = fma(G.x, ep[r], sp[r][j].x);
+                  sm[r][j].x = fma(G.x, em[r], sm[r][j].x);
+                }
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  sp[r][j].y = fma(G.y, ep[r], sp[r][j].y);
+                  sm[r][j].y = fma(G.y, em[r], sm[r][j].y);
+                }
+              } else {
+                const double2 X1 = cA[(i + odd) * NC + NA * j];
+                const double2 X2 = cA[(i + odd) * NC + NA * j + 1];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  SP[r][j].x = fma(X1.x, ep[r], SP[r][j].x);
+                  TM[r][j].x = fma(X1.x, odd ? -em[r] : em[r], TM[r][j].x);
+                }
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  SP[r][j].y = fma(X1.y, ep[r], SP[r][j].y);
+                  TM[r][j].y = fma(X1.y, odd ? -em[r] : em[r], TM[r][j].y);
+                }
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  SM[r][j].x = fma(X2.x, em[r], SM[r][j].x);
+                  TP[r][j].x = fma(X2.x, odd ? -ep[r] : ep[r], TP[r][j].x);
+                }
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  SM[r][j].y = fma(X2.y, em[r], SM[r][j].y);
+                  TP[r][j].y = fma(X2.y, odd ? -ep[r] : ep[r], TP[r][j].y);
+                }
               }
             }
           }
-          const double np_ = fma(fma(ab0.x, x[r], -ab0.y), mp1[r], -mp0[r]);
-          const double nm_ = fma(fma(ab0.x, x[r], ab0.y), mm1[r], -mm0[r]);
-          // odd offset: px = p2, py = p1
-          if (act[r]) {
-            const double lw = np_ + nm_, lx = nm_ - np_;
+        }
+        if (state == kFull) continue;
+      } else {
+#pragma unroll 4
+        for (int i = sb; i < sb + kLBlock; ++i) {
+          const double2 ab = cab[i];
 #pragma unroll
-            for (int j = 0; j < NT; ++j) {
-              const double2 G1 = cA[(i + 1) * NC + NA * j];
-              q2[r][j].x = fma(G1.x, lw, q2[r][j].x);
-              q2[r][j].y = fma(G1.y, lw, q2[r][j].y);
-              u1[r][j].x = fma(G1.y, lx, u1[r][j].x);
-              u1[r][j].y = fma(-G1.x, lx, u1[r][j].y);
-              if (!DERIV) {
-                const double2 C1 = cA[(i + 1) * NC + NA * j + 1];
-                u2[r][j].x = fma(C1.x, lw, u2[r][j].x);
-                u2[r][j].y = fma(C1.y, lw, u2[r][j].y);
-                q1[r][j].x = fma(-C1.y, lx, q1[r][j].x);
-                q1[r][j].y = fma(C1.x, lx, q1[r][j].y);
-              }
-            }
+          for (int r = 0; r < R; ++r) {
+            const double np = fma(fma(ab.x, x[r], -ab.y), mp1[r], -mp0[r]);
+            const double nm = fma(fma(ab.x, x[r], ab.y), mm1[r], -mm0[r]);
+            mp0[r] = mp1[r];
+            mm0[r] = mm1[r];
+            mp1[r] = np;
+            mm1[r] = nm;
           }
-          const double nnp = fma(fma(ab1.x, x[r], -ab1.y), np_, -mp1[r]);
-          const double nnm = fma(fma(ab1.x, x[r], ab1.y), nm_, -mm1[r]);
-          mp0[r] = np_;
-          mp1[r] = nnp;
-          mm0[r] = nm_;
-          mm1[r] = nnm;
         }
       }
 #pragma unroll
-      for (int r = 0; r < R; ++r)
+      for (int r = 0; r < R; ++r) {
+        const bool was = act[r];
         spin_renorm(live[r], act[r], mp0[r], mp1[r], mm0[r], mm1[r], Ep[r], Em[r]);
+        if (act[r] && !was)   // what the scaled steps added
+#pragma unroll
+          for (int j = 0; j < NT; ++j)
+            SP[r][j] = SM[r][j] = TP[r][j] = TM[r][j] = make_double2(0.0, 0.0);
+      }
+      state = warp_state(act, live);
     }
   }
 
   const double flip = ((mhi - m + s) & 1) ? -1.0 : 1.0;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int p = it.y * (128 * R) + r * 128 + threadIdx.x;
+    const int p = p0 + r * 32;
     if (p >= cnt) continue;
     const bool has_s = nph_ring[2 * p + 1] > 0;
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
       const long long rq = phase_row(p, ncm, pcomp0 + 2 * j, 0, ms);
       const long long ru = phase_row(p, ncm, pcomp0 + 2 * j + 1, 0, ms);
-      phase[rq + m] = make_double2(q1[r][j].x + q2[r][j].x, q1[r][j].y + q2[r][j].y);
-      phase[ru + m] = make_double2(u1[r][j].x + u2[r][j].x, u1[r][j].y + u2[r][j].y);
+      double2 P = SP[r][j], M = SM[r][j], Pd = TP[r][j], Md = TM[r][j];
+      if (!act[r]) P = M = Pd = Md = make_double2(0.0, 0.0);
+      if (DERIV) {
+        const double2 pe = P, po = Pd, me = M, mo_ = Md;
+        P = make_double2(pe.x + po.x, pe.y + po.y);
+        Pd = make_double2(pe.x - po.x, pe.y - po.y);
+        M = make_double2(me.x + mo_.x, me.y + mo_.y);
+        Md = make_double2(me.x - mo_.x, me.y - mo_.y);
+      }
+      phase[rq + m] = make_double2(P.x + M.x, P.y + M.y);
+      phase[ru + m] = make_double2(M.y - P.y, P.x - M.x);
       if (has_s) {
-        phase[rq + ms + m] = make_double2(flip * (q1[r][j].x - q2[r][j].x),
-                                          flip * (q1[r][j].y - q2[r][j].y));
-        phase[ru + ms + m] = make_double2(flip * (u1[r][j].x - u2[r][j].x),
-                                          flip * (u1[r][j].y - u2[r][j].y));
+        phase[rq + ms + m] = make_double2(flip * (Pd.x + Md.x), flip * (Pd.y + Md.y));
+        phase[ru + ms + m] = make_double2(flip * (Pd.y - Md.y), flip * (Md.x - Pd.x));
       }
     }
   }
 }
 
 // ---------------------------------------------------------------------------
-// Analysis.  One CTA of 128 threads per m loops over tiles of 128*R ring
-// pairs.  Per l-block (LB steps, LB*VPL == 32 values) every lane accumulates
+// Analysis.  One CTA of W warps per m loops over tiles of 32*W*R ring pairs.  Per l-block (LB steps, LB*VPL == 32 values) every lane accumulates
 // its R rings' contributions; a warp transpose-reduction leaves one sum per
-// lane, kept in a per-warp shared array for the whole chunk.  At the next
-// chunk's barrier (the same one that publishes staged coefficients) warp 0
-// adds the four warps' sums in a fixed order to Aout, which this CTA owns:
-// no atomics, bitwise repeatable, one barrier per 32 l-steps.
+// lane, kept in a per-warp shared array for the whole chunk.  After the next
+// chunk's barrier (the same one that publishes staged coefficients) the warps
+// share out the sub-blocks, add the warps' sums in a fixed order and store
+// them (first tile) or add them (later tiles; the same thread owns an entry
+// in every tile) to Aout, which this CTA owns: no atomics, bitwise repeatable,
+// one barrier per kAChunk l-steps.  Every row l in [m, lmax] is written.
+//
+// The reduction through shared memory takes 42 instructions per 16 values;
+// recursive halving with shuffles took 107, more than half of them selects, and
+// left the FP64 pipe at 40%.  With it and the loops free of tests, Nside 1024 /
+// lmax 2048: spin 2 5.02 ms, spin 0 1.77 (before: 6.11 and 1.99); Nside 2048 /
+// lmax 4096: 35.2 and 12.4 (44.8 and 14.1).  Rings of a thread spread over the
+// tile (equal work for the warps between two barriers), with loops compiled for
+// each number of active ones: 5.1-5.3 and 1.94 ms, so a warp's rings stay
+// consecutive.  The contraction on the FP64 tensor instructions fills 4 (spin s)
+// or 2 (spin 0) of the 8 columns of an m8n8k4 with one transform: no gain.
 // ---------------------------------------------------------------------------
-template <int VPL>
-__device__ __forceinline__ void flush_chunk(const double (*wred)[kChunk * VPL / 32][32], int lane,
-                                            int l0, long long mo, int ncA, int comp0,
+// l-steps per chunk: the warps' sums of two chunks within 48 KB of shared memory
+template <int VPL, int W>
+constexpr int kAChunkOf = VPL * W >= 32 ? 32 : 64;
+constexpr int kRed = 16;   // values per transpose-reduction
+
+template <int VPL, int W>
+__device__ __forceinline__ void flush_chunk(const double *wred, int nwarps, bool first, int l0,
+                                            int lmax, long long mo, int ncA, int comp0,
                                             double *__restrict__ Aout) {
-  constexpr int LB = 32 / VPL;
-#pragma unroll 1
-  for (int sb = 0; sb < kChunk / LB; ++sb) {
-    const double acc = (wred[0][sb][lane] + wred[1][sb][lane]) +
-                       (wred[2][sb][lane] + wred[3][sb][lane]);
-    const int l = l0 + sb * LB + lane / VPL;
-    Aout[((mo + l) * ncA + comp0) * 2 + lane % VPL] += acc;
+  constexpr int ld = kAChunkOf<VPL, W> * VPL;
+  const int n = min(kAChunkOf<VPL, W>, lmax + 1 - l0) * VPL;
+  for (int t = threadIdx.x; t < n; t += 32 * W) {
+    double acc = wred[t];
+    for (int w = 1; w < nwarps; ++w) acc += wred[w * ld + t];
+    double *out = Aout + ((mo + l0 + t / VPL) * ncA + comp0) * 2 + t % VPL;
+    *out = first ? acc : *out + acc;
   }
 }
 
-template <int NT, int R>
-__global__ void __launch_bounds__(128)
+// Dynamic shared memory of an analysis CTA: the warps' transposition buffers and
+// their sums of two chunks.
+template <int VPL, int W>
+constexpr size_t anal_smem() {
+  return sizeof(double) * W * (32 * kRed + 2 * kAChunkOf<VPL, W> * VPL);
+}
+__host__ __device__ constexpr int anal_min_blocks(int spin, int NT, int R, int W) {
+  return W == 8 ? (NT * (spin + 1) > 2 ? 1 : 2) : NT > 1 ? 2 : spin == 0 || R <= 2 ? 4 : 3;
+}
+
+// Rows [l0, l1) of this CTA's m that no ring reaches.
+template <int VPL>
+__device__ __forceinline__ void zero_rows(int l0, int l1, long long mo, int ncA, int comp0,
+                                          double *__restrict__ Aout) {
+  for (int t = threadIdx.x; t < (l1 - l0) * VPL; t += blockDim.x)
+    Aout[((mo + l0 + t / VPL) * ncA + comp0) * 2 + t % VPL] = 0.0;
+}
+
+// Phase factors of rings that are not active yet are multiplied by zero in the
+// mixed state.  Those that are not finite must not enter there: hold() moves
+// them to local memory and leaves zeros until release() at the ring's
+// activation.
+template <int N>
+__device__ __forceinline__ bool hold(double *(&f)[N], volatile double *kept) {
+  double t = 0.0;
+#pragma unroll
+  for (int k = 0; k < N; ++k) t += 0.0 * *f[k];
+  if (t == 0.0) return false;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    kept[k] = *f[k];
+    *f[k] = 0.0;
+  }
+  return true;
+}
+template <int N>
+__device__ __forceinline__ void release(double *(&f)[N], const volatile double *kept) {
+#pragma unroll
+  for (int k = 0; k < N; ++k) *f[k] = kept[k];
+}
+
+template <int NT, int R, int W>
+__global__ void __launch_bounds__(32 * W, anal_min_blocks(0, NT, R, W))
 anal_spin0_kernel(const int *__restrict__ count, const double *__restrict__ cth,
                   const double *__restrict__ sth, const int *__restrict__ nph_ring,
                   const long long *__restrict__ moff, const double *__restrict__ alpha,
@@ -443,111 +647,145 @@ anal_spin0_kernel(const int *__restrict__ count, const double *__restrict__ cth,
                   int pcomp0, int lmax, int ms, double *__restrict__ Aout, int ncA,
                   int comp0) {
   constexpr int VPL = 2 * NT;
-  constexpr int LB = 32 / VPL;
-  constexpr int NSB = kChunk / LB;
-  static_assert(LB % 2 == 0 && kChunk % LB == 0, "l-block must be even and divide a chunk");
-  __shared__ double wred[2][kWarps][NSB][32];
-  __shared__ double s_al[3][kChunk];
+  constexpr int LB = kRed / VPL, kAChunk = kAChunkOf<VPL, W>;
+  static_assert(LB % 2 == 0 && kLBlock % LB == 0, "l-block must be even and divide kLBlock");
+  extern __shared__ double2 smem[];
+  double2(*red)[32 * kRed / 2] = reinterpret_cast<double2(*)[32 * kRed / 2]>(smem);
+  double(*wred)[W][kAChunk * VPL] =
+      reinterpret_cast<double(*)[W][kAChunk * VPL]>(smem + W * (32 * kRed / 2));
+  __shared__ __align__(16) double s_al[3][kAChunk];
   const int m = blockIdx.x;
   const int cnt = count[m];
   const long long mo = moff[m] - m;
+  if (cnt == 0) {
+    zero_rows<VPL>(m, lmax + 1, mo, ncA, comp0, Aout);
+    return;
+  }
   const double *al = alpha + mo;
   const double sgn_mfac = (m & 1) ? -mfac[m] : mfac[m];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nchunks = (lmax - m + kChunk) / kChunk;
+  const int nchunks = (lmax - m + kAChunk) / kAChunk;
   auto stage = [&](int ch) {
+    const int l0 = m + ch * kAChunk;
+    // up to the end of the last kLBlock steps (inside the table's padding)
     if (ch < nchunks)
-      for (int t = threadIdx.x; t < kChunk; t += blockDim.x)
-        copy8(&s_al[ch % 3][t], al + m + ch * kChunk + t);
+      for (int t = threadIdx.x; t < min(kAChunk, lmax + kLBlock - l0); t += 32 * W)
+        copy8(&s_al[ch % 3][t], al + l0 + t);
     __pipeline_commit();
   };
 
-  for (int tb = 0; tb < cnt; tb += 128 * R) {
+  for (int tb = 0; tb < cnt; tb += 32 * W * R) {
     stage(0);
     stage(1);
+    const int nwarps = min(W, (cnt - tb + 32 * R - 1) / (32 * R));
+    const int p0 = tb + warp * (32 * R) + lane;
     double x[R], mu0[R], mu1[R];
     int E[R];
     bool act[R], live[R];
     double2 P1[R][NT], P2[R][NT];
+    volatile double kept[R][NT][4];
+    unsigned held = 0;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int p = tb + r * 128 + threadIdx.x;
+      const int p = p0 + r * 32;
       const bool valid = p < cnt;
       x[r] = valid ? cth[p] : 0.0;
-      XD sd = valid ? xd_pow(sth[p], m) : XD{0.0, 0};
-      sd = xd_norm(sd.v * sgn_mfac, sd.e);
-      mu0[r] = 0.0;
-      mu1[r] = sd.v;
-      E[r] = sd.e;
-      live[r] = valid && sd.v != 0.0;
-      act[r] = live[r] && E[r] >= -kSwitchExp;
-      if (act[r]) mu1[r] = ldexp(mu1[r], E[r]);
-      const bool has_s = valid && nph_ring[2 * p + 1] > 0;
+      spin0_start(valid, valid ? sth[p] : 0.0, m, sgn_mfac, mu0[r], mu1[r], E[r], live[r],
+                  act[r]);
+      const bool has_s = live[r] && nph_ring[2 * p + 1] > 0;   // dead rings stay out of the sums
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
-        const long long row = phase_row(valid ? p : 0, ncm, pcomp0 + j, 0, ms);
-        const double2 n = valid ? phase[row + m] : make_double2(0.0, 0.0);
+        const long long row = phase_row(live[r] ? p : 0, ncm, pcomp0 + j, 0, ms);
+        const double2 n = live[r] ? phase[row + m] : make_double2(0.0, 0.0);
         const double2 sv = has_s ? phase[row + ms + m] : make_double2(0.0, 0.0);
         P1[r][j] = make_double2(n.x + sv.x, n.y + sv.y);
         P2[r][j] = make_double2(n.x - sv.x, n.y - sv.y);
+        double *f[4] = {&P1[r][j].x, &P1[r][j].y, &P2[r][j].x, &P2[r][j].y};
+        if (!act[r] && hold(f, kept[r][j])) held |= 1u << (r * NT + j);
       }
     }
+    WarpState state = warp_state(act, live);
 
     for (int ch = 0; ch < nchunks; ++ch) {
       __pipeline_wait_prior(1);
       __syncthreads();
       stage(ch + 2);
-      if (ch > 0 && warp == 0)
-        flush_chunk<VPL>(wred[(ch - 1) & 1], lane, m + (ch - 1) * kChunk, mo, ncA, comp0, Aout);
-      const double *ca = s_al[ch % 3];
+      if (ch > 0)
+        flush_chunk<VPL, W>(wred[(ch - 1) & 1][0], nwarps, tb == 0, m + (ch - 1) * kAChunk, lmax, mo,
+                         ncA, comp0, Aout);
+      if (warp >= nwarps) continue;
+      const double2 *ca = reinterpret_cast<const double2 *>(s_al[ch % 3]);
+      const int nb = min(kAChunk, lmax + 1 - (m + ch * kAChunk));
 #pragma unroll 1
-      for (int sb = 0; sb < NSB; ++sb) {
-        double v[32];
+      for (int b0 = 0; b0 < nb; b0 += kLBlock) {
+        auto steps = [&](auto masked) {
+          constexpr bool MASK = decltype(masked)::value;
+#pragma unroll 1
+          for (int sb = b0 / LB; sb < (b0 + kLBlock) / LB; ++sb) {
+            double v[kRed];
 #pragma unroll
-        for (int k = 0; k < 32; ++k) v[k] = 0.0;
-        bool any = false;
+            for (int i = 0; i < LB; i += 2) {
+              const double2 a = ca[(sb * LB + i) >> 1];
 #pragma unroll
-        for (int i = 0; i < LB; i += 2) {
-          const double a0 = ca[sb * LB + i], a1 = ca[sb * LB + i + 1];
+              for (int r = 0; r < R; ++r) {
+                const double nm = fma(a.x * x[r], mu1[r], -mu0[r]);
+                const double nn = fma(a.y * x[r], nm, -mu1[r]);
+                const double e = MASK && !act[r] ? 0.0 : mu1[r];
+                const double o = MASK && !act[r] ? 0.0 : nm;
 #pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const double nm = fma(a0 * x[r], mu1[r], -mu0[r]);
-            const double nn = fma(a1 * x[r], nm, -mu1[r]);
-            if (act[r]) {
-#pragma unroll
-              for (int j = 0; j < NT; ++j) {
-                v[i * VPL + 2 * j] = fma(mu1[r], P1[r][j].x, v[i * VPL + 2 * j]);
-                v[i * VPL + 2 * j + 1] = fma(mu1[r], P1[r][j].y, v[i * VPL + 2 * j + 1]);
-                v[(i + 1) * VPL + 2 * j] = fma(nm, P2[r][j].x, v[(i + 1) * VPL + 2 * j]);
-                v[(i + 1) * VPL + 2 * j + 1] =
-                    fma(nm, P2[r][j].y, v[(i + 1) * VPL + 2 * j + 1]);
+                for (int j = 0; j < NT; ++j) {
+                  double *ve = v + i * VPL + 2 * j, *vo = ve + VPL;
+                  ve[0] = r == 0 ? e * P1[r][j].x : fma(e, P1[r][j].x, ve[0]);
+                  ve[1] = r == 0 ? e * P1[r][j].y : fma(e, P1[r][j].y, ve[1]);
+                  vo[0] = r == 0 ? o * P2[r][j].x : fma(o, P2[r][j].x, vo[0]);
+                  vo[1] = r == 0 ? o * P2[r][j].y : fma(o, P2[r][j].y, vo[1]);
+                }
+                mu0[r] = nm;
+                mu1[r] = nn;
               }
             }
-            mu0[r] = nm;
-            mu1[r] = nn;
+            const double2 sum = warp_reduce16(v, red[warp]);
+            if (lane < kRed / 2)
+              *reinterpret_cast<double2 *>(&wred[ch & 1][warp][sb * kRed + 2 * lane]) = sum;
           }
+        };
+        if (state == kFull) {
+          steps(std::false_type{});
+          continue;
+        }
+        if (state == kMixed) {
+          steps(std::true_type{});
+        } else {
+#pragma unroll 4
+          for (int i = b0; i < b0 + kLBlock; i += 2) {
+            const double2 a = ca[i >> 1];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const double nm = fma(a.x * x[r], mu1[r], -mu0[r]);
+              mu1[r] = fma(a.y * x[r], nm, -mu1[r]);
+              mu0[r] = nm;
+            }
+          }
+          for (int t = lane; t < kLBlock * VPL; t += 32) wred[ch & 1][warp][b0 * VPL + t] = 0.0;
         }
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          any |= act[r];
-          if (live[r] && !act[r] && ((sb + 1) * LB) % kLBlock == 0) {
-            live[r] = renorm_pair(mu1[r], mu0[r], E[r]);
-            if (live[r] && E[r] >= -kSwitchExp) {
-              mu1[r] = ldexp(mu1[r], E[r]);
-              mu0[r] = ldexp(mu0[r], E[r]);
-              act[r] = true;
+          const bool was = act[r];
+          spin0_renorm(live[r], act[r], mu0[r], mu1[r], E[r]);
+          if (held && act[r] && !was)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+              double *f[4] = {&P1[r][j].x, &P1[r][j].y, &P2[r][j].x, &P2[r][j].y};
+              if (held >> (r * NT + j) & 1) release(f, kept[r][j]);
             }
-          }
         }
-        wred[ch & 1][warp][sb][lane] =
-            __any_sync(0xffffffffu, any) ? warp_transpose_reduce32(v) : 0.0;
+        state = warp_state(act, live);
       }
     }
     __pipeline_wait_prior(0);
     __syncthreads();
-    if (warp == 0)
-      flush_chunk<VPL>(wred[(nchunks - 1) & 1], lane, m + (nchunks - 1) * kChunk, mo, ncA, comp0,
-                       Aout);
+    flush_chunk<VPL, W>(wred[(nchunks - 1) & 1][0], nwarps, tb == 0, m + (nchunks - 1) * kAChunk, lmax,
+                     mo, ncA, comp0, Aout);
     __syncthreads();
   }
 }
@@ -556,10 +794,11 @@ anal_spin0_kernel(const int *__restrict__ count, const double *__restrict__ cth,
 // transform (saddstep2, libsharp/sharp_core_inc2.c:338-364), written directly
 // in terms of mu+ and mu- (lw = mu+ + mu-, lx = mu- - mu+):
 //   lw X - lx Y = mu+ (X+Y) + mu- (X-Y),   lw X + lx Y = mu+ (X-Y) + mu- (X+Y)
-// so each output takes 2 FMAs and lw, lx are never formed.  H?p / H?m hold
-// the combined phase factors of mu+ / mu- for even (e) and odd (o) l-mhi.
-template <int NT, int R>
-__global__ void __launch_bounds__(128)
+// so each output takes 2 FMAs and lw, lx are never formed.  h / g hold the
+// combined phase factors of mu+ / mu- for even l-mhi; those of odd l-mhi are
+// the same eight numbers in reverse order with alternating signs.
+template <int NT, int R, int W>
+__global__ void __launch_bounds__(32 * W, anal_min_blocks(1, NT, R, W))
 anal_spin_kernel(const int *__restrict__ count, const double *__restrict__ cth,
                  const double *__restrict__ sth, const int *__restrict__ nph_ring,
                  const long long *__restrict__ moff, const double *__restrict__ ca,
@@ -568,51 +807,59 @@ anal_spin_kernel(const int *__restrict__ count, const double *__restrict__ cth,
                  int ncm, int pcomp0, int lmax, int ms, double *__restrict__ Aout, int ncA,
                  int comp0) {
   constexpr int VPL = 4 * NT;
-  constexpr int LB = 32 / VPL;
-  constexpr int NSB = kChunk / LB;
-  static_assert(LB % 2 == 0 && kChunk % LB == 0, "l-block must be even and divide a chunk");
-  __shared__ double wred[2][kWarps][NSB][32];
-  __shared__ double2 s_ab[3][kChunk];
+  constexpr int LB = kRed / VPL, kAChunk = kAChunkOf<VPL, W>;
+  static_assert(LB % 2 == 0 && kLBlock % LB == 0, "l-block must be even and divide kLBlock");
+  extern __shared__ double2 smem[];
+  double2(*red)[32 * kRed / 2] = reinterpret_cast<double2(*)[32 * kRed / 2]>(smem);
+  double(*wred)[W][kAChunk * VPL] =
+      reinterpret_cast<double(*)[W][kAChunk * VPL]>(smem + W * (32 * kRed / 2));
+  __shared__ double2 s_ab[3][kAChunk];
   const int m = blockIdx.x;
   const int cnt = count[m];
   const int mhi = max(m, s);
   const long long mo = moff[m] - m;
+  zero_rows<VPL>(m, cnt == 0 ? lmax + 1 : mhi, mo, ncA, comp0, Aout);
+  if (cnt == 0) return;
   const double *aa = ca + mo;
   const double *bb = cb + mo;
   const double flip = ((mhi - m + s) & 1) ? -1.0 : 1.0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nchunks = (lmax - mhi + kChunk) / kChunk;
+  const int nchunks = (lmax - mhi + kAChunk) / kAChunk;
   auto stage = [&](int ch) {
+    const int l0 = mhi + ch * kAChunk;
+    // up to the end of the last kLBlock steps (inside the tables' padding)
     if (ch < nchunks)
-      for (int t = threadIdx.x; t < 2 * kChunk; t += blockDim.x) {
-        double *dst = reinterpret_cast<double *>(&s_ab[ch % 3][t >> 1]) + (t & 1);
-        copy8(dst, ((t & 1) ? bb : aa) + mhi + ch * kChunk + (t >> 1));
-      }
+      for (int t = threadIdx.x; t < 2 * min(kAChunk, lmax + kLBlock - l0); t += 32 * W)
+        copy8(reinterpret_cast<double *>(&s_ab[ch % 3][t >> 1]) + (t & 1),
+              ((t & 1) ? bb : aa) + l0 + (t >> 1));
     __pipeline_commit();
   };
 
-  for (int tb = 0; tb < cnt; tb += 128 * R) {
+  for (int tb = 0; tb < cnt; tb += 32 * W * R) {
     stage(0);
     stage(1);
+    const int nwarps = min(W, (cnt - tb + 32 * R - 1) / (32 * R));
+    const int p0 = tb + warp * (32 * R) + lane;
     double x[R], mp0[R], mp1[R], mm0[R], mm1[R];
     int Ep[R], Em[R];
     bool act[R], live[R];
-    // [r][j][k]: k = G.re, G.im, C.re, C.im
-    double Hep[R][NT][4], Hem[R][NT][4], Hop[R][NT][4], Hom[R][NT][4];
+    double h[R][NT][4], g[R][NT][4];   // G.re, G.im, C.re, C.im
+    volatile double kept[R][NT][8];
+    unsigned held = 0;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int p = tb + r * 128 + threadIdx.x;
+      const int p = p0 + r * 32;
       const bool valid = p < cnt;
       x[r] = valid ? cth[p] : 0.0;
       live[r] = spin_start(valid, x[r], valid ? sth[p] : 0.0, m, s, pre_v[m], pre_e[m],
                            mp0[r], mp1[r], mm0[r], mm1[r], Ep[r], Em[r], act[r]);
-      const bool has_s = valid && nph_ring[2 * p + 1] > 0;
+      const bool has_s = live[r] && nph_ring[2 * p + 1] > 0;   // dead rings stay out of the sums
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
-        const long long rq = phase_row(valid ? p : 0, ncm, pcomp0 + 2 * j, 0, ms);
-        const long long ru = phase_row(valid ? p : 0, ncm, pcomp0 + 2 * j + 1, 0, ms);
-        const double2 qn = valid ? phase[rq + m] : make_double2(0.0, 0.0);
-        const double2 un = valid ? phase[ru + m] : make_double2(0.0, 0.0);
+        const long long rq = phase_row(live[r] ? p : 0, ncm, pcomp0 + 2 * j, 0, ms);
+        const long long ru = phase_row(live[r] ? p : 0, ncm, pcomp0 + 2 * j + 1, 0, ms);
+        const double2 qn = live[r] ? phase[rq + m] : make_double2(0.0, 0.0);
+        const double2 un = live[r] ? phase[ru + m] : make_double2(0.0, 0.0);
         double2 qs = has_s ? phase[rq + ms + m] : make_double2(0.0, 0.0);
         double2 us = has_s ? phase[ru + ms + m] : make_double2(0.0, 0.0);
         qs.x *= flip; qs.y *= flip; us.x *= flip; us.y *= flip;
@@ -623,80 +870,114 @@ anal_spin_kernel(const int *__restrict__ count, const double *__restrict__ cth,
         // even offset: px = p1, py = p2
         //   G.re = lw P1q.re - lx P2u.im   G.im = lw P1q.im + lx P2u.re
         //   C.re = lw P1u.re + lx P2q.im   C.im = lw P1u.im - lx P2q.re
-        Hep[r][j][0] = P1q.x + P2u.y; Hem[r][j][0] = P1q.x - P2u.y;
-        Hep[r][j][1] = P1q.y - P2u.x; Hem[r][j][1] = P1q.y + P2u.x;
-        Hep[r][j][2] = P1u.x - P2q.y; Hem[r][j][2] = P1u.x + P2q.y;
-        Hep[r][j][3] = P1u.y + P2q.x; Hem[r][j][3] = P1u.y - P2q.x;
         // odd offset: px = p2, py = p1
-        Hop[r][j][0] = P2q.x + P1u.y; Hom[r][j][0] = P2q.x - P1u.y;
-        Hop[r][j][1] = P2q.y - P1u.x; Hom[r][j][1] = P2q.y + P1u.x;
-        Hop[r][j][2] = P2u.x - P1q.y; Hom[r][j][2] = P2u.x + P1q.y;
-        Hop[r][j][3] = P2u.y + P1q.x; Hom[r][j][3] = P2u.y - P1q.x;
+        h[r][j][0] = P1q.x + P2u.y; g[r][j][0] = P1q.x - P2u.y;
+        h[r][j][1] = P1q.y - P2u.x; g[r][j][1] = P1q.y + P2u.x;
+        h[r][j][2] = P1u.x - P2q.y; g[r][j][2] = P1u.x + P2q.y;
+        h[r][j][3] = P1u.y + P2q.x; g[r][j][3] = P1u.y - P2q.x;
+        double *f[8] = {&h[r][j][0], &h[r][j][1], &h[r][j][2], &h[r][j][3],
+                        &g[r][j][0], &g[r][j][1], &g[r][j][2], &g[r][j][3]};
+        if (!act[r] && hold(f, kept[r][j])) held |= 1u << (r * NT + j);
       }
     }
+    WarpState state = warp_state(act, live);
 
     for (int ch = 0; ch < nchunks; ++ch) {
       __pipeline_wait_prior(1);
       __syncthreads();
       stage(ch + 2);
-      if (ch > 0 && warp == 0)
-        flush_chunk<VPL>(wred[(ch - 1) & 1], lane, mhi + (ch - 1) * kChunk, mo, ncA, comp0,
-                         Aout);
+      if (ch > 0)
+        flush_chunk<VPL, W>(wred[(ch - 1) & 1][0], nwarps, tb == 0, mhi + (ch - 1) * kAChunk, lmax, mo,
+                         ncA, comp0, Aout);
+      if (warp >= nwarps) continue;
       const double2 *cab = s_ab[ch % 3];
+      const int nb = min(kAChunk, lmax + 1 - (mhi + ch * kAChunk));
 #pragma unroll 1
-      for (int sb = 0; sb < NSB; ++sb) {
-        double v[32];
+      for (int b0 = 0; b0 < nb; b0 += kLBlock) {
+        auto steps = [&](auto masked) {
+          constexpr bool MASK = decltype(masked)::value;
+#pragma unroll 1
+          for (int sb = b0 / LB; sb < (b0 + kLBlock) / LB; ++sb) {
+            double v[kRed];
 #pragma unroll
-        for (int k = 0; k < 32; ++k) v[k] = 0.0;
-        bool any = false;
+            for (int i = 0; i < LB; ++i) {
+              const double2 ab = cab[sb * LB + i];
 #pragma unroll
-        for (int i = 0; i < LB; i += 2) {
-          const double2 ab0 = cab[sb * LB + i], ab1 = cab[sb * LB + i + 1];
+              for (int r = 0; r < R; ++r) {
+                const double ep = MASK && !act[r] ? 0.0 : mp1[r];
+                const double em = MASK && !act[r] ? 0.0 : mm1[r];
 #pragma unroll
-          for (int r = 0; r < R; ++r) {
-            if (act[r]) {
+                for (int j = 0; j < NT; ++j) {
+                  double *o = v + i * VPL + 4 * j;
 #pragma unroll
-              for (int j = 0; j < NT; ++j)
+                  for (int k = 0; k < 4; ++k) {
+                    // odd: +h3, -h2, -h1, +h0
+                    const double f = (i & 1) ? ((k == 1 || k == 2) ? -h[r][j][3 - k] : h[r][j][3 - k])
+                                             : h[r][j][k];
+                    o[k] = r == 0 ? ep * f : fma(ep, f, o[k]);
+                  }
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  double &o = v[i * VPL + 4 * j + k];
-                  o = fma(mp1[r], Hep[r][j][k], fma(mm1[r], Hem[r][j][k], o));
+                  for (int k = 0; k < 4; ++k) {
+                    // odd: -g3, +g2, +g1, -g0
+                    const double f = (i & 1) ? ((k == 1 || k == 2) ? g[r][j][3 - k] : -g[r][j][3 - k])
+                                             : g[r][j][k];
+                    o[k] = fma(em, f, o[k]);
+                  }
                 }
+                const double np = fma(fma(ab.x, x[r], -ab.y), mp1[r], -mp0[r]);
+                const double nm = fma(fma(ab.x, x[r], ab.y), mm1[r], -mm0[r]);
+                mp0[r] = mp1[r];
+                mm0[r] = mm1[r];
+                mp1[r] = np;
+                mm1[r] = nm;
+              }
             }
-            const double np_ = fma(fma(ab0.x, x[r], -ab0.y), mp1[r], -mp0[r]);
-            const double nm_ = fma(fma(ab0.x, x[r], ab0.y), mm1[r], -mm0[r]);
-            if (act[r]) {
-#pragma unroll
-              for (int j = 0; j < NT; ++j)
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  double &o = v[(i + 1) * VPL + 4 * j + k];
-                  o = fma(np_, Hop[r][j][k], fma(nm_, Hom[r][j][k], o));
-                }
-            }
-            const double nnp = fma(fma(ab1.x, x[r], -ab1.y), np_, -mp1[r]);
-            const double nnm = fma(fma(ab1.x, x[r], ab1.y), nm_, -mm1[r]);
-            mp0[r] = np_;
-            mp1[r] = nnp;
-            mm0[r] = nm_;
-            mm1[r] = nnm;
+            const double2 sum = warp_reduce16(v, red[warp]);
+            if (lane < kRed / 2)
+              *reinterpret_cast<double2 *>(&wred[ch & 1][warp][sb * kRed + 2 * lane]) = sum;
           }
+        };
+        if (state == kFull) {
+          steps(std::false_type{});
+          continue;
+        }
+        if (state == kMixed) {
+          steps(std::true_type{});
+        } else {
+#pragma unroll 4
+          for (int i = b0; i < b0 + kLBlock; ++i) {
+            const double2 ab = cab[i];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const double np = fma(fma(ab.x, x[r], -ab.y), mp1[r], -mp0[r]);
+              const double nm = fma(fma(ab.x, x[r], ab.y), mm1[r], -mm0[r]);
+              mp0[r] = mp1[r];
+              mm0[r] = mm1[r];
+              mp1[r] = np;
+              mm1[r] = nm;
+            }
+          }
+          for (int t = lane; t < kLBlock * VPL; t += 32) wred[ch & 1][warp][b0 * VPL + t] = 0.0;
         }
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          any |= act[r];
-          if (((sb + 1) * LB) % kLBlock == 0)
-            spin_renorm(live[r], act[r], mp0[r], mp1[r], mm0[r], mm1[r], Ep[r], Em[r]);
+          const bool was = act[r];
+          spin_renorm(live[r], act[r], mp0[r], mp1[r], mm0[r], mm1[r], Ep[r], Em[r]);
+          if (held && act[r] && !was)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+              double *f[8] = {&h[r][j][0], &h[r][j][1], &h[r][j][2], &h[r][j][3],
+                              &g[r][j][0], &g[r][j][1], &g[r][j][2], &g[r][j][3]};
+              if (held >> (r * NT + j) & 1) release(f, kept[r][j]);
+            }
         }
-        wred[ch & 1][warp][sb][lane] =
-            __any_sync(0xffffffffu, any) ? warp_transpose_reduce32(v) : 0.0;
+        state = warp_state(act, live);
       }
     }
     __pipeline_wait_prior(0);
     __syncthreads();
-    if (warp == 0)
-      flush_chunk<VPL>(wred[(nchunks - 1) & 1], lane, mhi + (nchunks - 1) * kChunk, mo, ncA,
-                       comp0, Aout);
+    flush_chunk<VPL, W>(wred[(nchunks - 1) & 1][0], nwarps, tb == 0, mhi + (nchunks - 1) * kAChunk,
+                     lmax, mo, ncA, comp0, Aout);
     __syncthreads();
   }
 }
@@ -724,32 +1005,34 @@ void launch_legendre_synth(const JobDesc &job, const GeomPlan &gp, const CoefPla
   const int nitems = int(gp.synth_items.size());
   if (nitems == 0) return;
   ProfScope ps("legendre_synth", st);
-  constexpr int R = 2;
-  SHT_REQUIRE(gp.synth_tile == 128 * R, "synthesis tile mismatch");
   const bool deriv = job.type == SHARP_ALM2MAP_DERIV1;
-  if (job.spin == 0 && !deriv) {
-#define SHT_S0(NTV)                                                                           \
-  synth_spin0_kernel<NTV, R><<<nitems, 128, 0, st>>>(                                         \
-      gp.items, gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff, cp.alpha, cp.seed, A, ncA, comp0, \
-      job.lmax, phase, ncm, pcomp0, job.mmax + 1)
-    if (nt == 1) SHT_S0(1);
-    else if (nt == 2) SHT_S0(2);
-    else SHT_S0(4);
-#undef SHT_S0
-  } else {
-#define SHT_SS(NTV, DV)                                                                         \
-  synth_spin_kernel<NTV, R, DV><<<nitems, 128, 0, st>>>(                                        \
-      gp.items, gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff, cp.alpha, cp.beta, cp.seed,        \
-      cp.seed_exp, cp.spin, A, ncA, comp0, job.lmax, phase, ncm, pcomp0, job.mmax + 1)
-    if (deriv) {
-      if (nt == 1) SHT_SS(1, true);
-      else SHT_SS(2, true);
+  SHT_REQUIRE(gp.synth_tile == 128 || gp.synth_tile == 256, "synthesis tile mismatch");
+  auto spin0 = [&](auto kernel) {
+    kernel<<<nitems, 128, 0, st>>>(gp.items, gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff,
+                                   cp.alpha, cp.seed, A, ncA, comp0, job.lmax, phase, ncm,
+                                   pcomp0, job.mmax + 1);
+  };
+  auto spins = [&](auto kernel) {
+    kernel<<<nitems, 128, 0, st>>>(gp.items, gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff,
+                                   cp.alpha, cp.beta, cp.seed, cp.seed_exp, cp.spin, A, ncA,
+                                   comp0, job.lmax, phase, ncm, pcomp0, job.mmax + 1);
+  };
+  auto width = [&](auto r) {
+    constexpr int RV = decltype(r)::value;
+    if (job.spin == 0 && !deriv) {
+      if (nt == 1) spin0(synth_spin0_kernel<1, RV>);
+      else if (nt == 2) spin0(synth_spin0_kernel<2, RV>);
+      else spin0(synth_spin0_kernel<4, RV>);
+    } else if (deriv) {
+      if (nt == 1) spins(synth_spin_kernel<1, RV, true>);
+      else spins(synth_spin_kernel<2, RV, true>);
     } else {
-      if (nt == 1) SHT_SS(1, false);
-      else SHT_SS(2, false);
+      if (nt == 1) spins(synth_spin_kernel<1, RV, false>);
+      else spins(synth_spin_kernel<2, RV, false>);
     }
-#undef SHT_SS
-  }
+  };
+  if (gp.synth_tile == 128) width(std::integral_constant<int, 1>{});
+  else width(std::integral_constant<int, 2>{});
   SHT_CUDA(cudaGetLastError());
 }
 
@@ -758,23 +1041,58 @@ void launch_legendre_anal(const JobDesc &job, const GeomPlan &gp, const CoefPlan
                           int ncA, int comp0, cudaStream_t st) {
   const int nblocks = job.mmax + 1;
   ProfScope ps("legendre_anal", st);
+  auto spin0 = [&](auto nt_, auto r_, auto w_) {
+    constexpr int NT = decltype(nt_)::value, R = decltype(r_)::value, W = decltype(w_)::value;
+    auto kernel = anal_spin0_kernel<NT, R, W>;
+    constexpr size_t smem = anal_smem<2 * NT, W>();
+    SHT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    kernel<<<nblocks, 32 * W, smem, st>>>(gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff, cp.alpha,
+                                          cp.seed, phase, ncm, pcomp0, job.lmax, job.mmax + 1,
+                                          Aout, ncA, comp0);
+  };
+  auto spins = [&](auto nt_, auto r_, auto w_) {
+    constexpr int NT = decltype(nt_)::value, R = decltype(r_)::value, W = decltype(w_)::value;
+    auto kernel = anal_spin_kernel<NT, R, W>;
+    constexpr size_t smem = anal_smem<4 * NT, W>();
+    SHT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    kernel<<<nblocks, 32 * W, smem, st>>>(gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff, cp.alpha,
+                                          cp.beta, cp.seed, cp.seed_exp, cp.spin, phase, ncm,
+                                          pcomp0, job.lmax, job.mmax + 1, Aout, ncA, comp0);
+  };
+  using std::integral_constant;
+  constexpr integral_constant<int, 1> c1{};
+  constexpr integral_constant<int, 2> c2{};
+  constexpr integral_constant<int, 4> c4{};
+  constexpr integral_constant<int, 8> c8{};
+  // Shape (R rings per thread, W warps).  More rings per thread share a
+  // reduction and more warps a tile; but one warp walks all l of its m alone, so
+  // with few ring pairs that chain is the kernel's time and smaller R is faster.
+  // Measured with one transform, us, spin 0 / spin 2 (Nside: pairs):
+  //   Nside 64 (128):    R1 W4 8.9 / 15.4   R2 W4 10.7 / 21.1   R4 W4 15.7 / 33.9
+  //   Nside 128 (256):   R1 W4 29.0 / 53.6  R2 W4 20.1 / 41.0   R4 W4 28.5 / 61.7
+  //   Nside 256 (512):   R2 W4 79.9 / 177   R2 W8 58.5 / 144    R4 W4 66.3 / 145
+  //   Nside 512 (1024):  R2 W4 342 / 834    R2 W8 343 / 801     R4 W4 299 / 813
+  //   Nside 1024 (2048): R2 W4 2296 / 5120  R2 W8 2343 / 5437   R4 W4 1767 / 5017
+  // The shape fixes the order of the sums over rings, so it does not depend on
+  // the number of transforms of the pass: a transform's result is the same bits
+  // alone and in any batch.
+  auto shape = [&](auto n, auto f) {
+    if (gp.npairs <= 128) f(n, c1, c4);
+    else if (gp.npairs <= 256) f(n, c2, c4);
+    else if (gp.npairs <= kAnalWidePairs) f(n, c2, c8);
+    else f(n, c4, c4);
+  };
   if (job.spin == 0) {
-#define SHT_A0(NTV)                                                                       \
-  anal_spin0_kernel<NTV, 4><<<nblocks, 128, 0, st>>>(                                     \
-      gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff, cp.alpha, cp.seed, phase, ncm, pcomp0, \
-      job.lmax, job.mmax + 1, Aout, ncA, comp0)
-    if (nt == 1) SHT_A0(1);
-    else if (nt == 2) SHT_A0(2);
-    else SHT_A0(4);
-#undef SHT_A0
+    if (nt == 1) shape(c1, spin0);
+    else if (nt == 2) shape(c2, spin0);
+    else shape(c4, spin0);
+  } else if (nt == 1) {
+    shape(c1, spins);
   } else {
-#define SHT_AS(NTV)                                                                        \
-  anal_spin_kernel<NTV, 2><<<nblocks, 128, 0, st>>>(                                       \
-      gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff, cp.alpha, cp.beta, cp.seed, cp.seed_exp, \
-      cp.spin, phase, ncm, pcomp0, job.lmax, job.mmax + 1, Aout, ncA, comp0)
-    if (nt == 1) SHT_AS(1);
-    else SHT_AS(2);
-#undef SHT_AS
+    SHT_REQUIRE(gp.npairs <= kAnalWidePairs, "analysis pass too wide");
+    if (gp.npairs <= 128) spins(c2, c1, c4);
+    else if (gp.npairs <= 256) spins(c2, c2, c4);
+    else spins(c2, c2, c8);
   }
   SHT_CUDA(cudaGetLastError());
 }

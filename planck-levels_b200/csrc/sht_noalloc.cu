@@ -243,7 +243,7 @@ int alm2map_noalloc(const sharp_geom_info *g, const sharp_alm_info *a, const voi
   launch_coef_tables(cp, st);
   auto *ptr_dev = static_cast<void *const *>(at(o_ptr));
   launch_stage_alm(job, ap, 0, cp, static_cast<double *>(at(o_norm)), ptr_dev, 1,
-                   static_cast<double2 *>(at(o_A)), 1, st);
+                   static_cast<double2 *>(at(o_A)), 1, false, st);
   launch_legendre_synth(job, gp, cp, static_cast<double2 *>(at(o_A)), 1, 0, 1,
                         static_cast<double2 *>(at(o_phase)), 1, 0, st);
   launch_phase2ring(job, gp, 0, static_cast<double2 *>(at(o_phase)), 1, ptr_dev + 1, 1, st);

@@ -1449,7 +1449,8 @@ stage_alm_kernel(int lmax, int nalmptr, const long long *__restrict__ mvstart,
                  long long astride, bool packed, long long alm_lo,
                  const long long *__restrict__ moff, const double *__restrict__ cfac,
                  const double *__restrict__ norm_l, bool use_norm, double norm_m0,
-                 const T *const *__restrict__ alm, double2 *__restrict__ A, int ncA, int lgtl) {
+                 const T *const *__restrict__ alm, double2 *__restrict__ A, int ncA, int lgtl,
+                 bool pm) {
   extern __shared__ double2 tile[];
   const int tl = 1 << lgtl, ld = nalmptr | 1;
   const int m = blockIdx.x;
@@ -1485,7 +1486,12 @@ stage_alm_kernel(int lmax, int nalmptr, const long long *__restrict__ mvstart,
     __syncthreads();
     for (int e = threadIdx.x; e < tl * nalmptr; e += blockDim.x) {
       const int r = e / nalmptr, c = e - r * nalmptr;
-      if (l0 + r < nl) A[(mo + m + l0 + r) * ncA + c] = tile[r * ld + c];
+      double2 v = tile[r * ld + c];
+      if (pm) {   // G - iC in place of G, G + iC in place of C
+        const double2 u = tile[r * ld + (c ^ 1)];
+        v = (c & 1) ? make_double2(u.x - v.y, u.y + v.x) : make_double2(v.x + u.y, v.y - u.x);
+      }
+      if (l0 + r < nl) A[(mo + m + l0 + r) * ncA + c] = v;
     }
     __syncthreads();
   }
@@ -1927,7 +1933,7 @@ static int stage_tile_lg(int nalmptr) {
 
 void launch_stage_alm(const JobDesc &job, const AlmPlan &ap, long long alm_lo,
                       const CoefPlan &cp, const double *norm_l, const void *const *alm_dev,
-                      int nalmptr, double2 *A, int ncA, cudaStream_t st) {
+                      int nalmptr, double2 *A, int ncA, bool pm, cudaStream_t st) {
   const bool use_norm = job.spin > 0 || job.type == SHARP_ALM2MAP_DERIV1;
   const double norm_m0 = (job.flags & SHARP_REAL_HARMONICS) ? kSqrtTwo : 1.0;
   const int blocks = job.mmax + 1;
@@ -1937,11 +1943,11 @@ void launch_stage_alm(const JobDesc &job, const AlmPlan &ap, long long alm_lo,
   if (job.dp)
     stage_alm_kernel<double><<<blocks, 256, smem, st>>>(
         job.lmax, nalmptr, ap.mvstart, ap.stride, ap.packed, alm_lo, cp.d_moff, cp.cfac, norm_l,
-        use_norm, norm_m0, reinterpret_cast<const double *const *>(alm_dev), A, ncA, lg);
+        use_norm, norm_m0, reinterpret_cast<const double *const *>(alm_dev), A, ncA, lg, pm);
   else
     stage_alm_kernel<float><<<blocks, 256, smem, st>>>(
         job.lmax, nalmptr, ap.mvstart, ap.stride, ap.packed, alm_lo, cp.d_moff, cp.cfac, norm_l,
-        use_norm, norm_m0, reinterpret_cast<const float *const *>(alm_dev), A, ncA, lg);
+        use_norm, norm_m0, reinterpret_cast<const float *const *>(alm_dev), A, ncA, lg, pm);
   SHT_CUDA(cudaGetLastError());
 }
 
