@@ -154,6 +154,7 @@ struct CoefPlan {
   double *cfac = nullptr;            // c_l
   double *seed = nullptr;            // spin 0: mfac[m]; spin>0: prefac mantissa
   int *seed_exp = nullptr;           // spin>0: prefac exponent (base 2)
+  double *norm = nullptr;            // spin>0: norm_l, then (spin 1) that of the derivatives
   double2 *mx_coef = nullptr;        // mixed analysis: (alpha_l, c_l 2^30 / b_l), lazily built
   CoefPlan() = default;
   CoefPlan(const CoefPlan &) = delete;
@@ -197,6 +198,17 @@ void launch_mixed_anal(const JobDesc &job, const GeomPlan &gp, CoefPlan &cp,
                        const double2 *phase, int ncm, double2 *Aout, int ncA, int *d_err,
                        cudaStream_t st);
 
+// The device arrays of a job, passed to the kernels by value: no table to
+// upload, and a captured launch keeps its arrays.
+struct PtrList {
+  void *p[2 * kMaxTrans];
+};
+
+// Lets a kernel take `bytes` of dynamic shared memory (static and dynamic
+// together, 48 KB need no leave).
+template <class K>
+inline void allow_smem(K kernel, size_t bytes);
+
 // Kernel launchers (sht_legendre.cu)
 // Ring pairs up to which the spin analysis takes two transforms per pass (above,
 // four rings per thread leave no registers for a second one).
@@ -231,25 +243,25 @@ inline size_t ring_fft_smem_entries(int bufA, int bufB, int mmax, int nmax_compl
 }
 
 void launch_phase2ring(const JobDesc &job, const GeomPlan &gp, long long map_lo,
-                       const double2 *phase, int ncm, void *const *maps_dev, int nmapptr,
+                       const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
                        cudaStream_t st);
 void launch_ring2phase(const JobDesc &job, const GeomPlan &gp, long long map_lo,
-                       const void *const *maps_dev, int nmapptr, double2 *phase, int ncm,
+                       const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
                        cudaStream_t st);
 void launch_phase2ring_direct(const JobDesc &job, const GeomPlan &gp, long long map_lo,
-                              const double2 *phase, int ncm, void *const *maps_dev, int nmapptr,
+                              const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
                               cudaStream_t st);
 void launch_ring2phase_direct(const JobDesc &job, const GeomPlan &gp, long long map_lo,
-                              const void *const *maps_dev, int nmapptr, double2 *phase,
+                              const PtrList &maps_dev, int nmapptr, double2 *phase,
                               int ncm, cudaStream_t st);
 // pm: pairs of components (G, C) are stored as (G - iC, G + iC), the basis of
 // the FP64 spin synthesis.
 void launch_stage_alm(const JobDesc &job, const AlmPlan &ap, long long alm_lo,
-                      const CoefPlan &cp, const double *norm_l, const void *const *alm_dev,
+                      const CoefPlan &cp, const double *norm_l, const PtrList &alm_dev,
                       int nalmptr, double2 *A, int ncA, bool pm, cudaStream_t st);
 void launch_scatter_alm(const JobDesc &job, const AlmPlan &ap, long long alm_lo,
                         const CoefPlan &cp, const double *norm_l, const double *Aout, int ncA,
-                        void *const *alm_dev, int nalmptr, cudaStream_t st);
+                        const PtrList &alm_dev, int nalmptr, cudaStream_t st);
 
 // Launch accounting: every launcher wraps its kernel in a ProfScope, which
 // counts the launch and, when profiling is on, records CUDA events on the
@@ -269,6 +281,12 @@ class ProfScope {
 
 void check_cuda(cudaError_t e, const char *what, const char *file, int line);
 #define SHT_CUDA(call) ::sht::check_cuda((call), #call, __FILE__, __LINE__)
+
+template <class K>
+inline void allow_smem(K kernel, size_t bytes) {
+  if (bytes > 32 * 1024)
+    SHT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+}
 
 // Stream-ordered workspace allocation from the library's own memory pool on
 // the current device (free with cudaFreeAsync, never cudaFree, which leaves

@@ -76,10 +76,30 @@ std::vector<int> factor_fft(int N) {
   return r;
 }
 
+// Content hash of a long array: eight independent lanes of 64-bit words.  Every
+// call hashes its geometry, 393 KB at Nside 2048; a serial byte-wise FNV took
+// most of the host time there (623 us a call, 93 with this).
+uint64_t hash_words(const void *data, size_t n, uint64_t h0) {
+  constexpr uint64_t kMul = 0x9e3779b97f4a7c15ull;
+  const auto *p = static_cast<const unsigned char *>(data);
+  uint64_t h[8];
+  for (int k = 0; k < 8; ++k) h[k] = h0 + kMul * (k + 1);
+  size_t i = 0;
+  for (; i + 64 <= n; i += 64)
+    for (int k = 0; k < 8; ++k) {
+      uint64_t w;
+      std::memcpy(&w, p + i + 8 * k, 8);
+      h[k] = (h[k] ^ w) * kMul;
+      h[k] ^= h[k] >> 32;
+    }
+  const uint64_t tail = fnv1a(p + i, n - i, h0);
+  return fnv1a(h, sizeof(h), tail);
+}
+
 uint64_t hash_geom(const sharp_geom_info *g) {
   uint64_t h = fnv1a(&g->npairs, sizeof(int));
   h = fnv1a(&g->nphmax, sizeof(int), h);
-  if (g->npairs > 0) h = fnv1a(g->pair, sizeof(sharp_ringpair) * g->npairs, h);
+  if (g->npairs > 0) h = hash_words(g->pair, sizeof(sharp_ringpair) * g->npairs, h);
   return h;
 }
 
@@ -89,8 +109,8 @@ uint64_t hash_alm(const sharp_alm_info *a) {
   h = fnv1a(&a->flags, sizeof(int), h);
   h = fnv1a(&a->stride, sizeof(ptrdiff_t), h);
   if (a->nm > 0) {
-    h = fnv1a(a->mval, sizeof(int) * a->nm, h);
-    h = fnv1a(a->mvstart, sizeof(ptrdiff_t) * a->nm, h);
+    h = hash_words(a->mval, sizeof(int) * a->nm, h);
+    h = hash_words(a->mvstart, sizeof(ptrdiff_t) * a->nm, h);
   }
   return h;
 }
@@ -510,6 +530,15 @@ CoefPlan *get_coef_plan(int lmax, int mmax, int spin, cudaStream_t st) {
     spin_prefactor(lmax, mmax, spin, mant, ex);
     cp->seed = dev_upload(mant, st);
     cp->seed_exp = dev_upload(ex, st);
+    // norm_l (libsharp/sharp_ylmgen_c.c:200-232)
+    std::vector<double> norm(size_t(lmax + 1) * (spin == 1 ? 2 : 1));
+    const double spinsign = (spin & 1) ? 1.0 : -1.0;
+    for (int l = 0; l <= lmax; ++l)
+      norm[l] = (l < spin) ? 0. : spinsign * 0.5 * std::sqrt((2 * l + 1) / (4 * M_PI));
+    if (spin == 1)
+      for (int l = 0; l <= lmax; ++l)
+        norm[lmax + 1 + l] = (l < 1) ? 0. : 0.5 * std::sqrt(l * (l + 1.) * (2 * l + 1.) / (4 * M_PI));
+    cp->norm = dev_upload(norm, st);
   } else {
     std::vector<double> mfac(mmax + 1);
     mfac[0] = 0.2820947917738781434740397257803862929220;  // 1/sqrt(4 pi)
@@ -801,27 +830,15 @@ void execute_impl(sharp_jobtype type_in, int spin, void *alm, void *map,
   void **alm_in = static_cast<void **>(alm);
   void **map_in = static_cast<void **>(map);
 
-  // norm_l (libsharp/sharp_ylmgen_c.c:200-232)
-  std::vector<double> norm(job.lmax + 1, 1.0);
-  if (deriv) {
-    for (int l = 0; l <= job.lmax; ++l)
-      norm[l] = (l < 1) ? 0. : 0.5 * std::sqrt(l * (l + 1.) * (2 * l + 1.) / (4 * M_PI));
-  } else if (spin > 0) {
-    double spinsign = -1.0;
-    if (spin & 1) spinsign = -spinsign;
-    for (int l = 0; l <= job.lmax; ++l)
-      norm[l] = (l < spin) ? 0. : spinsign * 0.5 * std::sqrt((2 * l + 1) / (4 * M_PI));
-  }
-  DevBuf d_norm(sizeof(double) * norm.size(), st);
-  SHT_CUDA(cudaMemcpyAsync(d_norm.p, norm.data(), sizeof(double) * norm.size(),
-                           cudaMemcpyHostToDevice, st));
+  const double *norm = deriv ? cp->norm + (job.lmax + 1) : cp->norm;   // unused at spin 0
 
   // device views of the user arrays
   const size_t esz_map = (job.dp ? 8 : 4) * (no_fft ? 2 : 1);
   const size_t esz_alm = (job.dp ? 8 : 4) * (ap->packed ? 1 : 2);
   const long long map_n = gp->map_hi - gp->map_lo;
   const long long alm_n = ap->hi - ap->lo;
-  std::vector<void *> dmap(nmapptr), dalm(nalmptr);
+  PtrList maps{}, alms{};
+  void **dmap = maps.p, **dalm = alms.p;
   std::vector<std::unique_ptr<DevBuf>> owned;
   long long map_lo = 0, alm_lo = 0;
   if (device_ptrs) {
@@ -847,15 +864,13 @@ void execute_impl(sharp_jobtype type_in, int spin, void *alm, void *map,
                                  esz_alm * alm_n, cudaMemcpyHostToDevice, st));
     }
   }
-  DevBuf d_mapptr(sizeof(void *) * nmapptr, st), d_almptr(sizeof(void *) * nalmptr, st);
-  SHT_CUDA(cudaMemcpyAsync(d_mapptr.p, dmap.data(), sizeof(void *) * nmapptr,
-                           cudaMemcpyHostToDevice, st));
-  SHT_CUDA(cudaMemcpyAsync(d_almptr.p, dalm.data(), sizeof(void *) * nalmptr,
-                           cudaMemcpyHostToDevice, st));
-
   const size_t phase_bytes = sizeof(double2) * 2 * size_t(mmax + 1) * gp->npairs * ncm;
-  DevBuf d_phase(phase_bytes, st);
-  double2 *phase = d_phase.as<double2>();
+  // workspace: the phase rows and the staged (or summed) a_lm
+  const size_t a_bytes = sizeof(double2) * size_t(cp->total) * ncA;
+  const size_t a_at = (phase_bytes + 255) & ~size_t(255);
+  DevBuf d_work(a_at + a_bytes, st);
+  double2 *phase = d_work.as<double2>();
+  double2 *work_A = reinterpret_cast<double2 *>(d_work.as<char>() + a_at);
   const int ntmax_synth = (spin == 0 && !deriv) ? 4 : 2;
   // FP64 analysis: one transform per launch is fastest per transform (the
   // per-thread phase factors of several transforms cost occupancy): at Nside
@@ -869,21 +884,19 @@ void execute_impl(sharp_jobtype type_in, int spin, void *alm, void *map,
   };
 
   if (!analysis) {
-    DevBuf d_A(sizeof(double2) * size_t(cp->total) * ncA, st);
     const bool mixed = (flags & SHARP_MIXED) && mixed_synth_supported(job);
-    launch_stage_alm(job, *ap, alm_lo, *cp, d_norm.as<double>(),
-                     reinterpret_cast<void *const *>(d_almptr.p), nalmptr, d_A.as<double2>(), ncA,
+    launch_stage_alm(job, *ap, alm_lo, *cp, norm, alms, nalmptr, work_A, ncA,
                      spin > 0 && !deriv && !mixed, st);
     if (mixed) {
       int *d_err = nullptr;
       tc_error_word(&d_err);
-      launch_mixed_synth(job, *gp, *cp, d_A.as<double2>(), ncA, phase, ncm, d_err, st);
+      launch_mixed_synth(job, *gp, *cp, work_A, ncA, phase, ncm, d_err, st);
     } else {
       auto passes = [&](int width) {
         for (int t0 = 0; t0 < ntrans;) {
           const int nt = group(ntrans - t0, width);
-          launch_legendre_synth(job, *gp, *cp, d_A.as<double2>(), ncA, t0 * job.nalm, nt,
-                                phase, ncm, t0 * job.nmaps, st);
+          launch_legendre_synth(job, *gp, *cp, work_A, ncA, t0 * job.nalm, nt, phase, ncm,
+                                t0 * job.nmaps, st);
           t0 += nt;
         }
       };
@@ -895,35 +908,29 @@ void execute_impl(sharp_jobtype type_in, int spin, void *alm, void *map,
       passes(width);
     }
     if (no_fft)
-      launch_phase2ring_direct(job, *gp, map_lo, phase, ncm,
-                               reinterpret_cast<void *const *>(d_mapptr.p), nmapptr, st);
+      launch_phase2ring_direct(job, *gp, map_lo, phase, ncm, maps, nmapptr, st);
     else
-      launch_phase2ring(job, *gp, map_lo, phase, ncm, reinterpret_cast<void *const *>(d_mapptr.p),
-                        nmapptr, st);
+      launch_phase2ring(job, *gp, map_lo, phase, ncm, maps, nmapptr, st);
     if (!device_ptrs && map_n > 0)
       for (int i = 0; i < nmapptr; ++i)
         SHT_CUDA(cudaMemcpyAsync(static_cast<char *>(map_in[i]) + esz_map * map_lo, dmap[i],
                                  esz_map * map_n, cudaMemcpyDeviceToHost, st));
   } else {
     if (no_fft)
-      launch_ring2phase_direct(job, *gp, map_lo,
-                               reinterpret_cast<const void *const *>(d_mapptr.p), nmapptr, phase,
-                               ncm, st);
+      launch_ring2phase_direct(job, *gp, map_lo, maps, nmapptr, phase, ncm, st);
     else
-      launch_ring2phase(job, *gp, map_lo, reinterpret_cast<const void *const *>(d_mapptr.p),
-                        nmapptr, phase, ncm, st);
-    DevBuf d_Aout(sizeof(double2) * size_t(cp->total) * ncA, st);
+      launch_ring2phase(job, *gp, map_lo, maps, nmapptr, phase, ncm, st);
     if ((flags & SHARP_MIXED) && mixed_anal_supported(job)) {
-      SHT_CUDA(cudaMemsetAsync(d_Aout.p, 0, sizeof(double2) * size_t(cp->total) * ncA, st));
+      SHT_CUDA(cudaMemsetAsync(work_A, 0, a_bytes, st));
       int *d_err = nullptr;
       tc_error_word(&d_err);
-      launch_mixed_anal(job, *gp, *cp, phase, ncm, d_Aout.as<double2>(), ncA, d_err, st);
+      launch_mixed_anal(job, *gp, *cp, phase, ncm, work_A, ncA, d_err, st);
     } else {
       auto passes = [&](int width) {
         for (int t0 = 0; t0 < ntrans;) {
           const int nt = group(ntrans - t0, width);
           launch_legendre_anal(job, *gp, *cp, phase, ncm, t0 * job.nmaps, nt,
-                               d_Aout.as<double>(), ncA, t0 * job.nalm, st);
+                               reinterpret_cast<double *>(work_A), ncA, t0 * job.nalm, st);
           t0 += nt;
         }
       };
@@ -935,8 +942,8 @@ void execute_impl(sharp_jobtype type_in, int spin, void *alm, void *map,
                             ntmax_anal, passes, [] {}, st);
       passes(width);
     }
-    launch_scatter_alm(job, *ap, alm_lo, *cp, d_norm.as<double>(), d_Aout.as<double>(), ncA,
-                       reinterpret_cast<void *const *>(d_almptr.p), nalmptr, st);
+    launch_scatter_alm(job, *ap, alm_lo, *cp, norm, reinterpret_cast<double *>(work_A), ncA, alms,
+                       nalmptr, st);
     if (!device_ptrs && alm_n > 0)
       for (int i = 0; i < nalmptr; ++i)
         SHT_CUDA(cudaMemcpyAsync(static_cast<char *>(alm_in[i]) + esz_alm * alm_lo, dalm[i],
@@ -1428,6 +1435,7 @@ GeomPlan::~GeomPlan() {
 CoefPlan::~CoefPlan() {
   dev_free(d_moff); dev_free(alpha); dev_free(beta); dev_free(cfac); dev_free(seed);
   dev_free(seed_exp);
+  dev_free(norm);
   dev_free(mx_coef);
 }
 AlmPlan::~AlmPlan() { dev_free(mvstart); }

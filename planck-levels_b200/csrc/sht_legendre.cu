@@ -1045,7 +1045,7 @@ void launch_legendre_anal(const JobDesc &job, const GeomPlan &gp, const CoefPlan
     constexpr int NT = decltype(nt_)::value, R = decltype(r_)::value, W = decltype(w_)::value;
     auto kernel = anal_spin0_kernel<NT, R, W>;
     constexpr size_t smem = anal_smem<2 * NT, W>();
-    SHT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    allow_smem(kernel, smem);
     kernel<<<nblocks, 32 * W, smem, st>>>(gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff, cp.alpha,
                                           cp.seed, phase, ncm, pcomp0, job.lmax, job.mmax + 1,
                                           Aout, ncA, comp0);
@@ -1054,7 +1054,7 @@ void launch_legendre_anal(const JobDesc &job, const GeomPlan &gp, const CoefPlan
     constexpr int NT = decltype(nt_)::value, R = decltype(r_)::value, W = decltype(w_)::value;
     auto kernel = anal_spin_kernel<NT, R, W>;
     constexpr size_t smem = anal_smem<4 * NT, W>();
-    SHT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    allow_smem(kernel, smem);
     kernel<<<nblocks, 32 * W, smem, st>>>(gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff, cp.alpha,
                                           cp.beta, cp.seed, cp.seed_exp, cp.spin, phase, ncm,
                                           pcomp0, job.lmax, job.mmax + 1, Aout, ncA, comp0);

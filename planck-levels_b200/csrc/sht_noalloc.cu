@@ -241,12 +241,14 @@ int alm2map_noalloc(const sharp_geom_info *g, const sharp_alm_info *a, const voi
                                    static_cast<int *>(at(o_blue2)), int(h.blue2_idx.size()),
                                    st);
   launch_coef_tables(cp, st);
-  auto *ptr_dev = static_cast<void *const *>(at(o_ptr));
-  launch_stage_alm(job, ap, 0, cp, static_cast<double *>(at(o_norm)), ptr_dev, 1,
+  PtrList alms{}, maps{};
+  alms.p[0] = const_cast<void *>(alm);
+  maps.p[0] = map;
+  launch_stage_alm(job, ap, 0, cp, static_cast<double *>(at(o_norm)), alms, 1,
                    static_cast<double2 *>(at(o_A)), 1, false, st);
   launch_legendre_synth(job, gp, cp, static_cast<double2 *>(at(o_A)), 1, 0, 1,
                         static_cast<double2 *>(at(o_phase)), 1, 0, st);
-  launch_phase2ring(job, gp, 0, static_cast<double2 *>(at(o_phase)), 1, ptr_dev + 1, 1, st);
+  launch_phase2ring(job, gp, 0, static_cast<double2 *>(at(o_phase)), 1, maps, 1, st);
   return 0;
 }
 

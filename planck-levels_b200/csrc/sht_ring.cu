@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(1024) phase2ring_kernel(const int *__restrict_
                                   const double2 *__restrict__ wpow2, int P,
                                   const double2 *__restrict__ bhat,
                                   const double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                                  int nbufA, int nbufB, int twcap, T *const *__restrict__ maps,
+                                  int nbufA, int nbufB, int twcap, const __grid_constant__ PtrList maps,
                                   long long map_lo, double2 *__restrict__ gbuf, int npc,
                                   int nitems) {
   extern __shared__ double2 smem[];
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(1024) phase2ring_kernel(const int *__restrict_
   const int p = gb ? pairs[it % npc] : pairs[blockIdx.x];
   const int c = gb ? it / npc : blockIdx.y;
   const int mm = min(mmax, mlim[p]);
-  T *map = maps[c];
+  T *map = static_cast<T *>(maps.p[c]);
   for (int h = 0; h < 2; ++h) {
     const int ring = 2 * p + h;
     const int n = nph[ring];
@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(1024) ring2phase_kernel(const int *__restrict_
                                   const double2 *__restrict__ wpow2, int P,
                                   const double2 *__restrict__ bhat, double2 *__restrict__ phase,
                                   int ncm, int mmax, int flags, int nbufA, int nbufB, int twcap,
-                                  const T *const *__restrict__ maps, long long map_lo,
+                                  const __grid_constant__ PtrList maps, long long map_lo,
                                   double2 *__restrict__ gbuf, int npc, int nitems) {
   extern __shared__ double2 smem[];
   const int ms = mmax + 1;
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(1024) ring2phase_kernel(const int *__restrict_
   const int p = gb ? pairs[it % npc] : pairs[blockIdx.x];
   const int c = gb ? it / npc : blockIdx.y;
   const int mm = min(mmax, mlim[p]);
-  const T *map = maps[c];
+  const T *map = static_cast<const T *>(maps.p[c]);
   for (int h = 0; h < 2; ++h) {
     const int ring = 2 * p + h;
     const int n = nph[ring];
@@ -925,7 +925,7 @@ phase2ring_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const double *__restrict__ phi0, const double *__restrict__ weight,
                        const int *__restrict__ fftidx, const FftDesc *__restrict__ fdesc,
                        const double2 *__restrict__ twiddle, const double2 *__restrict__ phase,
-                       int ncm, int mmax, int flags, T *const *__restrict__ maps,
+                       int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
                        long long map_lo) {
   extern __shared__ double2 smem[];
   __shared__ uint64_t row_full;
@@ -1004,7 +1004,7 @@ phase2ring_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
   __syncthreads();
   pw_fft_rest<N, true>(buf, W, 2 * N);
   // pixels 2j, 2j+1 = Re, Im z_j
-  T *map = maps[c] + (ofs[ring] - map_lo);
+  T *map = static_cast<T *>(maps.p[c]) + (ofs[ring] - map_lo);
 #pragma unroll 4
   for (int s2 = 0; s2 < 16; ++s2) {
     const int j = threadIdx.x + (N / 16) * s2;
@@ -1022,7 +1022,7 @@ ring2phase_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const double *__restrict__ phi0, const double *__restrict__ weight,
                        const int *__restrict__ fftidx, const FftDesc *__restrict__ fdesc,
                        const double2 *__restrict__ twiddle, double2 *__restrict__ phase,
-                       int ncm, int mmax, int flags, const T *const *__restrict__ maps,
+                       int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
                        long long map_lo) {
   extern __shared__ double2 smem[];
   double2 *buf = smem;
@@ -1040,7 +1040,7 @@ ring2phase_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
   const double ph = phi0[ring];
   const bool rot = fabs(ph) >= 1e-14;
   const double2 *W = twiddle + fdesc[fftidx[ring]].tw;
-  const T *map = maps[c] + (ofs[ring] - map_lo);
+  const T *map = static_cast<const T *>(maps.p[c]) + (ofs[ring] - map_lo);
   if (rot) build_shift(slo, shi, mm, -ph);
   load_twshared(twl, twh, W, N + 1);   // W: the table of 2N entries
   // pixels 2j, 2j+1 for j = tid + (N/16) s2: this thread's inputs of the
@@ -1194,7 +1194,7 @@ phase2ring_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const double2 *__restrict__ wpow2, int P,
                        const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                        const double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                       T *const *__restrict__ maps, long long map_lo, int stage_row) {
+                       const __grid_constant__ PtrList maps, long long map_lo, int stage_row) {
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   __shared__ uint64_t row_full;
@@ -1280,7 +1280,7 @@ phase2ring_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
   __syncthreads();
   pb_convolve<M>(buf, wpow2, P, bh);
   // z_j = conj(c_j conv_j): pixels 2j, 2j+1 = Re, Im z_j
-  T *map = maps[c] + (ofs[ring] - map_lo);
+  T *map = static_cast<T *>(maps.p[c]) + (ofs[ring] - map_lo);
   const long long st = stride[ring];
   for (int j = threadIdx.x; j < N; j += NT) {
     const double2 z = cmul(buf[pw_pad(j)], __ldg(cz + j));
@@ -1300,7 +1300,7 @@ ring2phase_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const double2 *__restrict__ wpow2, int P,
                        const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                        double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                       const T *const *__restrict__ maps, long long map_lo) {
+                       const __grid_constant__ PtrList maps, long long map_lo) {
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   double2 *buf = smem;
@@ -1321,7 +1321,7 @@ ring2phase_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                      ((flags & SHARP_REAL_HARMONICS) ? kSqrtTwo : 1.0);
   const double ph = phi0[ring];
   const bool rot = fabs(ph) >= 1e-14;
-  const T *map = maps[c] + (ofs[ring] - map_lo);
+  const T *map = static_cast<const T *>(maps.p[c]) + (ofs[ring] - map_lo);
   const long long st = stride[ring];
   if (rot) build_shift(slo, shi, mm, -ph);
   // x_j c_j, x_j = pixels 2j + i (2j+1), zero on [N, M): for j = tid + NT i
@@ -1378,12 +1378,12 @@ __global__ void phase2ring_direct_kernel(const int *__restrict__ mlim, const int
                                          const int *__restrict__ stride,
                                          const double *__restrict__ weight,
                                          const double2 *__restrict__ phase, int ncm,
-                                         int mmax, int flags, T2 *const *__restrict__ maps,
+                                         int mmax, int flags, const __grid_constant__ PtrList maps,
                                          long long map_lo) {
   const int p = blockIdx.x, c = blockIdx.y;
   const int mm = min(mmax, mlim[p]);
   const bool add = (flags & (SHARP_ADD | SHARP_SUBTRACT)) != 0;
-  T2 *map = maps[c];
+  T2 *map = static_cast<T2 *>(maps.p[c]);
   for (int h = 0; h < 2; ++h) {
     const int ring = 2 * p + h;
     const int n = nph[ring];
@@ -1412,11 +1412,11 @@ __global__ void ring2phase_direct_kernel(const int *__restrict__ mlim, const int
                                          const int *__restrict__ stride,
                                          const double *__restrict__ weight,
                                          double2 *__restrict__ phase, int ncm,
-                                         int mmax, int flags, const T2 *const *__restrict__ maps,
+                                         int mmax, int flags, const __grid_constant__ PtrList maps,
                                          long long map_lo) {
   const int p = blockIdx.x, c = blockIdx.y;
   const int mm = min(mmax, mlim[p]);
-  const T2 *map = maps[c];
+  const T2 *map = static_cast<const T2 *>(maps.p[c]);
   for (int h = 0; h < 2; ++h) {
     const int ring = 2 * p + h;
     const int n = nph[ring];
@@ -1449,7 +1449,7 @@ stage_alm_kernel(int lmax, int nalmptr, const long long *__restrict__ mvstart,
                  long long astride, bool packed, long long alm_lo,
                  const long long *__restrict__ moff, const double *__restrict__ cfac,
                  const double *__restrict__ norm_l, bool use_norm, double norm_m0,
-                 const T *const *__restrict__ alm, double2 *__restrict__ A, int ncA, int lgtl,
+                 const __grid_constant__ PtrList alm, double2 *__restrict__ A, int ncA, int lgtl,
                  bool pm) {
   extern __shared__ double2 tile[];
   const int tl = 1 << lgtl, ld = nalmptr | 1;
@@ -1463,7 +1463,7 @@ stage_alm_kernel(int lmax, int nalmptr, const long long *__restrict__ mvstart,
       const int l = m + l0 + r;
       double2 v = make_double2(0.0, 0.0);
       if (l <= lmax) {
-        const T *a = alm[c];
+        const T *a = static_cast<const T *>(alm.p[c]);
         if (packed) {
           if (m == 0) {
             v.x = double(a[base + l * astride - alm_lo]);
@@ -1504,7 +1504,7 @@ scatter_alm_kernel(int lmax, int nalmptr, const long long *__restrict__ mvstart,
                    const long long *__restrict__ moff, const double *__restrict__ cfac,
                    const double *__restrict__ norm_l, bool use_norm, double norm_m0, double sgn,
                    bool add, const double *__restrict__ Aout, int ncA,
-                   T *const *__restrict__ alm, int lgtl) {
+                   const __grid_constant__ PtrList alm, int lgtl) {
   extern __shared__ double2 tile[];
   const int tl = 1 << lgtl, ld = nalmptr | 1;
   const int m = blockIdx.x;
@@ -1526,7 +1526,7 @@ scatter_alm_kernel(int lmax, int nalmptr, const long long *__restrict__ mvstart,
       double f = cfac[mo + l] * sgn;
       if (use_norm) f *= norm_l[l];
       double vr = v.x * f, vi = v.y * f;
-      T *a = alm[c];
+      T *a = static_cast<T *>(alm.p[c]);
       if (m == 0) {
         vr *= norm_m0;
         if (packed) {
@@ -1699,16 +1699,16 @@ FftLaunch plan_fft_launch(const GeomPlan &gp, int cls, int mmax, int ncomp, cuda
 
 template <typename T>
 void phase2ring_class(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
-                      const double2 *phase, int ncm, void *const *maps_dev, int nmapptr,
+                      const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
                       cudaStream_t st) {
   const FftLaunch L = plan_fft_launch(gp, cls, job.mmax, nmapptr, st);
   auto k = phase2ring_kernel<T>;
-  SHT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(L.smem)));
+  allow_smem(k, L.smem);
   k<<<L.grid, L.thr, L.smem, st>>>(gp.cls_pairs + gp.cls_start[cls], gp.mlim, gp.nph, gp.ofs,
                                    gp.stride, gp.phi0, gp.weight, gp.fft, gp.fdesc, gp.twiddle,
                                    gp.wpow2, gp.P, gp.bhat, phase, ncm, job.mmax, job.flags,
                                    gp.cls_bufA[cls], gp.cls_bufB[cls], fft_twcap(gp),
-                                   reinterpret_cast<T *const *>(maps_dev), map_lo, L.gbuf, L.npc,
+                                   maps_dev, map_lo, L.gbuf, L.npc,
                                    L.nitems);
   SHT_CUDA(cudaGetLastError());
   if (L.gbuf) SHT_CUDA(cudaFreeAsync(L.gbuf, st));
@@ -1716,16 +1716,16 @@ void phase2ring_class(const JobDesc &job, const GeomPlan &gp, int cls, long long
 
 template <typename T>
 void ring2phase_class(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
-                      const void *const *maps_dev, int nmapptr, double2 *phase, int ncm,
+                      const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
                       cudaStream_t st) {
   const FftLaunch L = plan_fft_launch(gp, cls, job.mmax, nmapptr, st);
   auto k = ring2phase_kernel<T>;
-  SHT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(L.smem)));
+  allow_smem(k, L.smem);
   k<<<L.grid, L.thr, L.smem, st>>>(gp.cls_pairs + gp.cls_start[cls], gp.mlim, gp.nph, gp.ofs,
                                    gp.stride, gp.phi0, gp.weight, gp.fft, gp.fdesc, gp.twiddle,
                                    gp.wpow2, gp.P, gp.bhat, phase, ncm, job.mmax, job.flags,
                                    gp.cls_bufA[cls], gp.cls_bufB[cls], fft_twcap(gp),
-                                   reinterpret_cast<const T *const *>(maps_dev), map_lo, L.gbuf,
+                                   maps_dev, map_lo, L.gbuf,
                                    L.npc, L.nitems);
   SHT_CUDA(cudaGetLastError());
   if (L.gbuf) SHT_CUDA(cudaFreeAsync(L.gbuf, st));
@@ -1741,36 +1741,36 @@ size_t pow2_smem(int N, int mmax) {
 
 template <typename T, int N>
 void phase2ring_pow2(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
-                     const double2 *phase, int ncm, void *const *maps_dev, int nmapptr,
+                     const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
                      cudaStream_t st) {
   auto k = phase2ring_pow2_kernel<T, N>;
   const size_t smem = pow2_smem(N, job.mmax);
-  SHT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  allow_smem(k, smem);
   k<<<dim3(2 * gp.pw_count[cls], nmapptr), N / 16, smem, st>>>(
       gp.pw_pairs + gp.pw_start[cls], gp.mlim, gp.nph, gp.ofs, gp.phi0, gp.weight, gp.fft,
       gp.fdesc, gp.twiddle, phase, ncm, job.mmax, job.flags,
-      reinterpret_cast<T *const *>(maps_dev), map_lo);
+      maps_dev, map_lo);
   SHT_CUDA(cudaGetLastError());
 }
 
 template <typename T, int N>
 void ring2phase_pow2(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
-                     const void *const *maps_dev, int nmapptr, double2 *phase, int ncm,
+                     const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
                      cudaStream_t st) {
   auto k = ring2phase_pow2_kernel<T, N>;
   // plus the twiddle slices of the unpacking
   const size_t smem = pow2_smem(N, job.mmax) + sizeof(double2) * (kTwLo + N / kTwLo + 1);
-  SHT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  allow_smem(k, smem);
   k<<<dim3(2 * gp.pw_count[cls], nmapptr), N / 16, smem, st>>>(
       gp.pw_pairs + gp.pw_start[cls], gp.mlim, gp.nph, gp.ofs, gp.phi0, gp.weight, gp.fft,
       gp.fdesc, gp.twiddle, phase, ncm, job.mmax, job.flags,
-      reinterpret_cast<const T *const *>(maps_dev), map_lo);
+      maps_dev, map_lo);
   SHT_CUDA(cudaGetLastError());
 }
 
 template <typename T, int M>
 void phase2ring_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
-                     const double2 *phase, int ncm, void *const *maps_dev, int nmapptr,
+                     const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
                      cudaStream_t st) {
   auto k = phase2ring_blue_kernel<T, M>;
   // the phase row is staged in shared memory where that keeps the CTAs per
@@ -1779,31 +1779,31 @@ void phase2ring_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long 
   const size_t with_row = base + sizeof(double2) * (job.mmax + 1);
   const int stage_row = (M == 8192 && with_row + 1024 <= 227 * 1024) ? 1 : 0;
   const size_t smem = stage_row ? with_row : base;
-  SHT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  allow_smem(k, smem);
   k<<<dim3(2 * gp.pb_count[cls], nmapptr), M / 16, smem, st>>>(
       gp.pb_pairs + gp.pb_start[cls], gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.weight,
       gp.fft, gp.fdesc, gp.twiddle, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase, ncm, job.mmax,
-      job.flags, reinterpret_cast<T *const *>(maps_dev), map_lo, stage_row);
+      job.flags, maps_dev, map_lo, stage_row);
   SHT_CUDA(cudaGetLastError());
 }
 
 template <typename T, int M>
 void ring2phase_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
-                     const void *const *maps_dev, int nmapptr, double2 *phase, int ncm,
+                     const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
                      cudaStream_t st) {
   auto k = ring2phase_blue_kernel<T, M>;
   const size_t smem = pow2_smem(M, job.mmax);
-  SHT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  allow_smem(k, smem);
   k<<<dim3(2 * gp.pb_count[cls], nmapptr), M / 16, smem, st>>>(
       gp.pb_pairs + gp.pb_start[cls], gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.weight,
       gp.fft, gp.fdesc, gp.twiddle, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase, ncm, job.mmax,
-      job.flags, reinterpret_cast<const T *const *>(maps_dev), map_lo);
+      job.flags, maps_dev, map_lo);
   SHT_CUDA(cudaGetLastError());
 }
 
 template <typename T>
 void phase2ring_pow2_classes(const JobDesc &job, const GeomPlan &gp, long long map_lo,
-                             const double2 *phase, int ncm, void *const *maps_dev, int nmapptr,
+                             const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
                              cudaStream_t st) {
   for (int c = 0; c < int(gp.pw_N.size()); ++c) {
     if (gp.pw_count[c] == 0) continue;
@@ -1827,7 +1827,7 @@ void phase2ring_pow2_classes(const JobDesc &job, const GeomPlan &gp, long long m
 
 template <typename T>
 void ring2phase_pow2_classes(const JobDesc &job, const GeomPlan &gp, long long map_lo,
-                             const void *const *maps_dev, int nmapptr, double2 *phase, int ncm,
+                             const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
                              cudaStream_t st) {
   for (int c = 0; c < int(gp.pw_N.size()); ++c) {
     if (gp.pw_count[c] == 0) continue;
@@ -1852,7 +1852,7 @@ void ring2phase_pow2_classes(const JobDesc &job, const GeomPlan &gp, long long m
 }  // namespace
 
 void launch_phase2ring(const JobDesc &job, const GeomPlan &gp, long long map_lo,
-                       const double2 *phase, int ncm, void *const *maps_dev, int nmapptr,
+                       const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
                        cudaStream_t st) {
   ProfScope ps("ring_synth", st);
   if (job.dp)
@@ -1869,7 +1869,7 @@ void launch_phase2ring(const JobDesc &job, const GeomPlan &gp, long long map_lo,
 }
 
 void launch_ring2phase(const JobDesc &job, const GeomPlan &gp, long long map_lo,
-                       const void *const *maps_dev, int nmapptr, double2 *phase, int ncm,
+                       const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
                        cudaStream_t st) {
   ProfScope ps("ring_anal", st);
   if (job.dp)
@@ -1886,7 +1886,7 @@ void launch_ring2phase(const JobDesc &job, const GeomPlan &gp, long long map_lo,
 }
 
 void launch_phase2ring_direct(const JobDesc &job, const GeomPlan &gp, long long map_lo,
-                              const double2 *phase, int ncm, void *const *maps_dev, int nmapptr,
+                              const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
                               cudaStream_t st) {
   if (gp.npairs == 0) return;
   dim3 grid(gp.npairs, nmapptr);
@@ -1894,16 +1894,16 @@ void launch_phase2ring_direct(const JobDesc &job, const GeomPlan &gp, long long 
   if (job.dp)
     phase2ring_direct_kernel<double2><<<grid, 128, 0, st>>>(
         gp.mlim, gp.nph, gp.ofs, gp.stride, gp.weight, phase, ncm, job.mmax,
-        job.flags, reinterpret_cast<double2 *const *>(maps_dev), map_lo);
+        job.flags, maps_dev, map_lo);
   else
     phase2ring_direct_kernel<float2><<<grid, 128, 0, st>>>(
         gp.mlim, gp.nph, gp.ofs, gp.stride, gp.weight, phase, ncm, job.mmax,
-        job.flags, reinterpret_cast<float2 *const *>(maps_dev), map_lo);
+        job.flags, maps_dev, map_lo);
   SHT_CUDA(cudaGetLastError());
 }
 
 void launch_ring2phase_direct(const JobDesc &job, const GeomPlan &gp, long long map_lo,
-                              const void *const *maps_dev, int nmapptr, double2 *phase,
+                              const PtrList &maps_dev, int nmapptr, double2 *phase,
                               int ncm, cudaStream_t st) {
   if (gp.npairs == 0) return;
   dim3 grid(gp.npairs, nmapptr);
@@ -1911,11 +1911,11 @@ void launch_ring2phase_direct(const JobDesc &job, const GeomPlan &gp, long long 
   if (job.dp)
     ring2phase_direct_kernel<double2><<<grid, 128, 0, st>>>(
         gp.mlim, gp.nph, gp.ofs, gp.stride, gp.weight, phase, ncm, job.mmax,
-        job.flags, reinterpret_cast<const double2 *const *>(maps_dev), map_lo);
+        job.flags, maps_dev, map_lo);
   else
     ring2phase_direct_kernel<float2><<<grid, 128, 0, st>>>(
         gp.mlim, gp.nph, gp.ofs, gp.stride, gp.weight, phase, ncm, job.mmax,
-        job.flags, reinterpret_cast<const float2 *const *>(maps_dev), map_lo);
+        job.flags, maps_dev, map_lo);
   SHT_CUDA(cudaGetLastError());
 }
 
@@ -1932,7 +1932,7 @@ static int stage_tile_lg(int nalmptr) {
 }
 
 void launch_stage_alm(const JobDesc &job, const AlmPlan &ap, long long alm_lo,
-                      const CoefPlan &cp, const double *norm_l, const void *const *alm_dev,
+                      const CoefPlan &cp, const double *norm_l, const PtrList &alm_dev,
                       int nalmptr, double2 *A, int ncA, bool pm, cudaStream_t st) {
   const bool use_norm = job.spin > 0 || job.type == SHARP_ALM2MAP_DERIV1;
   const double norm_m0 = (job.flags & SHARP_REAL_HARMONICS) ? kSqrtTwo : 1.0;
@@ -1943,17 +1943,17 @@ void launch_stage_alm(const JobDesc &job, const AlmPlan &ap, long long alm_lo,
   if (job.dp)
     stage_alm_kernel<double><<<blocks, 256, smem, st>>>(
         job.lmax, nalmptr, ap.mvstart, ap.stride, ap.packed, alm_lo, cp.d_moff, cp.cfac, norm_l,
-        use_norm, norm_m0, reinterpret_cast<const double *const *>(alm_dev), A, ncA, lg, pm);
+        use_norm, norm_m0, alm_dev, A, ncA, lg, pm);
   else
     stage_alm_kernel<float><<<blocks, 256, smem, st>>>(
         job.lmax, nalmptr, ap.mvstart, ap.stride, ap.packed, alm_lo, cp.d_moff, cp.cfac, norm_l,
-        use_norm, norm_m0, reinterpret_cast<const float *const *>(alm_dev), A, ncA, lg, pm);
+        use_norm, norm_m0, alm_dev, A, ncA, lg, pm);
   SHT_CUDA(cudaGetLastError());
 }
 
 void launch_scatter_alm(const JobDesc &job, const AlmPlan &ap, long long alm_lo,
                         const CoefPlan &cp, const double *norm_l, const double *Aout, int ncA,
-                        void *const *alm_dev, int nalmptr, cudaStream_t st) {
+                        const PtrList &alm_dev, int nalmptr, cudaStream_t st) {
   const bool use_norm = job.spin > 0 || job.type == SHARP_ALM2MAP_DERIV1;
   const double norm_m0 = (job.flags & SHARP_REAL_HARMONICS) ? kSqrtHalf : 1.0;
   // SHARP_SUBTRACT: the negated result is added (negation is exact)
@@ -1966,11 +1966,11 @@ void launch_scatter_alm(const JobDesc &job, const AlmPlan &ap, long long alm_lo,
   if (job.dp)
     scatter_alm_kernel<double><<<blocks, 256, smem, st>>>(
         job.lmax, nalmptr, ap.mvstart, ap.stride, ap.packed, alm_lo, cp.d_moff, cp.cfac, norm_l,
-        use_norm, norm_m0, sgn, add, Aout, ncA, reinterpret_cast<double *const *>(alm_dev), lg);
+        use_norm, norm_m0, sgn, add, Aout, ncA, alm_dev, lg);
   else
     scatter_alm_kernel<float><<<blocks, 256, smem, st>>>(
         job.lmax, nalmptr, ap.mvstart, ap.stride, ap.packed, alm_lo, cp.d_moff, cp.cfac, norm_l,
-        use_norm, norm_m0, sgn, add, Aout, ncA, reinterpret_cast<float *const *>(alm_dev), lg);
+        use_norm, norm_m0, sgn, add, Aout, ncA, alm_dev, lg);
   SHT_CUDA(cudaGetLastError());
 }
 

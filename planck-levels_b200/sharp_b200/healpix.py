@@ -65,8 +65,9 @@ def alm_info(lmax: int, mmax: int | None = None) -> AlmInfo:
 
 
 def _f64(t: torch.Tensor) -> torch.Tensor:
-    """Real view of a complex128 tensor (the ABI takes interleaved re/im)."""
-    if t.is_complex():
+    """The interleaved re/im storage of a complex128 tensor (what the ABI takes):
+    the tensor itself where that is its storage."""
+    if t.is_complex() and (t.is_conj() or t.is_neg() or not t.is_contiguous()):
         return torch.view_as_real(t).reshape(-1)
     return t
 
