@@ -65,6 +65,11 @@ struct GeomHost {
   // pairs whose rings run the register Bluestein convolution
   // (blue_ring_length): length pb_M[c], listed at pb_pairs[pb_start[c] ..)
   std::vector<int> pb_M, pb_start, pb_count, pb_pairs;
+  // pairs of the short-ring kernels (short_ring_kind), longest first
+  std::vector<int> ps_pairs;
+  // pairs of odd rings (odd_pair_length): convolution length po_M[c], listed at
+  // po_pairs[po_start[c] ..)
+  std::vector<int> po_M, po_start, po_count, po_pairs;
   long long map_lo = 0, map_hi = 0;
   bool map_covered = false;
 };
@@ -92,12 +97,44 @@ inline int pow2_ring_length(int nph, int stride, int mm) {
 // kernel, one 1024-thread CTA per SM, ran the mixed-radix Stockham passes
 // about twice as slowly per ring as the register convolution).
 constexpr int kRegBluesteinMinN = 1024;
-inline int blue_ring_length(int nph, const FftDesc &d) {
+inline int blue_ring_length(int nph, const FftDesc &d, bool all) {
   if (nph <= 0 || (nph & 1)) return 0;
-  if (!d.blue && d.N <= kRegBluesteinMinN) return 0;
+  if (!all && !d.blue && d.N <= kRegBluesteinMinN) return 0;
   return (d.M == 1024 || d.M == 2048 || d.M == 4096 || d.M == 8192) ? d.M : 0;
 }
-GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin);
+// How the short-ring kernels run an even ring of complex length N, or kNone:
+// directly (N <= 32), by the passes of length L = N (64 .. 512, a power of two),
+// or by a Bluestein convolution of length L (N up to 256).
+enum class ShortKind { kNone, kDirect, kPasses };
+__host__ __device__ inline ShortKind short_ring_kind(int N, int *L, bool *blue) {
+  *L = N;
+  *blue = (N & (N - 1)) != 0;
+  if (N <= 32) return ShortKind::kDirect;
+  if (!*blue) return N <= 512 ? ShortKind::kPasses : ShortKind::kNone;
+  if (N > 256) return ShortKind::kNone;
+  *L = N <= 64 ? 128 : N <= 128 ? 256 : 512;
+  return ShortKind::kPasses;
+}
+// Convolution length M = 256 .. 8192 of the odd-ring kernels for a pair whose
+// rings have n0 and n1 pixels (<= 0: absent), else 0: one odd length of at least
+// 3.  (Rings of one pixel stay in the size classes, which reproduce the
+// reference's fold.)
+inline int odd_pair_length(int n0, int n1) {
+  const int n = n0 > 0 ? n0 : n1;
+  if (n < 3 || !(n & 1) || n > 4096 || (n0 > 0 && n1 > 0 && n0 != n1)) return 0;
+  int M = 256;
+  while (M < 2 * n - 1) M <<= 1;
+  return M;
+}
+inline size_t odd_ring_smem_entries(int M, int mmax) {
+  const int n = M - 1;
+  return size_t(n + (n >> 4) + (n >> 8) + 1) + 2 * size_t(64 + mmax / 64 + 1);
+}
+// registers: every ring that fits goes to the register kernels; false (the
+// allocation-free synthesis, whose tables share a fixed scratch) keeps those
+// that the size classes can take there.
+GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin,
+                         bool registers = true);
 
 // Per-geometry device tables (pairs in internal mlim order).
 struct GeomPlan {
@@ -135,6 +172,15 @@ struct GeomPlan {
   // register-Bluestein classes (see GeomHost)
   std::vector<int> pb_M, pb_start, pb_count;
   int *pb_pairs = nullptr;
+  // pairs of the short-ring kernels (see GeomHost)
+  int *ps_pairs = nullptr;
+  int ps_count = 0;
+  // odd-ring classes (see GeomHost)
+  std::vector<int> po_M, po_start, po_count;
+  int *po_pairs = nullptr;
+  // e^{i m phi0} per ring as two slices (see shift_table_kernel), or null
+  double2 *shift = nullptr;
+  int shift_width = 0;
   long long map_lo = 0, map_hi = 0;  // pixel index extent [lo, hi)
   bool map_covered = false;          // rings tile [lo,hi) exactly
   GeomPlan() = default;
@@ -224,6 +270,7 @@ void launch_legendre_anal(const JobDesc &job, const GeomPlan &gp, const CoefPlan
 // Ring FFT and staging launchers (sht_ring.cu)
 void launch_twiddles(GeomPlan &gp, int ntw, const std::vector<int> &tw_n,
                      const std::vector<int> &tw_off, cudaStream_t st);
+void launch_shift_table(GeomPlan &gp, cudaStream_t st);
 void launch_bluestein_setup(GeomPlan &gp, const GeomHost &h, cudaStream_t st);
 void launch_twiddles_preplaced(double2 *tw, const int *d_n, const int *d_off, int ntab,
                                cudaStream_t st);

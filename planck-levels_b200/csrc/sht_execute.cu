@@ -182,7 +182,8 @@ bool ws_bytes(unsigned long long *reserved, unsigned long long *used) {
 // chirp offsets) and the FFT size classes.  The cached plans and the
 // allocation-free synthesis both build on it.
 // ---------------------------------------------------------------------------
-GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin) {
+GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin,
+                         bool registers) {
   GeomHost h;
   const int np = g->npairs;
   // FP64 synthesis: ring pairs per CTA of 128 threads.  Few pairs: one ring per
@@ -190,7 +191,7 @@ GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin)
   // 37.4 us at spin 0 and 10.8, 25.0, 92.7 at spin 2, against 8.6, 14.6, 41.3
   // and 15.8, 28.8, 98.7 with two); many: two, which share the staged a_lm
   // (Nside 512: 190 and 531 us against 204 and 556)
-  h.synth_tile = np <= 512 ? 128 : 256;
+  h.synth_tile = registers && np <= 512 ? 128 : 256;
   h.npairs = np;
   h.nphmax = g->nphmax;
   std::vector<int> mlim(np);
@@ -261,7 +262,8 @@ GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin)
         while (M < 2 * d.N - 1) { M <<= 1; ++lg; }
         const long long blue_cost = 2ll * ((long long)M * lg + 2ll * d.N);
         d.blue = (d.N > 16 && blue_cost < direct) ? 1 : 0;
-        d.M = M;   // the convolution length, also for rings the register Bluestein takes
+        // the convolution length, also for rings the register Bluestein takes
+        d.M = registers && (d.n & 1) ? std::max(M, 256) : M;
         d.bhat = d.bhat2 = d.chirp = -1;
         h.tw_n.push_back(d.n);
         h.tw_off.push_back(int(h.tw_total));
@@ -300,23 +302,37 @@ GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin)
   // (the same for the register Bluestein kernels, keyed by the convolution
   // length); a length whose buffer and phi0 slices exceed the shared memory
   // of a CTA stays in the size classes
-  std::map<int, std::vector<int>> pw_lists, pb_lists;
-  std::vector<char> is_pw(np, 0);   // 1: power-of-two pair, 2: register Bluestein pair
+  std::map<int, std::vector<int>> pw_lists, pb_lists, po_lists;
+  // 1: power-of-two pair, 2: pair with a register Bluestein convolution
+  std::vector<char> is_pw(np, 0);
   auto fits = [&](int len) {
     return sizeof(double2) * pow2_ring_smem_entries(len, mmax) <= kRingSmemLimit;
   };
   for (int p = 0; p < np; ++p) {
     const int mm = std::min(mmax, h.mlim_sorted[p]);
     int N = -1, M = -1;
+    bool is_short = registers, sblue = false;
     for (int hh = 0; hh < 2; ++hh) {
       const int i = 2 * p + hh;
       if (h.nph[i] <= 0) continue;
+      int len = 0;
+      bool blue = false;
+      is_short = is_short && !(h.nph[i] & 1) &&
+                 short_ring_kind(h.nph[i] / 2, &len, &blue) != ShortKind::kNone;
+      if (is_short && h.nph[i] > 64 && blue) sblue = true;
       const int n = pow2_ring_length(h.nph[i], h.stride[i], mm);
       N = (N < 0 || N == n) ? n : 0;
-      const int b = blue_ring_length(h.nph[i], h.descs[h.fft[i]]);
+      const int b = blue_ring_length(h.nph[i], h.descs[h.fft[i]], registers);
       M = (M < 0 || M == b) ? b : 0;
     }
-    if (N > 0 && fits(N)) {
+    const int odd = registers ? odd_pair_length(h.nph[2 * p], h.nph[2 * p + 1]) : 0;
+    if (odd > 0 && sizeof(double2) * odd_ring_smem_entries(odd, mmax) <= kRingSmemLimit) {
+      po_lists[odd].push_back(p);
+      is_pw[p] = 2;
+    } else if (is_short) {
+      h.ps_pairs.push_back(p);
+      is_pw[p] = sblue ? 2 : 1;
+    } else if (N > 0 && fits(N)) {
       pw_lists[N].push_back(p);
       is_pw[p] = 1;
     } else if (M > 0 && fits(M)) {
@@ -329,6 +345,15 @@ GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin)
     h.pw_start.push_back(int(h.pw_pairs.size()));
     h.pw_count.push_back(int(kv.second.size()));
     h.pw_pairs.insert(h.pw_pairs.end(), kv.second.begin(), kv.second.end());
+  }
+  std::stable_sort(h.ps_pairs.begin(), h.ps_pairs.end(), [&](int a, int b) {
+    return std::max(h.nph[2 * a], h.nph[2 * a + 1]) > std::max(h.nph[2 * b], h.nph[2 * b + 1]);
+  });
+  for (auto &kv : po_lists) {
+    h.po_M.push_back(kv.first);
+    h.po_start.push_back(int(h.po_pairs.size()));
+    h.po_count.push_back(int(kv.second.size()));
+    h.po_pairs.insert(h.po_pairs.end(), kv.second.begin(), kv.second.end());
   }
   for (auto &kv : pb_lists) {
     h.pb_M.push_back(kv.first);
@@ -440,6 +465,12 @@ std::unique_ptr<GeomPlan> build_geom_plan(const sharp_geom_info *g, int lmax, in
   gp->pb_start = h.pb_start;
   gp->pb_count = h.pb_count;
   gp->pb_pairs = dev_upload(h.pb_pairs, st);
+  gp->ps_count = int(h.ps_pairs.size());
+  gp->ps_pairs = dev_upload(h.ps_pairs, st);
+  gp->po_M = h.po_M;
+  gp->po_start = h.po_start;
+  gp->po_count = h.po_count;
+  gp->po_pairs = dev_upload(h.po_pairs, st);
   gp->cth = dev_upload(h.cth, st);
   gp->sth = dev_upload(h.sth, st);
   gp->mlim = dev_upload(h.mlim_sorted, st);
@@ -459,6 +490,10 @@ std::unique_ptr<GeomPlan> build_geom_plan(const sharp_geom_info *g, int lmax, in
   SHT_CUDA(cudaMalloc(&gp->wpow2, sizeof(double2) * gp->P));
   SHT_CUDA(cudaMalloc(&gp->chirp, sizeof(double2) * std::max<long long>(h.chirp_total, 1)));
   launch_bluestein_setup(*gp, h, st);
+  gp->shift_width = 64 + mmax / 64 + 1;
+  SHT_CUDA(cudaMalloc(&gp->shift, sizeof(double2) * std::max<size_t>(2 * size_t(h.npairs), 1) *
+                                      gp->shift_width));
+  launch_shift_table(*gp, st);
   SHT_CUDA(cudaStreamSynchronize(st));
   return gp;
 }
@@ -1429,7 +1464,7 @@ GeomPlan::~GeomPlan() {
   dev_free(mitems);
   dev_free(phi0); dev_free(weight); dev_free(ofs); dev_free(nph); dev_free(stride);
   dev_free(fft); dev_free(fdesc); dev_free(twiddle); dev_free(cls_pairs); dev_free(pw_pairs);
-  dev_free(pb_pairs);
+  dev_free(pb_pairs); dev_free(ps_pairs); dev_free(po_pairs); dev_free(shift);
   dev_free(bhat); dev_free(wpow2); dev_free(chirp);
 }
 CoefPlan::~CoefPlan() {

@@ -87,7 +87,7 @@ int alm2map_noalloc(const sharp_geom_info *g, const sharp_alm_info *a, const voi
   SHT_REQUIRE(mmax <= lmax, "incorrect l_max: must be >= m_max");
 
   // ---- host tables (the same builder as the cached plans) --------------------
-  const GeomHost h = build_geom_host(g, lmax, mmax, 0);
+  const GeomHost h = build_geom_host(g, lmax, mmax, 0, false);
   const int np = h.npairs;
   // every size class must run its FFT buffers in shared memory: the
   // global-scratch variant of the ring kernels allocates workspace

@@ -7,14 +7,20 @@
 // and the SHARP_NO_FFT path); FFT conventions of libfftpack/ls_fft.c:130-212
 // (unnormalised backward transform, FFTPACK half-complex order).
 //
-// Three kernel families, chosen per ring pair when the geometry plan is built:
+// Kernel families, chosen per ring pair when the geometry plan is built:
 //  * power-of-two rings (2N pixels, N = 1024 .. 8192, no alias folding): one
 //    CTA per ring and component, radix-16 passes in registers
 //    (phase2ring_pow2_kernel / ring2phase_pow2_kernel);
-//  * long even rings that need a Bluestein convolution of length M = 1024 ..
-//    8192 (the polar HEALPix rings): the same register passes around the
-//    chirp product (phase2ring_blue_kernel / ring2phase_blue_kernel);
-//  * all other rings, in size classes (phase2ring_kernel / ring2phase_kernel),
+//  * other even rings with a Bluestein convolution of length M = 1024 .. 8192
+//    (the long polar HEALPix rings): the same register passes around the chirp
+//    product (phase2ring_blue_kernel / ring2phase_blue_kernel);
+//  * short even rings (N <= 512): one warp per ring and component, all in one
+//    launch (phase2ring_short_kernel / ring2phase_short_kernel);
+//  * odd rings: the two of a pair as one complex Bluestein convolution
+//    (phase2ring_odd_kernel / ring2phase_odd_kernel);
+//  * the rest (pairs of unequal odd lengths, single pixels, rings too long for
+//    shared memory, and the allocation-free synthesis, whose tables share a
+//    fixed scratch) in size classes (phase2ring_kernel / ring2phase_kernel),
 //    described here.
 //
 // Size classes: one CTA owns one (ring pair, component) and runs both
@@ -35,6 +41,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "sht_device.h"
 #include "sht_tc.cuh"   // mbarriers and bulk copies
@@ -458,20 +465,35 @@ __device__ __forceinline__ void store_px(T *p, double v, bool add) {
   else *p = T(v);
 }
 
-// e^{i m phi0} for m <= mm as hi[m >> 6] * lo[m & 63], built per ring in
-// shared memory (about 64 + mm/64 sincos calls instead of mm).
+// e^{i m phi0} for m <= mm as hi[m >> 6] * lo[m & 63].
 constexpr int kShiftLo = 64;
-__device__ void build_shift(double2 *lo, double2 *hi, int mm, double ph) {
-  const int nhi = (mm >> 6) + 1;
+__global__ void shift_table_kernel(const double *__restrict__ phi0, int nhi,
+                                   double2 *__restrict__ tab) {
+  const double ph = phi0[blockIdx.x];
+  double2 *row = tab + size_t(blockIdx.x) * (kShiftLo + nhi);
   for (int t = threadIdx.x; t < kShiftLo + nhi; t += blockDim.x) {
-    double sn, cs;
-    if (t < kShiftLo) {
-      sincos(t * ph, &sn, &cs);
-      lo[t] = make_double2(cs, sn);
+    double2 v;
+    sincos(double(t < kShiftLo ? t : (t - kShiftLo) * kShiftLo) * ph, &v.y, &v.x);
+    row[t] = v;
+  }
+}
+
+// The slices of one ring from the plan's table (launch_shift_table: per ring the 64
+// low entries, then the high ones), conjugated for the analysis; without a
+// table (the allocation-free synthesis) they are formed here.
+__device__ __forceinline__ void load_shift(double2 *lo, double2 *hi, int mm, double ph, bool conj,
+                                           const double2 *__restrict__ tab, int u, int nthreads) {
+  const int nhi = (mm >> 6) + 1;
+  for (int t = u; t < kShiftLo + nhi; t += nthreads) {
+    double2 v;
+    if (tab) {
+      v = __ldg(tab + t);
     } else {
-      sincos(double(t - kShiftLo) * kShiftLo * ph, &sn, &cs);
-      hi[t - kShiftLo] = make_double2(cs, sn);
+      sincos(double(t < kShiftLo ? t : (t - kShiftLo) * kShiftLo) * ph, &v.y, &v.x);
     }
+    if (conj) v.y = -v.y;
+    if (t < kShiftLo) lo[t] = v;
+    else hi[t - kShiftLo] = v;
   }
 }
 
@@ -486,6 +508,7 @@ template <typename T>
 __global__ void __launch_bounds__(1024) phase2ring_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
                                   const int *__restrict__ nph, const long long *__restrict__ ofs,
                                   const int *__restrict__ stride, const double *__restrict__ phi0,
+                       const double2 *__restrict__ shift, int sw,
                                   const double *__restrict__ weight, const int *__restrict__ fftidx,
                                   const FftDesc *__restrict__ fdesc,
                                   const double2 *__restrict__ twiddle,
@@ -532,7 +555,9 @@ __global__ void __launch_bounds__(1024) phase2ring_kernel(const int *__restrict_
     const int half = n / 2;  // highest bin kept (n odd: (n-1)/2)
     const Buf C{bufB}, Ab{bufA};
     const double2 *src = phase + ((long long)(p * ncm + c) * 2 + h) * ms;
-    if (rot) build_shift(slo, shi, mm, ph);
+    if (rot)
+      load_shift(slo, shi, mm, ph, false, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
+                 blockDim.x);
     load_twshared(twlo, twhi, twiddle + d.tw, n);
     __syncthreads();
     // fold phase_m * wgt * e^{i m phi0} into bins 0..half (sharp.c:265-300);
@@ -601,6 +626,7 @@ template <typename T>
 __global__ void __launch_bounds__(1024) ring2phase_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
                                   const int *__restrict__ nph, const long long *__restrict__ ofs,
                                   const int *__restrict__ stride, const double *__restrict__ phi0,
+                       const double2 *__restrict__ shift, int sw,
                                   const double *__restrict__ weight, const int *__restrict__ fftidx,
                                   const FftDesc *__restrict__ fdesc,
                                   const double2 *__restrict__ twiddle,
@@ -640,7 +666,9 @@ __global__ void __launch_bounds__(1024) ring2phase_kernel(const int *__restrict_
     const bool rot = fabs(ph) >= 1e-14;
     const long long o = ofs[ring] - map_lo;
     const long long st = stride[ring];
-    if (rot) build_shift(slo, shi, mm, -ph);
+    if (rot)
+      load_shift(slo, shi, mm, ph, true, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
+                 blockDim.x);
     load_twshared(twlo, twhi, twiddle + d.tw, n);
     const Buf Ab{bufA};
     if ((n & 1) == 0) {
@@ -711,10 +739,12 @@ __host__ __device__ constexpr int pw_entries(int N) {
   return (N - 1) + ((N - 1) >> 4) + ((N - 1) >> 8) + 1;
 }
 __host__ __device__ constexpr int pw_passes16(int N) {
-  return N >= 4096 ? 3 : 2;   // 1024 = 16^2 4, 2048 = 16^2 8, 4096 = 16^3, 8192 = 16^3 2
+  // 64 = 16 4, 128 = 16 8, 256 = 16^2, 512 = 16^2 2, 1024 = 16^2 4, 2048 = 16^2 8,
+  // 4096 = 16^3, 8192 = 16^3 2
+  return N >= 4096 ? 3 : N >= 256 ? 2 : 1;
 }
 __host__ __device__ constexpr int pw_last(int N) {
-  return N / (pw_passes16(N) == 3 ? 4096 : 256);
+  return N / (pw_passes16(N) == 3 ? 4096 : pw_passes16(N) == 2 ? 256 : 16);
 }
 
 // cos(2 pi e / 16), e = 0 .. 15
@@ -763,6 +793,28 @@ __device__ __forceinline__ void dft16(double2 (&v)[16]) {
   }
 }
 
+// v[f] *= w1^f.  TREE: w^f = w^(f/2) w^(f - f/2), a chain of 4 products instead
+// of 14, for the short rings, which run at the latency of their passes (the
+// long ones have other warps to cover it and no registers for it).
+template <bool TREE>
+__device__ __forceinline__ void mul_powers(double2 (&v)[16], double2 w1) {
+  if constexpr (TREE) {
+    double2 w[16];
+    w[1] = w1;
+#pragma unroll
+    for (int f = 2; f < 16; ++f) w[f] = cmul(w[f >> 1], w[f - (f >> 1)]);
+#pragma unroll
+    for (int f = 1; f < 16; ++f) v[f] = cmul(v[f], w[f]);
+  } else {
+    double2 w = w1;
+#pragma unroll
+    for (int f = 1; f < 16; ++f) {
+      v[f] = cmul(v[f], w);
+      if (f < 15) w = cmul(w, w1);
+    }
+  }
+}
+
 // One radix-16 DIF pass of length len (stride len/16) over the buffer;
 // twiddles W_len^(k0 f) from a table W of exp(-2 pi i j/tl), j < tl (a
 // multiple of len), so W_len^e = W[(tl/len) e].
@@ -771,21 +823,15 @@ __device__ __forceinline__ void dft16(double2 (&v)[16]) {
 // is the entry at base + s i (s = len/16, base = (u/s) len + k0, k0 = u mod s).
 template <int N, bool INV>
 __device__ __forceinline__ void pw_pass16_regs(double2 (&v)[16], double2 *buf, int len,
-                                               const double2 *__restrict__ W, int tl) {
+                                               const double2 *__restrict__ W, int tl, int u = threadIdx.x) {
   const int s = len >> 4;
-  const int u = threadIdx.x;
   const int k0 = u & (s - 1);
   const int base = (u / s) * len + k0;
   dft16<INV>(v);
   if (s > 1 && k0 > 0) {
     double2 w1 = __ldg(W + (tl / len) * k0);
     if (INV) w1.y = -w1.y;
-    double2 w = w1;
-#pragma unroll
-    for (int f = 1; f < 16; ++f) {
-      v[f] = cmul(v[f], w);
-      if (f < 15) w = cmul(w, w1);
-    }
+    mul_powers<(N < 1024)>(v, w1);
   }
 #pragma unroll
   for (int f = 0; f < 16; ++f) buf[pw_pad(base + s * f)] = v[f];
@@ -793,9 +839,8 @@ __device__ __forceinline__ void pw_pass16_regs(double2 (&v)[16], double2 *buf, i
 
 template <int N, bool INV, int NIN = 16>
 __device__ __forceinline__ void pw_pass16(double2 *buf, int len, const double2 *__restrict__ W,
-                                          int tl) {
+                                          int tl, int u = threadIdx.x) {
   const int s = len >> 4;
-  const int u = threadIdx.x;
   const int k0 = u & (s - 1);
   const int base = (u / s) * len + k0;
   double2 v[16];
@@ -806,23 +851,27 @@ __device__ __forceinline__ void pw_pass16(double2 *buf, int len, const double2 *
   if (s > 1 && k0 > 0) {
     double2 w1 = __ldg(W + (tl / len) * k0);
     if (INV) w1.y = -w1.y;
-    double2 w = w1;
-#pragma unroll
-    for (int f = 1; f < 16; ++f) {
-      v[f] = cmul(v[f], w);
-      if (f < 15) w = cmul(w, w1);
-    }
+    mul_powers<(N < 1024)>(v, w1);
   }
 #pragma unroll
   for (int f = 0; f < 16; ++f) buf[pw_pad(base + s * f)] = v[f];
 }
 
+// Lanes 0 .. n-1 of a warp.
+__device__ __forceinline__ unsigned sub_warp(int n) { return n >= 32 ? 0xffffffffu : (1u << n) - 1; }
+// Barrier between passes: of the CTA, or of the THREADS first lanes of a warp.
+template <bool WARP, int THREADS>
+__device__ __forceinline__ void pw_sync() {
+  if constexpr (WARP) __syncwarp(sub_warp(THREADS));
+  else __syncthreads();
+}
+
 // The last pass (radix R = 2, 4 or 8 over blocks of R, no twiddles)
 template <int N, int R, bool INV>
-__device__ __forceinline__ void pw_pass_last(double2 *buf) {
+__device__ __forceinline__ void pw_pass_last(double2 *buf, int u = threadIdx.x) {
 #pragma unroll
   for (int q = 0; q < 16 / R; ++q) {
-    const int b = threadIdx.x + (N / 16) * q;
+    const int b = u + (N / 16) * q;
     double2 v[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) v[i] = buf[pw_pad(b * R + i)];
@@ -834,19 +883,19 @@ __device__ __forceinline__ void pw_pass_last(double2 *buf) {
 
 // The passes of pw_fft after the first (which the caller ran from registers
 // with pw_pass16_regs and a __syncthreads).
-template <int N, bool INV>
-__device__ void pw_fft_rest(double2 *buf, const double2 *__restrict__ W, int tl) {
+template <int N, bool INV, bool WARP = false>
+__device__ void pw_fft_rest(double2 *buf, const double2 *__restrict__ W, int tl, int u = threadIdx.x) {
   int len = N >> 4;
 #pragma unroll
   for (int q = 1; q < pw_passes16(N); ++q) {
-    pw_pass16<N, INV>(buf, len, W, tl);
-    __syncthreads();
+    pw_pass16<N, INV>(buf, len, W, tl, u);
+    pw_sync<WARP, N / 16>();
     len >>= 4;
   }
   constexpr int RL = pw_last(N);
   if constexpr (RL > 1) {
-    pw_pass_last<N, RL, INV>(buf);
-    __syncthreads();
+    pw_pass_last<N, RL, INV>(buf, u);
+    pw_sync<WARP, N / 16>();
   }
 }
 
@@ -874,9 +923,8 @@ __device__ void pw_fft(double2 *buf, const double2 *__restrict__ W, int tl) {
 // i >= NOUT are not stored.
 template <int N, int NOUT = 16>
 __device__ __forceinline__ void pw_pass16_back(double2 *buf, int len,
-                                               const double2 *__restrict__ W, int tl) {
+                                               const double2 *__restrict__ W, int tl, int u = threadIdx.x) {
   const int s = len >> 4;
-  const int u = threadIdx.x;
   const int k0 = u & (s - 1);
   const int base = (u / s) * len + k0;
   double2 v[16];
@@ -885,12 +933,7 @@ __device__ __forceinline__ void pw_pass16_back(double2 *buf, int len,
   if (s > 1 && k0 > 0) {
     double2 w1 = __ldg(W + (tl / len) * k0);
     w1.y = -w1.y;
-    double2 w = w1;
-#pragma unroll
-    for (int f = 1; f < 16; ++f) {
-      v[f] = cmul(v[f], w);
-      if (f < 15) w = cmul(w, w1);
-    }
+    mul_powers<(N < 1024)>(v, w1);
   }
   dft16<true>(v);
 #pragma unroll
@@ -922,7 +965,8 @@ template <typename T, int N>
 __global__ void __launch_bounds__(N / 16, pow2_synth_min_blocks(N))
 phase2ring_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
                        const int *__restrict__ nph, const long long *__restrict__ ofs,
-                       const double *__restrict__ phi0, const double *__restrict__ weight,
+                       const double *__restrict__ phi0, const double2 *__restrict__ shift, int sw,
+                       const double *__restrict__ weight,
                        const int *__restrict__ fftidx, const FftDesc *__restrict__ fdesc,
                        const double2 *__restrict__ twiddle, const double2 *__restrict__ phase,
                        int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
@@ -963,7 +1007,9 @@ phase2ring_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
     bulk_g2s(buf, src, uint32_t(16 * (mm + 1)), &row_full);
   }
   if constexpr (kSlices) load_twshared(twl, twh, W, N);   // W: the table of 2N entries
-  if (rot) build_shift(slo, shi, mm, ph);
+  if (rot)
+      load_shift(slo, shi, mm, ph, false, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
+                 blockDim.x);
   // a copy that did not complete within the bounded wait is redone by the
   // threads from global memory (the same values, so a late bulk write
   // changes nothing)
@@ -1019,7 +1065,8 @@ template <typename T, int N>
 __global__ void __launch_bounds__(N / 16)
 ring2phase_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
                        const int *__restrict__ nph, const long long *__restrict__ ofs,
-                       const double *__restrict__ phi0, const double *__restrict__ weight,
+                       const double *__restrict__ phi0, const double2 *__restrict__ shift, int sw,
+                       const double *__restrict__ weight,
                        const int *__restrict__ fftidx, const FftDesc *__restrict__ fdesc,
                        const double2 *__restrict__ twiddle, double2 *__restrict__ phase,
                        int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
@@ -1041,7 +1088,9 @@ ring2phase_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
   const bool rot = fabs(ph) >= 1e-14;
   const double2 *W = twiddle + fdesc[fftidx[ring]].tw;
   const T *map = static_cast<const T *>(maps.p[c]) + (ofs[ring] - map_lo);
-  if (rot) build_shift(slo, shi, mm, -ph);
+  if (rot)
+      load_shift(slo, shi, mm, ph, true, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
+                 blockDim.x);
   load_twshared(twl, twh, W, N + 1);   // W: the table of 2N entries
   // pixels 2j, 2j+1 for j = tid + (N/16) s2: this thread's inputs of the
   // first pass, which runs from registers
@@ -1091,33 +1140,28 @@ ring2phase_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
 // the convolution, pairing k with N-k so that each thread updates its own
 // entries in place.
 // ---------------------------------------------------------------------------
-// c_j from the ring's table exp(-2 pi i e/n): c_j = W[j^2 mod n] (n = 2N)
-__device__ __forceinline__ double2 pb_chirp(const double2 *__restrict__ W, int j, int n) {
-  return __ldg(W + int((unsigned(j) * unsigned(j)) % unsigned(n)));
-}
-
 // In place: natural-order input (upper half zero) -> M times the cyclic
 // convolution with b, natural order, lower half.  W: exp(-2 pi i j/tl).
 // The callers run the first forward pass themselves from registers
 // (pw_pass16_regs on the entries tid + (M/16) i, i < 8, the rest zero,
 // then a __syncthreads); this runs the rest.
-template <int M>
+template <int M, bool WARP = false>
 __device__ void pb_convolve(double2 *buf, const double2 *__restrict__ W, int tl,
-                            const double2 *__restrict__ bh) {
+                            const double2 *__restrict__ bh, int u = threadIdx.x) {
   constexpr int P16 = pw_passes16(M), RL = pw_last(M);
   constexpr int FWD = (RL > 1) ? P16 : P16 - 1;   // radix-16 passes before the product
   int len = M >> 4;
 #pragma unroll
   for (int q = 1; q < FWD; ++q) {
-    pw_pass16<M, false>(buf, len, W, tl);
-    __syncthreads();
+    pw_pass16<M, false>(buf, len, W, tl, u);
+    pw_sync<WARP, M / 16>();
     len >>= 4;
   }
   if constexpr (RL > 1) {
     // last forward pass (radix RL, unit twiddles), product, its inverse
 #pragma unroll
     for (int q = 0; q < 16 / RL; ++q) {
-      const int b = threadIdx.x + (M / 16) * q;
+      const int b = u + (M / 16) * q;
       double2 v[RL];
 #pragma unroll
       for (int i = 0; i < RL; ++i) v[i] = buf[pw_pad(b * RL + i)];
@@ -1130,7 +1174,7 @@ __device__ void pb_convolve(double2 *buf, const double2 *__restrict__ W, int tl,
     }
   } else {
     // the radix-16 pass of length 16 (unit twiddles), product, its inverse
-    const int b = threadIdx.x * 16;
+    const int b = u * 16;
     double2 v[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = buf[pw_pad(b + i)];
@@ -1141,13 +1185,13 @@ __device__ void pb_convolve(double2 *buf, const double2 *__restrict__ W, int tl,
 #pragma unroll
     for (int i = 0; i < 16; ++i) buf[pw_pad(b + i)] = v[i];
   }
-  __syncthreads();
+  pw_sync<WARP, M / 16>();
   len = (RL > 1) ? 16 * RL : 256;
 #pragma unroll
   for (int q = 0; q < FWD; ++q) {
-    if (q == FWD - 1) pw_pass16_back<M, 8>(buf, len, W, tl);
-    else pw_pass16_back<M>(buf, len, W, tl);
-    __syncthreads();
+    if (q == FWD - 1) pw_pass16_back<M, 8>(buf, len, W, tl, u);
+    else pw_pass16_back<M>(buf, len, W, tl, u);
+    pw_sync<WARP, M / 16>();
     len <<= 4;
   }
 }
@@ -1166,10 +1210,11 @@ bluestein_pw_setup_kernel(const FftDesc *__restrict__ fdesc, const int *__restri
   const int N = d.N, n = d.n;
   const long long o = d.bhat2;
   const double2 *W = twiddle + d.tw;
-  for (int j = threadIdx.x; j < N; j += M / 16) chirp[d.chirp + j] = pb_chirp(W, j, n);
+  const TwGlobal Wn{W};
+  for (int j = threadIdx.x; j < N; j += M / 16) chirp[d.chirp + j] = chirp_of(j, n, N, Wn);
   for (int j = threadIdx.x; j < M; j += M / 16) {
     const int jj = j < N ? j : (j > M - N ? M - j : -1);
-    smem[pw_pad(j)] = jj >= 0 ? cconj(pb_chirp(W, jj, n)) : make_double2(0.0, 0.0);
+    smem[pw_pad(j)] = jj >= 0 ? cconj(chirp_of(jj, n, N, Wn)) : make_double2(0.0, 0.0);
   }
   __syncthreads();
   pw_fft<M, false>(smem, wpow2, P);
@@ -1189,6 +1234,7 @@ __global__ void __launch_bounds__(M / 16, blue_min_blocks(M))
 phase2ring_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
                        const int *__restrict__ nph, const long long *__restrict__ ofs,
                        const int *__restrict__ stride, const double *__restrict__ phi0,
+                       const double2 *__restrict__ shift, int sw,
                        const double *__restrict__ weight, const int *__restrict__ fftidx,
                        const FftDesc *__restrict__ fdesc, const double2 *__restrict__ twiddle,
                        const double2 *__restrict__ wpow2, int P,
@@ -1233,7 +1279,9 @@ phase2ring_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
       bulk_g2s(srow, src, uint32_t(16 * (mm + 1)), &row_full);
     }
   }
-  if (rot) build_shift(slo, shi, mm, ph);
+  if (rot)
+      load_shift(slo, shi, mm, ph, false, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
+                 blockDim.x);
   if (stage_row) {
     // a copy that did not complete within the bounded wait is redone by
     // the threads (the same values)
@@ -1295,6 +1343,7 @@ __global__ void __launch_bounds__(M / 16, blue_min_blocks(M))
 ring2phase_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
                        const int *__restrict__ nph, const long long *__restrict__ ofs,
                        const int *__restrict__ stride, const double *__restrict__ phi0,
+                       const double2 *__restrict__ shift, int sw,
                        const double *__restrict__ weight, const int *__restrict__ fftidx,
                        const FftDesc *__restrict__ fdesc, const double2 *__restrict__ twiddle,
                        const double2 *__restrict__ wpow2, int P,
@@ -1323,7 +1372,9 @@ ring2phase_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
   const bool rot = fabs(ph) >= 1e-14;
   const T *map = static_cast<const T *>(maps.p[c]) + (ofs[ring] - map_lo);
   const long long st = stride[ring];
-  if (rot) build_shift(slo, shi, mm, -ph);
+  if (rot)
+      load_shift(slo, shi, mm, ph, true, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
+                 blockDim.x);
   // x_j c_j, x_j = pixels 2j + i (2j+1), zero on [N, M): for j = tid + NT i
   // this thread's inputs of the first forward pass, run from registers
   double2 v[16];
@@ -1365,6 +1416,516 @@ ring2phase_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
     v = cscale(v, wgt);
     if (rot) v = cmul(v, shift_of(slo, shi, m));
     dst[m] = v;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Short even rings (complex length N up to 512): one warp per ring and
+// component, all of them in one launch, so that barriers cost nothing and a
+// ring's time is that of its few passes.  By length (short_ring_kind):
+//  * N <= 32: the sums are formed directly, a pixel or bin per thread;
+//  * N = 64 .. 512 a power of two: the register passes of the long rings;
+//  * other N up to 256: Bluestein convolution of length L = 128, 256 or 512.
+// The passes use L/16 of the threads, the folds and copies all.  With the
+// size-class kernel (a CTA per pair, its rings in turn, sincos of the phase
+// shifts, generic prime passes) the latency of one pair was the kernel's time
+// at Nside 64: 24 us (synthesis), 19 us (analysis) for 127 pairs, now 9.2 and
+// 9.1; Nside 256, lmax 767, three components: 184 us, now 37.
+// ---------------------------------------------------------------------------
+template <typename T>
+struct Vec2;
+template <>
+struct Vec2<double> {
+  using type = double2;
+};
+template <>
+struct Vec2<float> {
+  using type = float2;
+};
+// pixels 2j, 2j+1 of a ring; vec: unit stride and aligned to a pair
+template <typename T>
+__device__ __forceinline__ bool px2_vec(const T *map, long long st) {
+  return st == 1 && (reinterpret_cast<uintptr_t>(map) & (2 * sizeof(T) - 1)) == 0;
+}
+template <typename T>
+__device__ __forceinline__ double2 load_px2(const T *map, int j, long long st, bool vec) {
+  if (vec) {
+    const auto v = reinterpret_cast<const typename Vec2<T>::type *>(map)[j];
+    return make_double2(double(v.x), double(v.y));
+  }
+  return make_double2(double(map[(2 * j) * st]), double(map[(2 * j + 1) * st]));
+}
+template <typename T>
+__device__ __forceinline__ void store_px2(T *map, int j, long long st, bool vec, double a,
+                                          double b, bool add) {
+  if (vec) {
+    auto *q = reinterpret_cast<typename Vec2<T>::type *>(map) + j;
+    typename Vec2<T>::type v;
+    v.x = T(a);
+    v.y = T(b);
+    if (add) {
+      const auto o = *q;
+      v.x += o.x;
+      v.y += o.y;
+    }
+    *q = v;
+  } else {
+    store_px(map + (2 * j) * st, a, add);
+    store_px(map + (2 * j + 1) * st, b, add);
+  }
+}
+
+// Buffer entries of a short ring: the padded passes of up to 512 entries, or the
+// C_k (and their partial sums) of up to 513.
+constexpr int kShortEntries = 552;
+inline size_t short_smem(int mmax) {
+  return sizeof(double2) * (kShortEntries + size_t(kShiftLo) + mmax / kShiftLo + 1);
+}
+
+// C_k, k <= N, of phase2ring_blue_kernel, into at(k); few bins: several threads
+// per bin, their partial sums in buf + N + 1 (N <= 32).
+template <class TM, class AT>
+__device__ __forceinline__ void short_fold(int n, int mm, double2 *buf, const TM &tm,
+                                           const AT &at) {
+  const int N = n >> 1, nb = N + 1;
+  const int parts = nb <= 16 ? 32 / nb : 1;
+  auto sum = [&](int k, int j0, int step) {
+    double2 acc = make_double2(0.0, 0.0);
+    for (int m = k + j0 * n; m <= mm; m += step * n) acc = cadd(acc, tm(m));
+    for (int m = (k == 0 ? n : n - k) + j0 * n; m <= mm; m += step * n)
+      acc = cadd(acc, cconj(tm(m)));
+    return acc;
+  };
+  if (parts == 1) {
+    for (int k = threadIdx.x; k <= N; k += 32) {
+      double2 acc = sum(k, 0, 1);
+      if (k == 0 || k == N) acc.y = 0.0;
+      *at(k) = acc;
+    }
+    return;
+  }
+  const int part = threadIdx.x / nb;
+  if (part < parts) buf[nb + threadIdx.x] = sum(threadIdx.x - part * nb, part, parts);
+  __syncwarp();
+  if (threadIdx.x <= N) {
+    const int k = threadIdx.x;
+    double2 acc = buf[nb + k];
+    for (int q = 1; q < parts; ++q) acc = cadd(acc, buf[nb + q * nb + k]);
+    if (k == 0 || k == N) acc.y = 0.0;
+    *at(k) = acc;
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(32, 16)
+phase2ring_short_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
+                        const int *__restrict__ nph, const long long *__restrict__ ofs,
+                        const int *__restrict__ stride, const double *__restrict__ phi0,
+                        const double2 *__restrict__ shift, int sw,
+                        const double *__restrict__ weight, const int *__restrict__ fftidx,
+                        const FftDesc *__restrict__ fdesc, const double2 *__restrict__ twiddle,
+                        const double2 *__restrict__ wpow2, int P,
+                        const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
+                        const double2 *__restrict__ phase, int ncm, int mmax, int flags,
+                        const __grid_constant__ PtrList maps, long long map_lo) {
+  extern __shared__ double2 smem[];
+  double2 *buf = smem, *slo = buf + kShortEntries, *shi = slo + kShiftLo;
+  const int p = pairs[blockIdx.x >> 1], h = blockIdx.x & 1, c = blockIdx.y;
+  const int ring = 2 * p + h, n = nph[ring];
+  if (n <= 0) return;        // unpaired ring: nothing in this hemisphere
+  const int N = n / 2;
+  const FftDesc &fd = fdesc[fftidx[ring]];
+  const double2 *W = twiddle + fd.tw;     // exp(-2 pi i e/n)
+  const int ms = mmax + 1;
+  const int mm = min(mmax, mlim[p]);
+  const bool add = (flags & (SHARP_ADD | SHARP_SUBTRACT)) != 0;
+  const double wgt = ((flags & SHARP_USE_WEIGHTS) ? weight[ring] : 1.0) *
+                     ((flags & SHARP_REAL_HARMONICS) ? kSqrtHalf : 1.0) *
+                     ((flags & SHARP_SUBTRACT) ? -1.0 : 1.0);
+  const double ph = phi0[ring];
+  const bool rot = fabs(ph) >= 1e-14;
+  const double2 *src = phase + ((long long)(p * ncm + c) * 2 + h) * ms;
+  T *map = static_cast<T *>(maps.p[c]) + (ofs[ring] - map_lo);
+  const long long st = stride[ring];
+  const bool vec = px2_vec(map, st);
+  if (rot) {
+    load_shift(slo, shi, mm, ph, false, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
+               32);
+    __syncwarp();
+  }
+  auto tm = [&](int m) {
+    double2 t = cscale(src[m], wgt);
+    if (rot) t = cmul(t, shift_of(slo, shi, m));
+    return t;
+  };
+  int L;
+  bool blue;
+  if (short_ring_kind(N, &L, &blue) == ShortKind::kDirect) {
+    short_fold(n, mm, buf, tm, [&](int k) { return buf + k; });
+    __syncwarp();
+    // pixel j: C_0 + (-1)^j C_N + 2 sum_{0<k<N} Re(C_k e^{2 pi i j k/n})
+    for (int j = threadIdx.x; j < n; j += 32) {
+      double acc = 0.0;
+      int e = j;
+      for (int k = 1; k < N; ++k) {
+        const double2 w = __ldg(W + e), ck = buf[k];
+        acc = fma(ck.x, w.x, fma(ck.y, w.y, acc));
+        e += j;
+        if (e >= n) e -= n;
+      }
+      store_px(map + j * st, buf[0].x + ((j & 1) ? -buf[N].x : buf[N].x) + 2.0 * acc, add);
+    }
+    return;
+  }
+  short_fold(n, mm, buf, tm, [&](int k) { return buf + pw_pad(k); });
+  __syncwarp();
+  // Z_k as in phase2ring_blue_kernel
+  auto z_at = [&](int k) {
+    const double2 ck = buf[pw_pad(k)], cn = cconj(buf[pw_pad(N - k)]);
+    const double2 sm = cadd(ck, cn), df = csub(ck, cn);
+    const double2 w = __ldg(W + k);
+    return cadd(sm, cmul(make_double2(w.y, w.x), df));   // i conj(w)
+  };
+  auto convolve = [&](auto len) {
+    constexpr int LV = decltype(len)::value, TPR = LV / 16;
+    const double2 *cz = chirp + fd.chirp;   // c_j, j < N
+    const int u = threadIdx.x;
+    double2 v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int k = u + TPR * i;
+      v[i] = make_double2(0.0, 0.0);
+      if (i < 8 && u < TPR && k < N) v[i] = cmul(cconj(z_at(k)), __ldg(cz + k));
+    }
+    __syncwarp();
+    if (u < TPR) pw_pass16_regs<LV, false>(v, buf, LV, wpow2, P, u);
+    __syncwarp();
+    if (u < TPR) pb_convolve<LV, true>(buf, wpow2, P, bhat + fd.bhat2, u);
+    __syncwarp();
+    for (int j = u; j < N; j += 32) {
+      const double2 z = cmul(buf[pw_pad(j)], __ldg(cz + j));
+      store_px2(map, j, st, vec, z.x, -z.y, add);
+    }
+  };
+  auto passes = [&](auto len) {
+    constexpr int LV = decltype(len)::value, TPR = LV / 16;
+    const int u = threadIdx.x;
+    double2 v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = u < TPR ? z_at(u + TPR * i) : make_double2(0.0, 0.0);
+    __syncwarp();
+    if (u < TPR) {
+      pw_pass16_regs<LV, true>(v, buf, LV, W, 2 * LV, u);
+      __syncwarp(sub_warp(TPR));
+      pw_fft_rest<LV, true, true>(buf, W, 2 * LV, u);
+    }
+    __syncwarp();
+    for (int j = u; j < N; j += 32) {
+      const double2 z = buf[pw_pad(pw_pos<LV>(j))];
+      store_px2(map, j, st, vec, z.x, z.y, add);
+    }
+  };
+  using std::integral_constant;
+  if (blue) {
+    if (L == 128) convolve(integral_constant<int, 128>{});
+    else if (L == 256) convolve(integral_constant<int, 256>{});
+    else convolve(integral_constant<int, 512>{});
+  } else {
+    if (L == 64) passes(integral_constant<int, 64>{});
+    else if (L == 128) passes(integral_constant<int, 128>{});
+    else if (L == 256) passes(integral_constant<int, 256>{});
+    else passes(integral_constant<int, 512>{});
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(32, 16)
+ring2phase_short_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
+                        const int *__restrict__ nph, const long long *__restrict__ ofs,
+                        const int *__restrict__ stride, const double *__restrict__ phi0,
+                        const double2 *__restrict__ shift, int sw,
+                        const double *__restrict__ weight, const int *__restrict__ fftidx,
+                        const FftDesc *__restrict__ fdesc, const double2 *__restrict__ twiddle,
+                        const double2 *__restrict__ wpow2, int P,
+                        const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
+                        double2 *__restrict__ phase, int ncm, int mmax, int flags,
+                        const __grid_constant__ PtrList maps, long long map_lo) {
+  extern __shared__ double2 smem[];
+  double2 *buf = smem, *slo = buf + kShortEntries, *shi = slo + kShiftLo;
+  const int p = pairs[blockIdx.x >> 1], h = blockIdx.x & 1, c = blockIdx.y;
+  const int ring = 2 * p + h, n = nph[ring];
+  if (n <= 0) return;
+  const int N = n / 2;
+  const FftDesc &fd = fdesc[fftidx[ring]];
+  const double2 *W = twiddle + fd.tw;
+  const int ms = mmax + 1;
+  const int mm = min(mmax, mlim[p]);
+  const double wgt = ((flags & SHARP_USE_WEIGHTS) ? weight[ring] : 1.0) *
+                     ((flags & SHARP_REAL_HARMONICS) ? kSqrtTwo : 1.0);
+  const double ph = phi0[ring];
+  const bool rot = fabs(ph) >= 1e-14;
+  const T *map = static_cast<const T *>(maps.p[c]) + (ofs[ring] - map_lo);
+  const long long st = stride[ring];
+  const bool vec = px2_vec(map, st);
+  double2 *dst = phase + ((long long)(p * ncm + c) * 2 + h) * ms;
+  if (rot)
+    load_shift(slo, shi, mm, ph, true, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
+               32);
+  // phase_m = X_{m mod n} (conjugated above N) wgt e^{-i m phi0}, m <= mm
+  auto write = [&](const auto &x_at) {
+    for (int m = threadIdx.x; m <= mm; m += 32) {
+      const int idx = m % n;
+      const int k = idx <= N ? idx : n - idx;
+      double2 x = x_at(k);
+      if (k == 0 || k == N) x.y = 0.0;   // DC and Nyquist are real
+      if (idx > N) x.y = -x.y;
+      x = cscale(x, wgt);
+      if (rot) x = cmul(x, shift_of(slo, shi, m));
+      dst[m] = x;
+    }
+  };
+  int L;
+  bool blue;
+  const int u = threadIdx.x;
+  if (short_ring_kind(N, &L, &blue) == ShortKind::kDirect) {
+    double *px = reinterpret_cast<double *>(buf);
+    for (int j = u; j < n; j += 32) px[j] = double(map[j * st]);
+    double2 *X = buf + 32;   // n <= 64 pixels before it
+    __syncwarp();
+    for (int k = u; k <= N; k += 32) {
+      double2 acc = make_double2(0.0, 0.0);
+      int e = 0;
+      for (int j = 0; j < n; ++j) {
+        const double2 w = __ldg(W + e);
+        acc.x = fma(px[j], w.x, acc.x);
+        acc.y = fma(px[j], w.y, acc.y);
+        e += k;
+        if (e >= n) e -= n;
+      }
+      X[k] = acc;
+    }
+    __syncwarp();
+    write([&](int k) { return X[k]; });
+    return;
+  }
+  // X_k from Z_k, Z_{N-k} (Z_N = Z_0) as in ring2phase_blue_kernel
+  auto twist = [&](double2 zk, double2 zn, int k) {
+    zn = cconj(zn);
+    const double2 sm = cadd(zk, zn), df = csub(zk, zn);
+    const double2 w = __ldg(W + k);
+    return cscale(cadd(sm, cmul(make_double2(w.y, -w.x), df)), 0.5);   // -i w
+  };
+  auto convolve = [&](auto len) {
+    constexpr int LV = decltype(len)::value, TPR = LV / 16;
+    const double2 *cz = chirp + fd.chirp;
+    double2 v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int j = u + TPR * i;
+      v[i] = make_double2(0.0, 0.0);
+      if (i < 8 && u < TPR && j < N) v[i] = cmul(load_px2(map, j, st, vec), __ldg(cz + j));
+    }
+    if (u < TPR) {
+      pw_pass16_regs<LV, false>(v, buf, LV, wpow2, P, u);
+      __syncwarp(sub_warp(TPR));
+      pb_convolve<LV, true>(buf, wpow2, P, bhat + fd.bhat2, u);
+    }
+    __syncwarp();
+    auto z_at = [&](int k) {
+      const int kk = k == N ? 0 : k;
+      return cmul(buf[pw_pad(kk)], __ldg(cz + kk));
+    };
+    write([&](int k) { return twist(z_at(k), z_at(N - k), k); });
+  };
+  auto passes = [&](auto len) {
+    constexpr int LV = decltype(len)::value, TPR = LV / 16;
+    double2 v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      v[i] = u < TPR ? load_px2(map, u + TPR * i, st, vec) : make_double2(0.0, 0.0);
+    if (u < TPR) {
+      pw_pass16_regs<LV, false>(v, buf, LV, W, 2 * LV, u);
+      __syncwarp(sub_warp(TPR));
+      pw_fft_rest<LV, false, true>(buf, W, 2 * LV, u);
+    }
+    __syncwarp();
+    auto z_at = [&](int k) { return buf[pw_pad(pw_pos<LV>(k == N ? 0 : k))]; };
+    write([&](int k) { return twist(z_at(k), z_at(N - k), k); });
+  };
+  using std::integral_constant;
+  if (blue) {
+    if (L == 128) convolve(integral_constant<int, 128>{});
+    else if (L == 256) convolve(integral_constant<int, 256>{});
+    else convolve(integral_constant<int, 512>{});
+  } else {
+    if (L == 64) passes(integral_constant<int, 64>{});
+    else if (L == 128) passes(integral_constant<int, 128>{});
+    else if (L == 256) passes(integral_constant<int, 256>{});
+    else passes(integral_constant<int, 512>{});
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Odd rings in pairs: the two rings of a pair with the same odd number n of
+// pixels (or a single one) are the real and imaginary part of one complex
+// sequence of length n, transformed by one register Bluestein convolution of
+// length M >= 2n - 1.  One CTA of M/16 threads per pair and component.  A Gauss
+// grid of 251 pairs of 1001 = 7 11 13 pixels, 6 components of floats: 55 us
+// (synthesis) and 49 us (analysis), against 238 and 236 us with generic radix-7,
+// 11 and 13 passes in the size classes, one ring after the other.
+// ---------------------------------------------------------------------------
+template <typename T, int M>
+__global__ void __launch_bounds__(M / 16, blue_min_blocks(M))
+phase2ring_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
+                      const int *__restrict__ nph, const long long *__restrict__ ofs,
+                      const int *__restrict__ stride, const double *__restrict__ phi0,
+                      const double2 *__restrict__ shift, int sw,
+                      const double *__restrict__ weight, const int *__restrict__ fftidx,
+                      const FftDesc *__restrict__ fdesc, const double2 *__restrict__ wpow2,
+                      int P, const double2 *__restrict__ bhat,
+                      const double2 *__restrict__ chirp, const double2 *__restrict__ phase,
+                      int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
+                      long long map_lo) {
+  constexpr int NT = M / 16;
+  extern __shared__ double2 smem[];
+  double2 *buf = smem;
+  const int sl = kShiftLo + mmax / kShiftLo + 1;   // slices of one ring
+  double2 *slices = smem + pw_entries(M);
+  const int p = pairs[blockIdx.x], c = blockIdx.y;
+  const int nr[2] = {max(nph[2 * p], 0), max(nph[2 * p + 1], 0)};
+  const int n = max(nr[0], nr[1]), half = n / 2;
+  const FftDesc &fd = fdesc[fftidx[2 * p + (nr[0] ? 0 : 1)]];
+  const double2 *cz = chirp + fd.chirp;   // c_j, j < n
+  const int ms = mmax + 1;
+  const int mm = min(mmax, mlim[p]);
+  const bool add = (flags & (SHARP_ADD | SHARP_SUBTRACT)) != 0;
+  const double scale = ((flags & SHARP_REAL_HARMONICS) ? kSqrtHalf : 1.0) *
+                       ((flags & SHARP_SUBTRACT) ? -1.0 : 1.0);
+  for (int h = 0; h < 2; ++h)
+    load_shift(slices + h * sl, slices + h * sl + kShiftLo, mm, phi0[2 * p + h], false,
+               shift ? shift + size_t(2 * p + h) * sw : nullptr, threadIdx.x, NT);
+  __syncthreads();
+  // C_k, k <= half, of both rings (sharp.c:265-300): the first in entries [0,
+  // half], the second behind it
+  for (int h = 0; h < 2; ++h) {
+    const double2 *src = phase + ((long long)(p * ncm + c) * 2 + h) * ms;
+    const double wgt = ((flags & SHARP_USE_WEIGHTS) ? weight[2 * p + h] : 1.0) * scale;
+    const bool rot = fabs(phi0[2 * p + h]) >= 1e-14;
+    const double2 *slo = slices + h * sl, *shi = slo + kShiftLo;
+    auto tm = [&](int m) {
+      double2 t = cscale(src[m], wgt);
+      if (rot) t = cmul(t, shift_of(slo, shi, m));
+      return t;
+    };
+    for (int k = threadIdx.x; k <= half; k += NT) {
+      double2 acc = make_double2(0.0, 0.0);
+      if (nr[h]) {
+        for (int m = k; m <= mm; m += n) acc = cadd(acc, tm(m));
+        for (int m = (k == 0) ? n : n - k; m <= mm; m += n) acc = cadd(acc, cconj(tm(m)));
+      }
+      if (k == 0) acc.y = 0.0;
+      buf[pw_pad(h * (half + 1) + k)] = acc;
+    }
+  }
+  __syncthreads();
+  // conj(Z_k) c_k, Z_k = C_k + i C'_k over the whole (Hermitian) spectra
+  double2 v[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int k = threadIdx.x + NT * i;
+    v[i] = make_double2(0.0, 0.0);
+    if (i < 8 && k < n) {
+      const int kk = k <= half ? k : n - k;
+      double2 a = buf[pw_pad(kk)], b = buf[pw_pad(half + 1 + kk)];
+      if (k > half) {
+        a.y = -a.y;
+        b.y = -b.y;
+      }
+      v[i] = cmul(make_double2(a.x - b.y, -(a.y + b.x)), __ldg(cz + k));
+    }
+  }
+  __syncthreads();
+  pw_pass16_regs<M, false>(v, buf, M, wpow2, P);
+  __syncthreads();
+  pb_convolve<M>(buf, wpow2, P, bhat + fd.bhat2);
+  T *base = static_cast<T *>(maps.p[c]) - map_lo;
+  T *m0 = base + ofs[2 * p], *m1 = base + ofs[2 * p + 1];
+  const long long s0 = stride[2 * p], s1 = stride[2 * p + 1];
+  for (int j = threadIdx.x; j < n; j += NT) {
+    const double2 z = cmul(buf[pw_pad(j)], __ldg(cz + j));
+    if (nr[0]) store_px(m0 + j * s0, z.x, add);
+    if (nr[1]) store_px(m1 + j * s1, -z.y, add);
+  }
+}
+
+template <typename T, int M>
+__global__ void __launch_bounds__(M / 16, blue_min_blocks(M))
+ring2phase_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
+                      const int *__restrict__ nph, const long long *__restrict__ ofs,
+                      const int *__restrict__ stride, const double *__restrict__ phi0,
+                      const double2 *__restrict__ shift, int sw,
+                      const double *__restrict__ weight, const int *__restrict__ fftidx,
+                      const FftDesc *__restrict__ fdesc, const double2 *__restrict__ wpow2,
+                      int P, const double2 *__restrict__ bhat,
+                      const double2 *__restrict__ chirp, double2 *__restrict__ phase, int ncm,
+                      int mmax, int flags, const __grid_constant__ PtrList maps,
+                      long long map_lo) {
+  constexpr int NT = M / 16;
+  extern __shared__ double2 smem[];
+  double2 *buf = smem;
+  const int sl = kShiftLo + mmax / kShiftLo + 1;
+  double2 *slices = smem + pw_entries(M);
+  const int p = pairs[blockIdx.x], c = blockIdx.y;
+  const int nr[2] = {max(nph[2 * p], 0), max(nph[2 * p + 1], 0)};
+  const int n = max(nr[0], nr[1]), half = n / 2;
+  const FftDesc &fd = fdesc[fftidx[2 * p + (nr[0] ? 0 : 1)]];
+  const double2 *cz = chirp + fd.chirp;
+  const int ms = mmax + 1;
+  const int mm = min(mmax, mlim[p]);
+  const double scale = (flags & SHARP_REAL_HARMONICS) ? kSqrtTwo : 1.0;
+  for (int h = 0; h < 2; ++h)
+    load_shift(slices + h * sl, slices + h * sl + kShiftLo, mm, phi0[2 * p + h], true,
+               shift ? shift + size_t(2 * p + h) * sw : nullptr, threadIdx.x, NT);
+  const T *base = static_cast<const T *>(maps.p[c]) - map_lo;
+  const T *m0 = base + ofs[2 * p], *m1 = base + ofs[2 * p + 1];
+  const long long s0 = stride[2 * p], s1 = stride[2 * p + 1];
+  double2 v[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int j = threadIdx.x + NT * i;
+    v[i] = make_double2(0.0, 0.0);
+    if (i < 8 && j < n)
+      v[i] = cmul(make_double2(nr[0] ? double(m0[j * s0]) : 0.0, nr[1] ? double(m1[j * s1]) : 0.0),
+                  __ldg(cz + j));
+  }
+  pw_pass16_regs<M, false>(v, buf, M, wpow2, P);
+  __syncthreads();
+  pb_convolve<M>(buf, wpow2, P, bhat + fd.bhat2);
+  // Z_k = c_k conv_k; X_k = (Z_k + conj Z_{n-k})/2 and -i (Z_k - conj Z_{n-k})/2;
+  // phase_m = X_{m mod n} (conjugated above half) wgt e^{-i m phi0}, m <= mm
+  const bool rot0 = fabs(phi0[2 * p]) >= 1e-14, rot1 = fabs(phi0[2 * p + 1]) >= 1e-14;
+  const double w0 = ((flags & SHARP_USE_WEIGHTS) ? weight[2 * p] : 1.0) * scale;
+  const double w1 = ((flags & SHARP_USE_WEIGHTS) ? weight[2 * p + 1] : 1.0) * scale;
+  double2 *d0 = phase + ((long long)(p * ncm + c) * 2) * ms, *d1 = d0 + ms;
+  for (int m = threadIdx.x; m <= mm; m += NT) {
+    const int idx = m % n;
+    const int k = idx <= half ? idx : n - idx, kn = k == 0 ? 0 : n - k;
+    const double2 zk = cmul(buf[pw_pad(k)], __ldg(cz + k));
+    const double2 zn = cmul(buf[pw_pad(kn)], __ldg(cz + kn));
+    double2 x0 = make_double2(0.5 * (zk.x + zn.x), 0.5 * (zk.y - zn.y));
+    double2 x1 = make_double2(0.5 * (zk.y + zn.y), 0.5 * (zn.x - zk.x));
+    if (idx > half) {
+      x0.y = -x0.y;
+      x1.y = -x1.y;
+    }
+    if (nr[0]) {
+      x0 = cscale(x0, w0);
+      d0[m] = rot0 ? cmul(x0, shift_of(slices, slices + kShiftLo, m)) : x0;
+    }
+    if (nr[1]) {
+      x1 = cscale(x1, w1);
+      d1[m] = rot1 ? cmul(x1, shift_of(slices + sl, slices + sl + kShiftLo, m)) : x1;
+    }
   }
 }
 
@@ -1592,6 +2153,13 @@ void launch_twiddles(GeomPlan &gp, int ntw, const std::vector<int> &tw_n,
   SHT_CUDA(cudaFreeAsync(d_off, st));
 }
 
+void launch_shift_table(GeomPlan &gp, cudaStream_t st) {
+  ProfScope ps("shift_table", st);
+  if (gp.npairs > 0)
+    shift_table_kernel<<<2 * gp.npairs, 128, 0, st>>>(gp.phi0, gp.shift_width - kShiftLo, gp.shift);
+  SHT_CUDA(cudaGetLastError());
+}
+
 // Ring pairs are launched per size class (largest complex FFT length of
 // the pair <= cls_N[c]) so small polar rings do not reserve the shared
 // memory and threads of the largest rings.
@@ -1610,6 +2178,9 @@ void launch_bluestein_pw_setup(const GeomPlan &gp, const int *d_blue2_idx, int n
                                          gp.bhat, gp.chirp);
     SHT_CUDA(cudaGetLastError());
   };
+  if (gp.P >= 128) one(bluestein_pw_setup_kernel<128>, 128);
+  if (gp.P >= 256) one(bluestein_pw_setup_kernel<256>, 256);
+  if (gp.P >= 512) one(bluestein_pw_setup_kernel<512>, 512);
   if (gp.P >= 1024) one(bluestein_pw_setup_kernel<1024>, 1024);
   if (gp.P >= 2048) one(bluestein_pw_setup_kernel<2048>, 2048);
   if (gp.P >= 4096) one(bluestein_pw_setup_kernel<4096>, 4096);
@@ -1705,7 +2276,7 @@ void phase2ring_class(const JobDesc &job, const GeomPlan &gp, int cls, long long
   auto k = phase2ring_kernel<T>;
   allow_smem(k, L.smem);
   k<<<L.grid, L.thr, L.smem, st>>>(gp.cls_pairs + gp.cls_start[cls], gp.mlim, gp.nph, gp.ofs,
-                                   gp.stride, gp.phi0, gp.weight, gp.fft, gp.fdesc, gp.twiddle,
+                                   gp.stride, gp.phi0, gp.shift, gp.shift_width, gp.weight, gp.fft, gp.fdesc, gp.twiddle,
                                    gp.wpow2, gp.P, gp.bhat, phase, ncm, job.mmax, job.flags,
                                    gp.cls_bufA[cls], gp.cls_bufB[cls], fft_twcap(gp),
                                    maps_dev, map_lo, L.gbuf, L.npc,
@@ -1722,7 +2293,7 @@ void ring2phase_class(const JobDesc &job, const GeomPlan &gp, int cls, long long
   auto k = ring2phase_kernel<T>;
   allow_smem(k, L.smem);
   k<<<L.grid, L.thr, L.smem, st>>>(gp.cls_pairs + gp.cls_start[cls], gp.mlim, gp.nph, gp.ofs,
-                                   gp.stride, gp.phi0, gp.weight, gp.fft, gp.fdesc, gp.twiddle,
+                                   gp.stride, gp.phi0, gp.shift, gp.shift_width, gp.weight, gp.fft, gp.fdesc, gp.twiddle,
                                    gp.wpow2, gp.P, gp.bhat, phase, ncm, job.mmax, job.flags,
                                    gp.cls_bufA[cls], gp.cls_bufB[cls], fft_twcap(gp),
                                    maps_dev, map_lo, L.gbuf,
@@ -1747,7 +2318,7 @@ void phase2ring_pow2(const JobDesc &job, const GeomPlan &gp, int cls, long long 
   const size_t smem = pow2_smem(N, job.mmax);
   allow_smem(k, smem);
   k<<<dim3(2 * gp.pw_count[cls], nmapptr), N / 16, smem, st>>>(
-      gp.pw_pairs + gp.pw_start[cls], gp.mlim, gp.nph, gp.ofs, gp.phi0, gp.weight, gp.fft,
+      gp.pw_pairs + gp.pw_start[cls], gp.mlim, gp.nph, gp.ofs, gp.phi0, gp.shift, gp.shift_width, gp.weight, gp.fft,
       gp.fdesc, gp.twiddle, phase, ncm, job.mmax, job.flags,
       maps_dev, map_lo);
   SHT_CUDA(cudaGetLastError());
@@ -1762,7 +2333,7 @@ void ring2phase_pow2(const JobDesc &job, const GeomPlan &gp, int cls, long long 
   const size_t smem = pow2_smem(N, job.mmax) + sizeof(double2) * (kTwLo + N / kTwLo + 1);
   allow_smem(k, smem);
   k<<<dim3(2 * gp.pw_count[cls], nmapptr), N / 16, smem, st>>>(
-      gp.pw_pairs + gp.pw_start[cls], gp.mlim, gp.nph, gp.ofs, gp.phi0, gp.weight, gp.fft,
+      gp.pw_pairs + gp.pw_start[cls], gp.mlim, gp.nph, gp.ofs, gp.phi0, gp.shift, gp.shift_width, gp.weight, gp.fft,
       gp.fdesc, gp.twiddle, phase, ncm, job.mmax, job.flags,
       maps_dev, map_lo);
   SHT_CUDA(cudaGetLastError());
@@ -1781,7 +2352,7 @@ void phase2ring_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long 
   const size_t smem = stage_row ? with_row : base;
   allow_smem(k, smem);
   k<<<dim3(2 * gp.pb_count[cls], nmapptr), M / 16, smem, st>>>(
-      gp.pb_pairs + gp.pb_start[cls], gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.weight,
+      gp.pb_pairs + gp.pb_start[cls], gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.shift, gp.shift_width, gp.weight,
       gp.fft, gp.fdesc, gp.twiddle, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase, ncm, job.mmax,
       job.flags, maps_dev, map_lo, stage_row);
   SHT_CUDA(cudaGetLastError());
@@ -1795,9 +2366,52 @@ void ring2phase_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long 
   const size_t smem = pow2_smem(M, job.mmax);
   allow_smem(k, smem);
   k<<<dim3(2 * gp.pb_count[cls], nmapptr), M / 16, smem, st>>>(
-      gp.pb_pairs + gp.pb_start[cls], gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.weight,
+      gp.pb_pairs + gp.pb_start[cls], gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.shift, gp.shift_width, gp.weight,
       gp.fft, gp.fdesc, gp.twiddle, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase, ncm, job.mmax,
       job.flags, maps_dev, map_lo);
+  SHT_CUDA(cudaGetLastError());
+}
+
+template <typename T, bool SYNTH>
+void odd_rings(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
+               const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm, cudaStream_t st) {
+  auto length = [&](auto len) {
+    constexpr int M = decltype(len)::value;
+    const size_t smem = sizeof(double2) * odd_ring_smem_entries(M, job.mmax);
+    auto go = [&](auto kernel) {
+      allow_smem(kernel, smem);
+      kernel<<<dim3(gp.po_count[cls], nmapptr), M / 16, smem, st>>>(
+          gp.po_pairs + gp.po_start[cls], gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.shift,
+          gp.shift_width, gp.weight, gp.fft, gp.fdesc, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase,
+          ncm, job.mmax, job.flags, maps_dev, map_lo);
+    };
+    if constexpr (SYNTH) go(phase2ring_odd_kernel<T, M>);
+    else go(ring2phase_odd_kernel<T, M>);
+  };
+  switch (gp.po_M[cls]) {
+    case 256: length(std::integral_constant<int, 256>{}); break;
+    case 512: length(std::integral_constant<int, 512>{}); break;
+    case 1024: length(std::integral_constant<int, 1024>{}); break;
+    case 2048: length(std::integral_constant<int, 2048>{}); break;
+    case 4096: length(std::integral_constant<int, 4096>{}); break;
+    default: length(std::integral_constant<int, 8192>{}); break;
+  }
+  SHT_CUDA(cudaGetLastError());
+}
+
+template <typename T, bool SYNTH>
+void short_rings(const JobDesc &job, const GeomPlan &gp, long long map_lo, const PtrList &maps_dev,
+                 int nmapptr, double2 *phase, int ncm, cudaStream_t st) {
+  if (gp.ps_count == 0) return;
+  const size_t smem = short_smem(job.mmax);
+  auto go = [&](auto kernel) {
+    kernel<<<dim3(2 * gp.ps_count, nmapptr), 32, smem, st>>>(
+        gp.ps_pairs, gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.shift, gp.shift_width,
+        gp.weight, gp.fft, gp.fdesc, gp.twiddle, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase, ncm,
+        job.mmax, job.flags, maps_dev, map_lo);
+  };
+  if constexpr (SYNTH) go(phase2ring_short_kernel<T>);
+  else go(ring2phase_short_kernel<T>);
   SHT_CUDA(cudaGetLastError());
 }
 
@@ -1823,6 +2437,9 @@ void phase2ring_pow2_classes(const JobDesc &job, const GeomPlan &gp, long long m
       default: phase2ring_blue<T, 8192>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
     }
   }
+  for (int c = 0; c < int(gp.po_M.size()); ++c)
+    odd_rings<T, true>(job, gp, c, map_lo, maps_dev, nmapptr, const_cast<double2 *>(phase), ncm, st);
+  short_rings<T, true>(job, gp, map_lo, maps_dev, nmapptr, const_cast<double2 *>(phase), ncm, st);
 }
 
 template <typename T>
@@ -1847,6 +2464,9 @@ void ring2phase_pow2_classes(const JobDesc &job, const GeomPlan &gp, long long m
       default: ring2phase_blue<T, 8192>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
     }
   }
+  for (int c = 0; c < int(gp.po_M.size()); ++c)
+    odd_rings<T, false>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+  short_rings<T, false>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, st);
 }
 
 }  // namespace
