@@ -250,23 +250,13 @@ mixed_image_kernel(int lmax, int spin, const long long *__restrict__ moff,
         if (col >= NCOL) break;
         const double2 v = arow[lane][col >> 1];
         const int p = static_cast<int>(llrint(((col & 1) ? v.y : v.x) * inv[col]));
-        // signed base-256 digits, each in [-128, 127]
-        int d[4], r = p;
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          d[q] = ((r + 128) & 255) - 128;
-          r = (r - d[q]) >> 8;
-        }
-        d[3] = r;
         psum[k] += p;
+        uint32_t words[kClasses];
+        toeplitz_words(p, words);
 #pragma unroll
         for (int w = 2; w <= 6; ++w) {
-          uint32_t word = 0;
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if (w - q >= 0 && w - q <= 3) word |= uint32_t(uint8_t(int8_t(d[w - q]))) << (8 * q);
           const int row = col * kClasses + (w - 2);
-          *reinterpret_cast<uint32_t *>(tile + tile_off(row, 4 * jj)) = word;
+          *reinterpret_cast<uint32_t *>(tile + tile_off(row, 4 * jj)) = words[w - 2];
         }
       }
     }

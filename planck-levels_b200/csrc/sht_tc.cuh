@@ -161,6 +161,20 @@ __device__ __forceinline__ uint32_t quant(double v, double cq) {
   return static_cast<uint32_t>(__double2loint(fma(v, cq, kMagic)));
 }
 
+// The words of the five byte-product classes w = 2 .. 6 of an integer q, |q| <=
+// 2^30: byte k of word w is the signed base-256 digit d_(w-k) of q (0 outside
+// 0 .. 3).  Adding 128 to the three low digits and flipping their top bits
+// leaves the digits in the bytes; reversed, the words are shifts of them.
+__device__ __forceinline__ void toeplitz_words(int q, uint32_t (&word)[5]) {
+  const uint32_t d = (uint32_t(q) + 0x00808080u) ^ 0x00808080u;
+  const uint32_t r = __byte_perm(d, 0u, 0x0123);
+  word[0] = r >> 8;
+  word[1] = r;
+  word[2] = r << 8;
+  word[3] = r << 16;
+  word[4] = r << 24;
+}
+
 // Shared-memory accesses in explicit form (volatile: they stay behind the
 // mbarrier waits that publish the data).
 __device__ __forceinline__ double2 lds_f64x2(uint32_t a) {
