@@ -17,7 +17,7 @@
 //    renormalised once per l-block, nothing accumulated), then switches to
 //    plain IEEE values.  Skipped terms are < 2^-88 of the leading ones;
 //  * analysis reduces over rings through shared memory within a warp and in a
-//    fixed order across warps: no atomics, bitwise repeatable results.
+//    fixed order across warps and tiles: bitwise repeatable results.
 //
 // What bounds it: the FP64 pipe, and in it the register ports.  A DFMA with
 // three distinct register operands issues every 3 cycles per sub-partition, 2/3
@@ -565,22 +565,24 @@ synth_spin_kernel(const int2 *__restrict__ items, const int *__restrict__ count,
 // chunk's barrier (the same one that publishes staged coefficients) the warps
 // share out the sub-blocks, add the warps' sums in a fixed order and store
 // them (first tile) or add them (later tiles; the same thread owns an entry
-// in every tile) to Aout, which this CTA owns: no atomics, bitwise repeatable,
+// in every tile) to Aout, which this CTA owns: bitwise repeatable,
 // one barrier per kAChunk l-steps.  Every row l in [m, lmax] is written.
 //
 // The reduction through shared memory takes 42 instructions per 16 values;
 // recursive halving with shuffles took 107, more than half of them selects, and
 // left the FP64 pipe at 40%.  With it and the loops free of tests, Nside 1024 /
 // lmax 2048: spin 2 5.02 ms, spin 0 1.77 (before: 6.11 and 1.99); Nside 2048 /
-// lmax 4096: 35.2 and 12.4 (44.8 and 14.1).  Rings of a thread spread over the
+// lmax 4096: 34.4 and 11.8 (44.8 and 14.1).  Rings of a thread spread over the
 // tile (equal work for the warps between two barriers), with loops compiled for
 // each number of active ones: 5.1-5.3 and 1.94 ms, so a warp's rings stay
 // consecutive.  The contraction on the FP64 tensor instructions fills 4 (spin s)
 // or 2 (spin 0) of the 8 columns of an m8n8k4 with one transform: no gain.
 // ---------------------------------------------------------------------------
-// l-steps per chunk: the warps' sums of two chunks within 48 KB of shared memory
+// l-steps per chunk: as many as keep the CTAs per SM (the warps' sums of two
+// chunks lie in shared memory).  Spin 0: 256 (Nside 2048: 11.8 ms, 12.3 with 64),
+// spin s: 128 (34.4 ms, 34.8 with 64, 40.5 with 256).
 template <int VPL, int W>
-constexpr int kAChunkOf = VPL * W >= 32 ? 32 : 64;
+constexpr int kAChunkOf = VPL * W >= 32 ? 32 : VPL * W > 16 ? 64 : 512 / VPL;
 constexpr int kRed = 16;   // values per transpose-reduction
 
 template <int VPL, int W>
@@ -593,7 +595,10 @@ __device__ __forceinline__ void flush_chunk(const double *wred, int nwarps, bool
     double acc = wred[t];
     for (int w = 1; w < nwarps; ++w) acc += wred[w * ld + t];
     double *out = Aout + ((mo + l0 + t / VPL) * ncA + comp0) * 2 + t % VPL;
-    *out = first ? acc : *out + acc;
+    // the same thread owns an entry in every tile, so its additions are in order;
+    // as reductions they do not wait for the old value
+    if (first) *out = acc;
+    else atomicAdd(out, acc);
   }
 }
 
