@@ -257,7 +257,7 @@ inline void allow_smem(K kernel, size_t bytes);
 
 // Kernel launchers (sht_legendre.cu)
 // Ring pairs up to which the spin analysis takes two transforms per pass (above,
-// four rings per thread leave no registers for a second one).
+// three rings per thread leave no registers for a second one).
 constexpr int kAnalWidePairs = 512;
 void launch_coef_tables(CoefPlan &cp, cudaStream_t st);
 void launch_legendre_synth(const JobDesc &job, const GeomPlan &gp, const CoefPlan &cp,

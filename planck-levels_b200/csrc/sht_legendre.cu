@@ -71,6 +71,50 @@ __device__ __forceinline__ double2 warp_reduce16(const double (&v)[16], double2 
   return a;
 }
 
+// The same in two steps, so that the next values' loop covers the latency of the
+// loads, additions and exchanges: put() stores the values, sums() adds up those
+// stored before.
+struct WarpSums {
+  double2 *buf;        // 256 entries of this warp
+  double *dst;         // where the values in buf go, null: none there
+  __device__ __forceinline__ double2 sums() const {
+    const int lane = threadIdx.x & 31, q = lane >> 3, c = lane & 7;
+    double2 a = buf[q * 8 + (c ^ q)];
+#pragma unroll
+    for (int t = 1; t < 8; ++t) {
+      const int row = q + 4 * t;
+      const double2 w = buf[row * 8 + (c ^ (row & 7))];
+      a.x += w.x;
+      a.y += w.y;
+    }
+#pragma unroll
+    for (int s = 8; s <= 16; s <<= 1) {
+      a.x += __shfl_xor_sync(0xffffffffu, a.x, s);
+      a.y += __shfl_xor_sync(0xffffffffu, a.y, s);
+    }
+    return a;
+  }
+  // stores `a` (sums()) for the values in buf, then takes v for d
+  __device__ __forceinline__ void put(double2 a, const double (&v)[16], double *d) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    if (dst && lane < 8) *reinterpret_cast<double2 *>(dst + 2 * lane) = a;
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      buf[lane * 8 + (c ^ (lane & 7))] = make_double2(v[2 * c], v[2 * c + 1]);
+    dst = d;
+    __syncwarp();
+  }
+  __device__ __forceinline__ void drain() {
+    if (!dst) return;
+    const double2 a = sums();
+    const int lane = threadIdx.x & 31;
+    if (lane < 8) *reinterpret_cast<double2 *>(dst + 2 * lane) = a;
+    dst = nullptr;
+    __syncwarp();
+  }
+};
+
 // ---------------------------------------------------------------------------
 // Coefficient tables (one thread per m)
 // ---------------------------------------------------------------------------
@@ -571,8 +615,10 @@ synth_spin_kernel(const int2 *__restrict__ items, const int *__restrict__ count,
 // The reduction through shared memory takes 42 instructions per 16 values;
 // recursive halving with shuffles took 107, more than half of them selects, and
 // left the FP64 pipe at 40%.  With it and the loops free of tests, Nside 1024 /
-// lmax 2048: spin 2 5.02 ms, spin 0 1.77 (before: 6.11 and 1.99); Nside 2048 /
-// lmax 4096: 34.4 and 11.8 (44.8 and 14.1).  Rings of a thread spread over the
+// lmax 2048: spin 2 4.72 ms, spin 0 1.70 (before: 6.11 and 1.99); Nside 2048 /
+// lmax 4096: 32.9 and 11.8 (44.8 and 14.1).  Overlapping the reduction with the
+// next values' loop (WarpSums) is worth 1.5 ms of that at spin 2 (R = 3; R = 4
+// without it 34.4, with it 34.1).  Rings of a thread spread over the
 // tile (equal work for the warps between two barriers), with loops compiled for
 // each number of active ones: 5.1-5.3 and 1.94 ms, so a warp's rings stay
 // consecutive.  The contraction on the FP64 tensor instructions fills 4 (spin s)
@@ -580,7 +626,7 @@ synth_spin_kernel(const int2 *__restrict__ items, const int *__restrict__ count,
 // ---------------------------------------------------------------------------
 // l-steps per chunk: as many as keep the CTAs per SM (the warps' sums of two
 // chunks lie in shared memory).  Spin 0: 256 (Nside 2048: 11.8 ms, 12.3 with 64),
-// spin s: 128 (34.4 ms, 34.8 with 64, 40.5 with 256).
+// spin s: 128 (34.4 ms at R = 4, 34.8 with 64, 40.5 with 256).
 template <int VPL, int W>
 constexpr int kAChunkOf = VPL * W >= 32 ? 32 : VPL * W > 16 ? 64 : 512 / VPL;
 constexpr int kRed = 16;   // values per transpose-reduction
@@ -653,6 +699,8 @@ anal_spin0_kernel(const int *__restrict__ count, const double *__restrict__ cth,
                   int comp0) {
   constexpr int VPL = 2 * NT;
   constexpr int LB = kRed / VPL, kAChunk = kAChunkOf<VPL, W>;
+  // not with W = 8 (more warps cover the latency) or R = 4 (no registers for it)
+  constexpr bool kOverlap = W == 4 && R < 4;
   static_assert(LB % 2 == 0 && kLBlock % LB == 0, "l-block must be even and divide kLBlock");
   extern __shared__ double2 smem[];
   double2(*red)[32 * kRed / 2] = reinterpret_cast<double2(*)[32 * kRed / 2]>(smem);
@@ -719,6 +767,7 @@ anal_spin0_kernel(const int *__restrict__ count, const double *__restrict__ cth,
         flush_chunk<VPL, W>(wred[(ch - 1) & 1][0], nwarps, tb == 0, m + (ch - 1) * kAChunk, lmax, mo,
                          ncA, comp0, Aout);
       if (warp >= nwarps) continue;
+      WarpSums ws{red[warp], nullptr};
       const double2 *ca = reinterpret_cast<const double2 *>(s_al[ch % 3]);
       const int nb = min(kAChunk, lmax + 1 - (m + ch * kAChunk));
 #pragma unroll 1
@@ -727,6 +776,8 @@ anal_spin0_kernel(const int *__restrict__ count, const double *__restrict__ cth,
           constexpr bool MASK = decltype(masked)::value;
 #pragma unroll 1
           for (int sb = b0 / LB; sb < (b0 + kLBlock) / LB; ++sb) {
+            double2 sum = make_double2(0.0, 0.0);
+            if (kOverlap) sum = ws.sums();   // of the previous values
             double v[kRed];
 #pragma unroll
             for (int i = 0; i < LB; i += 2) {
@@ -749,9 +800,13 @@ anal_spin0_kernel(const int *__restrict__ count, const double *__restrict__ cth,
                 mu1[r] = nn;
               }
             }
-            const double2 sum = warp_reduce16(v, red[warp]);
-            if (lane < kRed / 2)
-              *reinterpret_cast<double2 *>(&wred[ch & 1][warp][sb * kRed + 2 * lane]) = sum;
+            if (kOverlap) {
+              ws.put(sum, v, &wred[ch & 1][warp][sb * kRed]);
+            } else {
+              sum = warp_reduce16(v, red[warp]);
+              if (lane < kRed / 2)
+                *reinterpret_cast<double2 *>(&wred[ch & 1][warp][sb * kRed + 2 * lane]) = sum;
+            }
           }
         };
         if (state == kFull) {
@@ -786,6 +841,7 @@ anal_spin0_kernel(const int *__restrict__ count, const double *__restrict__ cth,
         }
         state = warp_state(act, live);
       }
+      ws.drain();
     }
     __pipeline_wait_prior(0);
     __syncthreads();
@@ -813,6 +869,7 @@ anal_spin_kernel(const int *__restrict__ count, const double *__restrict__ cth,
                  int comp0) {
   constexpr int VPL = 4 * NT;
   constexpr int LB = kRed / VPL, kAChunk = kAChunkOf<VPL, W>;
+  constexpr bool kOverlap = W == 4;   // as at spin 0
   static_assert(LB % 2 == 0 && kLBlock % LB == 0, "l-block must be even and divide kLBlock");
   extern __shared__ double2 smem[];
   double2(*red)[32 * kRed / 2] = reinterpret_cast<double2(*)[32 * kRed / 2]>(smem);
@@ -895,6 +952,7 @@ anal_spin_kernel(const int *__restrict__ count, const double *__restrict__ cth,
         flush_chunk<VPL, W>(wred[(ch - 1) & 1][0], nwarps, tb == 0, mhi + (ch - 1) * kAChunk, lmax, mo,
                          ncA, comp0, Aout);
       if (warp >= nwarps) continue;
+      WarpSums ws{red[warp], nullptr};
       const double2 *cab = s_ab[ch % 3];
       const int nb = min(kAChunk, lmax + 1 - (mhi + ch * kAChunk));
 #pragma unroll 1
@@ -903,6 +961,8 @@ anal_spin_kernel(const int *__restrict__ count, const double *__restrict__ cth,
           constexpr bool MASK = decltype(masked)::value;
 #pragma unroll 1
           for (int sb = b0 / LB; sb < (b0 + kLBlock) / LB; ++sb) {
+            double2 sum = make_double2(0.0, 0.0);
+            if (kOverlap) sum = ws.sums();   // of the previous values
             double v[kRed];
 #pragma unroll
             for (int i = 0; i < LB; ++i) {
@@ -937,9 +997,13 @@ anal_spin_kernel(const int *__restrict__ count, const double *__restrict__ cth,
                 mm1[r] = nm;
               }
             }
-            const double2 sum = warp_reduce16(v, red[warp]);
-            if (lane < kRed / 2)
-              *reinterpret_cast<double2 *>(&wred[ch & 1][warp][sb * kRed + 2 * lane]) = sum;
+            if (kOverlap) {
+              ws.put(sum, v, &wred[ch & 1][warp][sb * kRed]);
+            } else {
+              sum = warp_reduce16(v, red[warp]);
+              if (lane < kRed / 2)
+                *reinterpret_cast<double2 *>(&wred[ch & 1][warp][sb * kRed + 2 * lane]) = sum;
+            }
           }
         };
         if (state == kFull) {
@@ -978,6 +1042,7 @@ anal_spin_kernel(const int *__restrict__ count, const double *__restrict__ cth,
         }
         state = warp_state(act, live);
       }
+      ws.drain();
     }
     __pipeline_wait_prior(0);
     __syncthreads();
@@ -1067,17 +1132,18 @@ void launch_legendre_anal(const JobDesc &job, const GeomPlan &gp, const CoefPlan
   using std::integral_constant;
   constexpr integral_constant<int, 1> c1{};
   constexpr integral_constant<int, 2> c2{};
+  constexpr integral_constant<int, 3> c3{};
   constexpr integral_constant<int, 4> c4{};
   constexpr integral_constant<int, 8> c8{};
   // Shape (R rings per thread, W warps).  More rings per thread share a
   // reduction and more warps a tile; but one warp walks all l of its m alone, so
   // with few ring pairs that chain is the kernel's time and smaller R is faster.
   // Measured with one transform, us, spin 0 / spin 2 (Nside: pairs):
-  //   Nside 64 (128):    R1 W4 8.9 / 15.4   R2 W4 10.7 / 21.1   R4 W4 15.7 / 33.9
-  //   Nside 128 (256):   R1 W4 29.0 / 53.6  R2 W4 20.1 / 41.0   R4 W4 28.5 / 61.7
-  //   Nside 256 (512):   R2 W4 79.9 / 177   R2 W8 58.5 / 144    R4 W4 66.3 / 145
-  //   Nside 512 (1024):  R2 W4 342 / 834    R2 W8 343 / 801     R4 W4 299 / 813
-  //   Nside 1024 (2048): R2 W4 2296 / 5120  R2 W8 2343 / 5437   R4 W4 1767 / 5017
+  //   Nside 64 (128):    R1 W4 8.8 / 15.0   R2 W4 10.7 / 21.1   R4 W4 15.7 / 33.9
+  //   Nside 128 (256):   R1 W4 29.0 / 53.6  R2 W4 19.9 / 38.5   R4 W4 28.5 / 61.7
+  //   Nside 256 (512):   R2 W4 79.9 / 177   R2 W8 56.9 / 142    R4 W4 66.3 / 145
+  //   Nside 512 (1024):  R2 W8 343 / 801    R3 W4 300 / 769     R4 W4 288 / 778
+  //   Nside 1024 (2048): R2 W8 2343 / 5437  R3 W4 1844 / 4719   R4 W4 1701 / 4951
   // The shape fixes the order of the sums over rings, so it does not depend on
   // the number of transforms of the pass: a transform's result is the same bits
   // alone and in any batch.
@@ -1085,7 +1151,8 @@ void launch_legendre_anal(const JobDesc &job, const GeomPlan &gp, const CoefPlan
     if (gp.npairs <= 128) f(n, c1, c4);
     else if (gp.npairs <= 256) f(n, c2, c4);
     else if (gp.npairs <= kAnalWidePairs) f(n, c2, c8);
-    else f(n, c4, c4);
+    else if (job.spin == 0) f(n, c4, c4);
+    else f(n, c3, c4);
   };
   if (job.spin == 0) {
     if (nt == 1) shape(c1, spin0);
