@@ -38,12 +38,11 @@ def _real(t: torch.Tensor) -> torch.Tensor:
     return torch.view_as_real(t).reshape(-1)
 
 
-def _m_weights(lmax: int, mmax: int, device) -> torch.Tensor:
-    """D: 1 on the m = 0 block (first lmax+1 entries), 2 elsewhere."""
-    nalm = ((mmax + 1) * (mmax + 2)) // 2 + (mmax + 1) * (lmax - mmax)
-    w = torch.full((nalm,), 2.0, dtype=torch.float64, device=device)
-    w[: lmax + 1] = 1.0
-    return w
+def _scale_m(alm: torch.Tensor, lmax: int, factor: float) -> torch.Tensor:
+    """alm *= factor in place except on the m = 0 block (the first lmax+1 entries):
+    D and its inverse for factors 2 and 1/2."""
+    torch.view_as_real(alm)[lmax + 1:].mul_(factor)
+    return alm
 
 
 class _Alm2Map(torch.autograd.Function):
@@ -60,15 +59,14 @@ class _Alm2Map(torch.autograd.Function):
     @staticmethod
     def backward(ctx, *gmaps):
         geom, ainfo, spin = ctx.geom, ctx.ainfo, ctx.spin
-        lmax, nm = ainfo.lmax, ainfo.nm
+        lmax = ainfo.lmax
         gm = [g.contiguous() for g in gmaps]
         galm = [torch.zeros(ainfo.nalm(), dtype=torch.complex128, device=gm[0].device)
                 for _ in gm]
         # Yt through the adjoint flag on the synthesis job type
         execute_device(SHARP_ALM2MAP, spin, [_real(a) for a in galm], gm, geom, ainfo, 1,
                        ctx.flags | SHARP_ADJOINT)
-        w = _m_weights(lmax, nm - 1, gm[0].device)
-        galm = [a * w for a in galm]
+        galm = [_scale_m(a, lmax, 2.0) for a in galm]
         return (None, None, None, None, None, *galm)
 
 
@@ -85,9 +83,8 @@ class _Map2Alm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, *galms):
         geom, ainfo, spin = ctx.geom, ctx.ainfo, ctx.spin
-        lmax, nm = ainfo.lmax, ainfo.nm
-        w = _m_weights(lmax, nm - 1, galms[0].device)
-        ga = [(g.contiguous() / w) for g in galms]
+        ga = [_scale_m(g.clone(memory_format=torch.contiguous_format), ainfo.lmax, 0.5)
+              for g in galms]
         npix = geom.npix()
         gmaps = [torch.zeros(npix, dtype=torch.float64, device=ga[0].device) for _ in ga]
         # (Yt W)^T = W Y: the adjoint of the analysis job type
