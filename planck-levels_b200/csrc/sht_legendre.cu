@@ -278,6 +278,8 @@ synth_spin0_kernel(const int2 *__restrict__ items, const int *__restrict__ count
                    const double *__restrict__ alpha, const double *__restrict__ mfac,
                    const double2 *__restrict__ A, int ncA, int comp0, int lmax,
                    double2 *__restrict__ phase, int ncm, int pcomp0, int ms) {
+  grid_wait();
+  grid_release_small();
   __shared__ __align__(16) double s_al[kWarps][3][kChunk];
   __shared__ double2 s_A[kWarps][3][kChunk * NT];
   const int2 it = items[blockIdx.x];
@@ -425,6 +427,8 @@ synth_spin_kernel(const int2 *__restrict__ items, const int *__restrict__ count,
                   const double *__restrict__ pre_v, const int *__restrict__ pre_e, int s,
                   const double2 *__restrict__ A, int ncA, int comp0, int lmax,
                   double2 *__restrict__ phase, int ncm, int pcomp0, int ms) {
+  grid_wait();
+  grid_release_small();
   constexpr int NA = DERIV ? 1 : 2;  // staged alm components per transform
   constexpr int NC = NA * NT;        // staged alm entries per l
   __shared__ double2 s_ab[kWarps][3][kChunk];  // (a_l, b_l)
@@ -697,6 +701,8 @@ anal_spin0_kernel(const int *__restrict__ count, const double *__restrict__ cth,
                   const double *__restrict__ mfac, const double2 *__restrict__ phase, int ncm,
                   int pcomp0, int lmax, int ms, double *__restrict__ Aout, int ncA,
                   int comp0) {
+  grid_wait();
+  grid_release_small();
   constexpr int VPL = 2 * NT;
   constexpr int LB = kRed / VPL, kAChunk = kAChunkOf<VPL, W>;
   // not with W = 8 (more warps cover the latency) or R = 4 (no registers for it)
@@ -867,6 +873,8 @@ anal_spin_kernel(const int *__restrict__ count, const double *__restrict__ cth,
                  const int *__restrict__ pre_e, int s, const double2 *__restrict__ phase,
                  int ncm, int pcomp0, int lmax, int ms, double *__restrict__ Aout, int ncA,
                  int comp0) {
+  grid_wait();
+  grid_release_small();
   constexpr int VPL = 4 * NT;
   constexpr int LB = kRed / VPL, kAChunk = kAChunkOf<VPL, W>;
   constexpr bool kOverlap = W == 4;   // as at spin 0
@@ -1078,14 +1086,14 @@ void launch_legendre_synth(const JobDesc &job, const GeomPlan &gp, const CoefPla
   const bool deriv = job.type == SHARP_ALM2MAP_DERIV1;
   SHT_REQUIRE(gp.synth_tile == 128 || gp.synth_tile == 256, "synthesis tile mismatch");
   auto spin0 = [&](auto kernel) {
-    kernel<<<nitems, 128, 0, st>>>(gp.items, gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff,
-                                   cp.alpha, cp.seed, A, ncA, comp0, job.lmax, phase, ncm,
-                                   pcomp0, job.mmax + 1);
+    launch_overlapped(kernel, dim3(nitems), 128, 0, st, gp.items, gp.count, gp.cth, gp.sth, gp.nph,
+                      cp.d_moff, cp.alpha, cp.seed, A, ncA, comp0, job.lmax, phase, ncm, pcomp0,
+                      job.mmax + 1);
   };
   auto spins = [&](auto kernel) {
-    kernel<<<nitems, 128, 0, st>>>(gp.items, gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff,
-                                   cp.alpha, cp.beta, cp.seed, cp.seed_exp, cp.spin, A, ncA,
-                                   comp0, job.lmax, phase, ncm, pcomp0, job.mmax + 1);
+    launch_overlapped(kernel, dim3(nitems), 128, 0, st, gp.items, gp.count, gp.cth, gp.sth, gp.nph,
+                      cp.d_moff, cp.alpha, cp.beta, cp.seed, cp.seed_exp, cp.spin, A, ncA, comp0,
+                      job.lmax, phase, ncm, pcomp0, job.mmax + 1);
   };
   auto width = [&](auto r) {
     constexpr int RV = decltype(r)::value;
@@ -1116,18 +1124,18 @@ void launch_legendre_anal(const JobDesc &job, const GeomPlan &gp, const CoefPlan
     auto kernel = anal_spin0_kernel<NT, R, W>;
     constexpr size_t smem = anal_smem<2 * NT, W>();
     allow_smem(kernel, smem);
-    kernel<<<nblocks, 32 * W, smem, st>>>(gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff, cp.alpha,
-                                          cp.seed, phase, ncm, pcomp0, job.lmax, job.mmax + 1,
-                                          Aout, ncA, comp0);
+    launch_overlapped(kernel, dim3(nblocks), 32 * W, smem, st, gp.count, gp.cth, gp.sth, gp.nph,
+                      cp.d_moff, cp.alpha, cp.seed, phase, ncm, pcomp0, job.lmax, job.mmax + 1,
+                      Aout, ncA, comp0);
   };
   auto spins = [&](auto nt_, auto r_, auto w_) {
     constexpr int NT = decltype(nt_)::value, R = decltype(r_)::value, W = decltype(w_)::value;
     auto kernel = anal_spin_kernel<NT, R, W>;
     constexpr size_t smem = anal_smem<4 * NT, W>();
     allow_smem(kernel, smem);
-    kernel<<<nblocks, 32 * W, smem, st>>>(gp.count, gp.cth, gp.sth, gp.nph, cp.d_moff, cp.alpha,
-                                          cp.beta, cp.seed, cp.seed_exp, cp.spin, phase, ncm,
-                                          pcomp0, job.lmax, job.mmax + 1, Aout, ncA, comp0);
+    launch_overlapped(kernel, dim3(nblocks), 32 * W, smem, st, gp.count, gp.cth, gp.sth, gp.nph,
+                      cp.d_moff, cp.alpha, cp.beta, cp.seed, cp.seed_exp, cp.spin, phase, ncm,
+                      pcomp0, job.lmax, job.mmax + 1, Aout, ncA, comp0);
   };
   using std::integral_constant;
   constexpr integral_constant<int, 1> c1{};

@@ -68,16 +68,26 @@ __device__ __forceinline__ double2 cscale(double2 a, double s) {
 }
 // The register ring kernels of one direction read the same phase rows or maps
 // and write disjoint rows, so each may start while its predecessor's last CTAs
-// run (programmatic launch, ring_launch below): a kernel lets its successor
+// run (launch_overlapped): a kernel lets its successor
 // start as soon as all its CTAs have started, and ends only after its
 // predecessor has, so that what follows the last one in the stream finds all
 // of them done.  The chi-square gradient at Nside 512 (three components, both
 // directions, four kernels each) takes 2.41 ms with it, 2.52 without; three
 // Jacobi sweeps at Nside 1024 11.8 against 12.2 ms.  The size-class kernels
 // stay out of it: their global scratch is reused from one to the next.
+// The first of a direction waits for what came before it, and only then lets the
+// others start; the last lets its successor start as grid_release_small does.
+constexpr int kChainFirst = 1, kChainLast = 2;
 struct GridChain {
-  __device__ __forceinline__ GridChain() { asm volatile("griddepcontrol.launch_dependents;"); }
-  __device__ __forceinline__ ~GridChain() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+  int place;
+  __device__ __forceinline__ explicit GridChain(int p) : place(p) {
+    if (place & kChainFirst) grid_wait();
+    if (place & kChainLast) grid_release_small();
+    else grid_release();
+  }
+  __device__ __forceinline__ ~GridChain() {
+    if (!(place & kChainFirst)) grid_wait();
+  }
 };
 
 // FFT buffer (shared memory, or a CTA's slot of global scratch) whose element
@@ -984,8 +994,9 @@ phase2ring_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const int *__restrict__ fftidx, const FftDesc *__restrict__ fdesc,
                        const double2 *__restrict__ twiddle, const double2 *__restrict__ phase,
                        int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
-                       long long map_lo) {
-  const GridChain chain;
+                       long long map_lo,
+                        int place) {
+  const GridChain chain(place);
   extern __shared__ double2 smem[];
   __shared__ uint64_t row_full;
   double2 *buf = smem;
@@ -1085,8 +1096,9 @@ ring2phase_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const int *__restrict__ fftidx, const FftDesc *__restrict__ fdesc,
                        const double2 *__restrict__ twiddle, double2 *__restrict__ phase,
                        int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
-                       long long map_lo) {
-  const GridChain chain;
+                       long long map_lo,
+                        int place) {
+  const GridChain chain(place);
   extern __shared__ double2 smem[];
   double2 *buf = smem;
   double2 *slo = smem + pw_entries(N);
@@ -1256,8 +1268,9 @@ phase2ring_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const double2 *__restrict__ wpow2, int P,
                        const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                        const double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                       const __grid_constant__ PtrList maps, long long map_lo, int stage_row) {
-  const GridChain chain;
+                       const __grid_constant__ PtrList maps, long long map_lo, int stage_row,
+                        int place) {
+  const GridChain chain(place);
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   __shared__ uint64_t row_full;
@@ -1366,8 +1379,9 @@ ring2phase_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const double2 *__restrict__ wpow2, int P,
                        const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                        double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                       const __grid_constant__ PtrList maps, long long map_lo) {
-  const GridChain chain;
+                       const __grid_constant__ PtrList maps, long long map_lo,
+                        int place) {
+  const GridChain chain(place);
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   double2 *buf = smem;
@@ -1545,8 +1559,9 @@ phase2ring_short_kernel(const int *__restrict__ pairs, const int *__restrict__ m
                         const double2 *__restrict__ wpow2, int P,
                         const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                         const double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                        const __grid_constant__ PtrList maps, long long map_lo) {
-  const GridChain chain;
+                        const __grid_constant__ PtrList maps, long long map_lo,
+                        int place) {
+  const GridChain chain(place);
   extern __shared__ double2 smem[];
   double2 *buf = smem, *slo = buf + kShortEntries, *shi = slo + kShiftLo;
   const int p = pairs[blockIdx.x >> 1], h = blockIdx.x & 1, c = blockIdx.y;
@@ -1668,8 +1683,9 @@ ring2phase_short_kernel(const int *__restrict__ pairs, const int *__restrict__ m
                         const double2 *__restrict__ wpow2, int P,
                         const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                         double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                        const __grid_constant__ PtrList maps, long long map_lo) {
-  const GridChain chain;
+                        const __grid_constant__ PtrList maps, long long map_lo,
+                        int place) {
+  const GridChain chain(place);
   extern __shared__ double2 smem[];
   double2 *buf = smem, *slo = buf + kShortEntries, *shi = slo + kShiftLo;
   const int p = pairs[blockIdx.x >> 1], h = blockIdx.x & 1, c = blockIdx.y;
@@ -1805,8 +1821,9 @@ phase2ring_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mli
                       int P, const double2 *__restrict__ bhat,
                       const double2 *__restrict__ chirp, const double2 *__restrict__ phase,
                       int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
-                      long long map_lo) {
-  const GridChain chain;
+                      long long map_lo,
+                        int place) {
+  const GridChain chain(place);
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   double2 *buf = smem;
@@ -1890,8 +1907,9 @@ ring2phase_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mli
                       int P, const double2 *__restrict__ bhat,
                       const double2 *__restrict__ chirp, double2 *__restrict__ phase, int ncm,
                       int mmax, int flags, const __grid_constant__ PtrList maps,
-                      long long map_lo) {
-  const GridChain chain;
+                      long long map_lo,
+                        int place) {
+  const GridChain chain(place);
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   double2 *buf = smem;
@@ -2034,6 +2052,8 @@ stage_alm_kernel(int lmax, int nalmptr, const long long *__restrict__ mvstart,
                  const double *__restrict__ norm_l, bool use_norm, double norm_m0,
                  const __grid_constant__ PtrList alm, double2 *__restrict__ A, int ncA, int lgtl,
                  bool pm) {
+  grid_wait();
+  grid_release_small();
   extern __shared__ double2 tile[];
   const int tl = 1 << lgtl, ld = nalmptr | 1;
   const int m = blockIdx.x;
@@ -2088,6 +2108,8 @@ scatter_alm_kernel(int lmax, int nalmptr, const long long *__restrict__ mvstart,
                    const double *__restrict__ norm_l, bool use_norm, double norm_m0, double sgn,
                    bool add, const double *__restrict__ Aout, int ncA,
                    const __grid_constant__ PtrList alm, int lgtl) {
+  grid_wait();
+  grid_release_small();
   extern __shared__ double2 tile[];
   const int tl = 1 << lgtl, ld = nalmptr | 1;
   const int m = blockIdx.x;
@@ -2328,25 +2350,20 @@ void ring2phase_class(const JobDesc &job, const GeomPlan &gp, int cls, long long
 
 namespace {
 
-// Launches a register ring kernel; all but the first of a direction start while
-// the one before is running out (GridChain).
+// Launches the register ring kernels of one direction (GridChain).
 struct RingStream {
   cudaStream_t st;
-  bool first = true;
+  int left;             // kernels to come
+  int place = kChainFirst;
+  RingStream(const GeomPlan &gp, cudaStream_t s) : st(s), left(gp.ps_count > 0 ? 1 : 0) {
+    for (const auto *v : {&gp.pw_count, &gp.pb_count, &gp.po_count})
+      for (int n : *v) left += n > 0;
+  }
   template <class... P, class... A>
   void launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, A &&...args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = first ? 0 : 1;
-    first = false;
-    SHT_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    if (--left == 0) place |= kChainLast;
+    launch_overlapped(kernel, grid, threads, smem, st, args..., place);
+    place = 0;
   }
 };
 
@@ -2517,7 +2534,7 @@ void launch_phase2ring(const JobDesc &job, const GeomPlan &gp, long long map_lo,
                        const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
                        cudaStream_t st) {
   ProfScope ps("ring_synth", st);
-  RingStream rs{st};
+  RingStream rs(gp, st);
   if (job.dp)
     phase2ring_pow2_classes<double>(job, gp, map_lo, phase, ncm, maps_dev, nmapptr, rs);
   else
@@ -2535,7 +2552,7 @@ void launch_ring2phase(const JobDesc &job, const GeomPlan &gp, long long map_lo,
                        const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
                        cudaStream_t st) {
   ProfScope ps("ring_anal", st);
-  RingStream rs{st};
+  RingStream rs(gp, st);
   if (job.dp)
     ring2phase_pow2_classes<double>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, rs);
   else
@@ -2605,11 +2622,11 @@ void launch_stage_alm(const JobDesc &job, const AlmPlan &ap, long long alm_lo,
   const size_t smem = (sizeof(double2) << lg) * size_t(nalmptr | 1);
   ProfScope ps("stage_alm", st);
   if (job.dp)
-    stage_alm_kernel<double><<<blocks, 256, smem, st>>>(
+    launch_overlapped(stage_alm_kernel<double>, dim3(blocks), 256, smem, st,
         job.lmax, nalmptr, ap.mvstart, ap.stride, ap.packed, alm_lo, cp.d_moff, cp.cfac, norm_l,
         use_norm, norm_m0, alm_dev, A, ncA, lg, pm);
   else
-    stage_alm_kernel<float><<<blocks, 256, smem, st>>>(
+    launch_overlapped(stage_alm_kernel<float>, dim3(blocks), 256, smem, st,
         job.lmax, nalmptr, ap.mvstart, ap.stride, ap.packed, alm_lo, cp.d_moff, cp.cfac, norm_l,
         use_norm, norm_m0, alm_dev, A, ncA, lg, pm);
   SHT_CUDA(cudaGetLastError());
@@ -2628,11 +2645,11 @@ void launch_scatter_alm(const JobDesc &job, const AlmPlan &ap, long long alm_lo,
   const size_t smem = (sizeof(double2) << lg) * size_t(nalmptr | 1);
   ProfScope ps("scatter_alm", st);
   if (job.dp)
-    scatter_alm_kernel<double><<<blocks, 256, smem, st>>>(
+    launch_overlapped(scatter_alm_kernel<double>, dim3(blocks), 256, smem, st,
         job.lmax, nalmptr, ap.mvstart, ap.stride, ap.packed, alm_lo, cp.d_moff, cp.cfac, norm_l,
         use_norm, norm_m0, sgn, add, Aout, ncA, alm_dev, lg);
   else
-    scatter_alm_kernel<float><<<blocks, 256, smem, st>>>(
+    launch_overlapped(scatter_alm_kernel<float>, dim3(blocks), 256, smem, st,
         job.lmax, nalmptr, ap.mvstart, ap.stride, ap.packed, alm_lo, cp.d_moff, cp.cfac, norm_l,
         use_norm, norm_m0, sgn, add, Aout, ncA, alm_dev, lg);
   SHT_CUDA(cudaGetLastError());
