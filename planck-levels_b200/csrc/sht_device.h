@@ -95,7 +95,8 @@ inline int pow2_ring_length(int nph, int stride, int mm) {
 // folding) whose complex length either calls for a Bluestein convolution by
 // the cost model of the size classes or exceeds 1024 (there the size-class
 // kernel, one 1024-thread CTA per SM, ran the mixed-radix Stockham passes
-// about twice as slowly per ring as the register convolution).
+// about twice as slowly per ring as the register convolution); with all set,
+// every ring that has such an M.
 constexpr int kRegBluesteinMinN = 1024;
 inline int blue_ring_length(int nph, const FftDesc &d, bool all) {
   if (nph <= 0 || (nph & 1)) return 0;
