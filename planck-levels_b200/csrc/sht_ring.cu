@@ -1805,7 +1805,13 @@ ring2phase_short_kernel(const int *__restrict__ pairs, const int *__restrict__ m
 // Odd rings in pairs: the two rings of a pair with the same odd number n of
 // pixels (or a single one) are the real and imaginary part of one complex
 // sequence of length n, transformed by one register Bluestein convolution of
-// length M >= 2n - 1.  One CTA of M/16 threads per pair and component.  A Gauss
+// length M >= 2n - 1.  The rounding error of either is relative to the larger of
+// the two, so the ring weights are applied where it can tell them apart: to the
+// pixels before the transform in the analysis (a ring of weight 0 contributes
+// zeros, whatever its pixels hold; the two rings' terms are added right after),
+// and to the pixels after it in the synthesis (the unweighted rings are of one
+// size, being the sum and difference of the same two partial sums).
+// One CTA of M/16 threads per pair and component.  A Gauss
 // grid of 251 pairs of 1001 = 7 11 13 pixels, 6 components of floats: 55 us
 // (synthesis) and 49 us (analysis), against 238 and 236 us with generic radix-7,
 // 11 and 13 passes in the size classes, one ring after the other.
@@ -1839,6 +1845,8 @@ phase2ring_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mli
   const bool add = (flags & (SHARP_ADD | SHARP_SUBTRACT)) != 0;
   const double scale = ((flags & SHARP_REAL_HARMONICS) ? kSqrtHalf : 1.0) *
                        ((flags & SHARP_SUBTRACT) ? -1.0 : 1.0);
+  const double w0 = ((flags & SHARP_USE_WEIGHTS) ? weight[2 * p] : 1.0) * scale;
+  const double w1 = ((flags & SHARP_USE_WEIGHTS) ? weight[2 * p + 1] : 1.0) * scale;
   for (int h = 0; h < 2; ++h)
     load_shift(slices + h * sl, slices + h * sl + kShiftLo, mm, phi0[2 * p + h], false,
                shift ? shift + size_t(2 * p + h) * sw : nullptr, threadIdx.x, NT);
@@ -1847,14 +1855,9 @@ phase2ring_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mli
   // half], the second behind it
   for (int h = 0; h < 2; ++h) {
     const double2 *src = phase + ((long long)(p * ncm + c) * 2 + h) * ms;
-    const double wgt = ((flags & SHARP_USE_WEIGHTS) ? weight[2 * p + h] : 1.0) * scale;
     const bool rot = fabs(phi0[2 * p + h]) >= 1e-14;
     const double2 *slo = slices + h * sl, *shi = slo + kShiftLo;
-    auto tm = [&](int m) {
-      double2 t = cscale(src[m], wgt);
-      if (rot) t = cmul(t, shift_of(slo, shi, m));
-      return t;
-    };
+    auto tm = [&](int m) { return rot ? cmul(src[m], shift_of(slo, shi, m)) : src[m]; };
     for (int k = threadIdx.x; k <= half; k += NT) {
       double2 acc = make_double2(0.0, 0.0);
       if (nr[h]) {
@@ -1891,8 +1894,8 @@ phase2ring_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mli
   const long long s0 = stride[2 * p], s1 = stride[2 * p + 1];
   for (int j = threadIdx.x; j < n; j += NT) {
     const double2 z = cmul(buf[pw_pad(j)], __ldg(cz + j));
-    if (nr[0]) store_px(m0 + j * s0, z.x, add);
-    if (nr[1]) store_px(m1 + j * s1, -z.y, add);
+    if (nr[0]) store_px(m0 + j * s0, z.x * w0, add);
+    if (nr[1]) store_px(m1 + j * s1, -z.y * w1, add);
   }
 }
 
@@ -1923,6 +1926,8 @@ ring2phase_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mli
   const int ms = mmax + 1;
   const int mm = min(mmax, mlim[p]);
   const double scale = (flags & SHARP_REAL_HARMONICS) ? kSqrtTwo : 1.0;
+  const double w0 = ((flags & SHARP_USE_WEIGHTS) ? weight[2 * p] : 1.0) * scale;
+  const double w1 = ((flags & SHARP_USE_WEIGHTS) ? weight[2 * p + 1] : 1.0) * scale;
   for (int h = 0; h < 2; ++h)
     load_shift(slices + h * sl, slices + h * sl + kShiftLo, mm, phi0[2 * p + h], true,
                shift ? shift + size_t(2 * p + h) * sw : nullptr, threadIdx.x, NT);
@@ -1935,17 +1940,16 @@ ring2phase_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mli
     const int j = threadIdx.x + NT * i;
     v[i] = make_double2(0.0, 0.0);
     if (i < 8 && j < n)
-      v[i] = cmul(make_double2(nr[0] ? double(m0[j * s0]) : 0.0, nr[1] ? double(m1[j * s1]) : 0.0),
+      v[i] = cmul(make_double2(nr[0] ? double(m0[j * s0]) * w0 : 0.0,
+                               nr[1] ? double(m1[j * s1]) * w1 : 0.0),
                   __ldg(cz + j));
   }
   pw_pass16_regs<M, false>(v, buf, M, wpow2, P);
   __syncthreads();
   pb_convolve<M>(buf, wpow2, P, bhat + fd.bhat2);
   // Z_k = c_k conv_k; X_k = (Z_k + conj Z_{n-k})/2 and -i (Z_k - conj Z_{n-k})/2;
-  // phase_m = X_{m mod n} (conjugated above half) wgt e^{-i m phi0}, m <= mm
+  // phase_m = X_{m mod n} (conjugated above half) e^{-i m phi0}, m <= mm
   const bool rot0 = fabs(phi0[2 * p]) >= 1e-14, rot1 = fabs(phi0[2 * p + 1]) >= 1e-14;
-  const double w0 = ((flags & SHARP_USE_WEIGHTS) ? weight[2 * p] : 1.0) * scale;
-  const double w1 = ((flags & SHARP_USE_WEIGHTS) ? weight[2 * p + 1] : 1.0) * scale;
   double2 *d0 = phase + ((long long)(p * ncm + c) * 2) * ms, *d1 = d0 + ms;
   for (int m = threadIdx.x; m <= mm; m += NT) {
     const int idx = m % n;
@@ -1958,14 +1962,8 @@ ring2phase_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mli
       x0.y = -x0.y;
       x1.y = -x1.y;
     }
-    if (nr[0]) {
-      x0 = cscale(x0, w0);
-      d0[m] = rot0 ? cmul(x0, shift_of(slices, slices + kShiftLo, m)) : x0;
-    }
-    if (nr[1]) {
-      x1 = cscale(x1, w1);
-      d1[m] = rot1 ? cmul(x1, shift_of(slices + sl, slices + sl + kShiftLo, m)) : x1;
-    }
+    if (nr[0]) d0[m] = rot0 ? cmul(x0, shift_of(slices, slices + kShiftLo, m)) : x0;
+    if (nr[1]) d1[m] = rot1 ? cmul(x1, shift_of(slices + sl, slices + sl + kShiftLo, m)) : x1;
   }
 }
 
