@@ -15,6 +15,7 @@
 
 #include <cstdint>
 #include <memory>
+#include <utility>
 #include <vector>
 
 #include "sht_internal.h"
@@ -367,7 +368,7 @@ inline void launch_overlapped(void (*kernel)(P...), dim3 grid, int threads, size
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  SHT_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+  SHT_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
 }
 
 template <class K>

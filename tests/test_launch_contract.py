@@ -1,0 +1,45 @@
+"""Host side of the kernel launches: launch_overlapped takes only arguments that
+convert to the kernel's parameters by themselves, as a plain launch does."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+CUDA_INCLUDE = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+
+SOURCE = """
+#include "sht_device.h"
+void kernel(const double *, double2 *, long long);
+void launch(double *d, const double *cd, double2 *d2, const double2 *cd2, void *v, int n) {
+  sht::launch_overlapped(&kernel, dim3(1), 32, 0, nullptr, %s);
+}
+"""
+
+
+def _compiles(args, tmp_path):
+    src = tmp_path / "launch.cc"
+    src.write_text(SOURCE % args)
+    cmd = ["g++", "-std=c++17", "-fsyntax-only", "-I", CUDA_INCLUDE, "-I", os.path.join(ROOT, "include"),
+           "-I", os.path.join(ROOT, "planck-levels_b200", "csrc"), str(src)]
+    return subprocess.run(cmd, capture_output=True, text=True).returncode == 0
+
+
+needs_toolkit = pytest.mark.skipif(
+    shutil.which("g++") is None or not os.path.exists(os.path.join(CUDA_INCLUDE, "cuda_runtime.h")),
+    reason="needs g++ and the CUDA headers")
+
+
+@needs_toolkit
+@pytest.mark.parametrize("args", ["cd, d2, 1ll", "d, d2, n"])
+def test_matching_arguments_compile(args, tmp_path):
+    assert _compiles(args, tmp_path)
+
+
+@needs_toolkit
+@pytest.mark.parametrize("args", ["cd2, d2, 1ll", "cd, cd2, 1ll", "cd, d, 1ll", "v, d2, 1ll",
+                                  "cd, d2, d", "n, d2, 1ll", "cd, d2"])
+def test_mismatched_arguments_do_not_compile(args, tmp_path):
+    assert not _compiles(args, tmp_path)
