@@ -262,8 +262,13 @@ inline void allow_smem(K kernel, size_t bytes);
 // grid_release or ended), which hides the launch latency, 1 to 2 us a kernel
 // (Nside 64: a synthesis of three kernels takes 18.0 us, 23.4 without; an
 // analysis 20.6 and 26.6).  Every kernel launched like this calls grid_wait
-// before it reads or writes what an earlier kernel may use, and in any case
-// before it ends.
+// first of all: only past it are the writes of earlier kernels sure to be
+// visible, and a kernel that ended before its predecessor would release its own
+// successors too soon.  (Letting the ring kernels of one direction start on the
+// phase rows or maps before that, because the first of them had waited, was
+// worth 2.6% of the chi-square gradient at Nside 512 and 3.3% of three Jacobi
+// sweeps at Nside 1024, but rested on an ordering that the instruction does not
+// promise.)
 template <class... P, class... A>
 inline void launch_overlapped(void (*kernel)(P...), dim3 grid, int threads, size_t smem,
                               cudaStream_t st, A &&...args);

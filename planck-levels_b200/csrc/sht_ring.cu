@@ -66,30 +66,6 @@ __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -
 __device__ __forceinline__ double2 cscale(double2 a, double s) {
   return make_double2(a.x * s, a.y * s);
 }
-// The register ring kernels of one direction read the same phase rows or maps
-// and write disjoint rows, so each may start while its predecessor's last CTAs
-// run (launch_overlapped): a kernel lets its successor
-// start as soon as all its CTAs have started, and ends only after its
-// predecessor has, so that what follows the last one in the stream finds all
-// of them done.  The chi-square gradient at Nside 512 (three components, both
-// directions, four kernels each) takes 2.41 ms with it, 2.52 without; three
-// Jacobi sweeps at Nside 1024 11.8 against 12.2 ms.  The size-class kernels
-// stay out of it: their global scratch is reused from one to the next.
-// The first of a direction waits for what came before it, and only then lets the
-// others start; the last lets its successor start as grid_release_small does.
-constexpr int kChainFirst = 1, kChainLast = 2;
-struct GridChain {
-  int place;
-  __device__ __forceinline__ explicit GridChain(int p) : place(p) {
-    if (place & kChainFirst) grid_wait();
-    if (place & kChainLast) grid_release_small();
-    else grid_release();
-  }
-  __device__ __forceinline__ ~GridChain() {
-    if (!(place & kChainFirst)) grid_wait();
-  }
-};
-
 // FFT buffer (shared memory, or a CTA's slot of global scratch) whose element
 // index is swizzled inside aligned blocks of 8 entries (16-byte units):
 // e -> e ^ ((e >> 3) & 7).  The butterflies' strided stores (2, 4 or 8
@@ -994,9 +970,9 @@ phase2ring_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const int *__restrict__ fftidx, const FftDesc *__restrict__ fdesc,
                        const double2 *__restrict__ twiddle, const double2 *__restrict__ phase,
                        int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
-                       long long map_lo,
-                        int place) {
-  const GridChain chain(place);
+                       long long map_lo) {
+  grid_wait();
+  grid_release_small();
   extern __shared__ double2 smem[];
   __shared__ uint64_t row_full;
   double2 *buf = smem;
@@ -1096,9 +1072,9 @@ ring2phase_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const int *__restrict__ fftidx, const FftDesc *__restrict__ fdesc,
                        const double2 *__restrict__ twiddle, double2 *__restrict__ phase,
                        int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
-                       long long map_lo,
-                        int place) {
-  const GridChain chain(place);
+                       long long map_lo) {
+  grid_wait();
+  grid_release_small();
   extern __shared__ double2 smem[];
   double2 *buf = smem;
   double2 *slo = smem + pw_entries(N);
@@ -1268,9 +1244,9 @@ phase2ring_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const double2 *__restrict__ wpow2, int P,
                        const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                        const double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                       const __grid_constant__ PtrList maps, long long map_lo, int stage_row,
-                        int place) {
-  const GridChain chain(place);
+                       const __grid_constant__ PtrList maps, long long map_lo, int stage_row) {
+  grid_wait();
+  grid_release_small();
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   __shared__ uint64_t row_full;
@@ -1379,9 +1355,9 @@ ring2phase_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const double2 *__restrict__ wpow2, int P,
                        const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                        double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                       const __grid_constant__ PtrList maps, long long map_lo,
-                        int place) {
-  const GridChain chain(place);
+                       const __grid_constant__ PtrList maps, long long map_lo) {
+  grid_wait();
+  grid_release_small();
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   double2 *buf = smem;
@@ -1559,9 +1535,9 @@ phase2ring_short_kernel(const int *__restrict__ pairs, const int *__restrict__ m
                         const double2 *__restrict__ wpow2, int P,
                         const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                         const double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                        const __grid_constant__ PtrList maps, long long map_lo,
-                        int place) {
-  const GridChain chain(place);
+                        const __grid_constant__ PtrList maps, long long map_lo) {
+  grid_wait();
+  grid_release_small();
   extern __shared__ double2 smem[];
   double2 *buf = smem, *slo = buf + kShortEntries, *shi = slo + kShiftLo;
   const int p = pairs[blockIdx.x >> 1], h = blockIdx.x & 1, c = blockIdx.y;
@@ -1683,9 +1659,9 @@ ring2phase_short_kernel(const int *__restrict__ pairs, const int *__restrict__ m
                         const double2 *__restrict__ wpow2, int P,
                         const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                         double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                        const __grid_constant__ PtrList maps, long long map_lo,
-                        int place) {
-  const GridChain chain(place);
+                        const __grid_constant__ PtrList maps, long long map_lo) {
+  grid_wait();
+  grid_release_small();
   extern __shared__ double2 smem[];
   double2 *buf = smem, *slo = buf + kShortEntries, *shi = slo + kShiftLo;
   const int p = pairs[blockIdx.x >> 1], h = blockIdx.x & 1, c = blockIdx.y;
@@ -1827,9 +1803,9 @@ phase2ring_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mli
                       int P, const double2 *__restrict__ bhat,
                       const double2 *__restrict__ chirp, const double2 *__restrict__ phase,
                       int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
-                      long long map_lo,
-                        int place) {
-  const GridChain chain(place);
+                      long long map_lo) {
+  grid_wait();
+  grid_release_small();
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   double2 *buf = smem;
@@ -1910,9 +1886,9 @@ ring2phase_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mli
                       int P, const double2 *__restrict__ bhat,
                       const double2 *__restrict__ chirp, double2 *__restrict__ phase, int ncm,
                       int mmax, int flags, const __grid_constant__ PtrList maps,
-                      long long map_lo,
-                        int place) {
-  const GridChain chain(place);
+                      long long map_lo) {
+  grid_wait();
+  grid_release_small();
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   double2 *buf = smem;
@@ -2348,23 +2324,6 @@ void ring2phase_class(const JobDesc &job, const GeomPlan &gp, int cls, long long
 
 namespace {
 
-// Launches the register ring kernels of one direction (GridChain).
-struct RingStream {
-  cudaStream_t st;
-  int left;             // kernels to come
-  int place = kChainFirst;
-  RingStream(const GeomPlan &gp, cudaStream_t s) : st(s), left(gp.ps_count > 0 ? 1 : 0) {
-    for (const auto *v : {&gp.pw_count, &gp.pb_count, &gp.po_count})
-      for (int n : *v) left += n > 0;
-  }
-  template <class... P, class... A>
-  void launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, A &&...args) {
-    if (--left == 0) place |= kChainLast;
-    launch_overlapped(kernel, grid, threads, smem, st, args..., place);
-    place = 0;
-  }
-};
-
 size_t pow2_smem(int N, int mmax) {
   return sizeof(double2) * (size_t(pw_entries(N)) + kShiftLo + mmax / kShiftLo + 2);
 }
@@ -2372,11 +2331,11 @@ size_t pow2_smem(int N, int mmax) {
 template <typename T, int N>
 void phase2ring_pow2(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
                      const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
-                     RingStream &rs) {
+                     cudaStream_t st) {
   auto k = phase2ring_pow2_kernel<T, N>;
   const size_t smem = pow2_smem(N, job.mmax);
   allow_smem(k, smem);
-  rs.launch(k, dim3(2 * gp.pw_count[cls], nmapptr), N / 16, smem,
+  launch_overlapped(k, dim3(2 * gp.pw_count[cls], nmapptr), N / 16, smem, st,
       gp.pw_pairs + gp.pw_start[cls], gp.mlim, gp.nph, gp.ofs, gp.phi0, gp.shift,
       gp.shift_width, gp.weight, gp.fft,
       gp.fdesc, gp.twiddle, phase, ncm, job.mmax, job.flags,
@@ -2386,12 +2345,12 @@ void phase2ring_pow2(const JobDesc &job, const GeomPlan &gp, int cls, long long 
 template <typename T, int N>
 void ring2phase_pow2(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
                      const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
-                     RingStream &rs) {
+                     cudaStream_t st) {
   auto k = ring2phase_pow2_kernel<T, N>;
   // plus the twiddle slices of the unpacking
   const size_t smem = pow2_smem(N, job.mmax) + sizeof(double2) * (kTwLo + N / kTwLo + 1);
   allow_smem(k, smem);
-  rs.launch(k, dim3(2 * gp.pw_count[cls], nmapptr), N / 16, smem,
+  launch_overlapped(k, dim3(2 * gp.pw_count[cls], nmapptr), N / 16, smem, st,
       gp.pw_pairs + gp.pw_start[cls], gp.mlim, gp.nph, gp.ofs, gp.phi0, gp.shift,
       gp.shift_width, gp.weight, gp.fft,
       gp.fdesc, gp.twiddle, phase, ncm, job.mmax, job.flags,
@@ -2401,7 +2360,7 @@ void ring2phase_pow2(const JobDesc &job, const GeomPlan &gp, int cls, long long 
 template <typename T, int M>
 void phase2ring_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
                      const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
-                     RingStream &rs) {
+                     cudaStream_t st) {
   auto k = phase2ring_blue_kernel<T, M>;
   // the phase row is staged in shared memory where that keeps the CTAs per
   // SM (M = 8192: one CTA per SM either way) and fits
@@ -2410,7 +2369,7 @@ void phase2ring_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long 
   const int stage_row = (M == 8192 && with_row + 1024 <= 227 * 1024) ? 1 : 0;
   const size_t smem = stage_row ? with_row : base;
   allow_smem(k, smem);
-  rs.launch(k, dim3(2 * gp.pb_count[cls], nmapptr), M / 16, smem,
+  launch_overlapped(k, dim3(2 * gp.pb_count[cls], nmapptr), M / 16, smem, st,
       gp.pb_pairs + gp.pb_start[cls], gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.shift,
       gp.shift_width, gp.weight,
       gp.fft, gp.fdesc, gp.twiddle, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase, ncm, job.mmax,
@@ -2420,11 +2379,11 @@ void phase2ring_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long 
 template <typename T, int M>
 void ring2phase_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
                      const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
-                     RingStream &rs) {
+                     cudaStream_t st) {
   auto k = ring2phase_blue_kernel<T, M>;
   const size_t smem = pow2_smem(M, job.mmax);
   allow_smem(k, smem);
-  rs.launch(k, dim3(2 * gp.pb_count[cls], nmapptr), M / 16, smem,
+  launch_overlapped(k, dim3(2 * gp.pb_count[cls], nmapptr), M / 16, smem, st,
       gp.pb_pairs + gp.pb_start[cls], gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.shift,
       gp.shift_width, gp.weight,
       gp.fft, gp.fdesc, gp.twiddle, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase, ncm, job.mmax,
@@ -2433,13 +2392,13 @@ void ring2phase_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long 
 
 template <typename T, bool SYNTH>
 void odd_rings(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
-               const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm, RingStream &rs) {
+               const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm, cudaStream_t st) {
   auto length = [&](auto len) {
     constexpr int M = decltype(len)::value;
     const size_t smem = sizeof(double2) * odd_ring_smem_entries(M, job.mmax);
     auto go = [&](auto kernel) {
       allow_smem(kernel, smem);
-      rs.launch(kernel, dim3(gp.po_count[cls], nmapptr), M / 16, smem,
+      launch_overlapped(kernel, dim3(gp.po_count[cls], nmapptr), M / 16, smem, st,
           gp.po_pairs + gp.po_start[cls], gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.shift,
           gp.shift_width, gp.weight, gp.fft, gp.fdesc, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase,
           ncm, job.mmax, job.flags, maps_dev, map_lo);
@@ -2459,11 +2418,11 @@ void odd_rings(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo
 
 template <typename T, bool SYNTH>
 void short_rings(const JobDesc &job, const GeomPlan &gp, long long map_lo, const PtrList &maps_dev,
-                 int nmapptr, double2 *phase, int ncm, RingStream &rs) {
+                 int nmapptr, double2 *phase, int ncm, cudaStream_t st) {
   if (gp.ps_count == 0) return;
   const size_t smem = short_smem(job.mmax);
   auto go = [&](auto kernel) {
-    rs.launch(kernel, dim3(2 * gp.ps_count, nmapptr), 32, smem,
+    launch_overlapped(kernel, dim3(2 * gp.ps_count, nmapptr), 32, smem, st,
         gp.ps_pairs, gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.shift, gp.shift_width,
         gp.weight, gp.fft, gp.fdesc, gp.twiddle, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase, ncm,
         job.mmax, job.flags, maps_dev, map_lo);
@@ -2475,55 +2434,55 @@ void short_rings(const JobDesc &job, const GeomPlan &gp, long long map_lo, const
 template <typename T>
 void phase2ring_pow2_classes(const JobDesc &job, const GeomPlan &gp, long long map_lo,
                              const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
-                             RingStream &rs) {
+                             cudaStream_t st) {
   for (int c = int(gp.pw_N.size()) - 1; c >= 0; --c) {
     if (gp.pw_count[c] == 0) continue;
     switch (gp.pw_N[c]) {
-      case 1024: phase2ring_pow2<T, 1024>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs); break;
-      case 2048: phase2ring_pow2<T, 2048>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs); break;
-      case 4096: phase2ring_pow2<T, 4096>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs); break;
-      default: phase2ring_pow2<T, 8192>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs); break;
+      case 1024: phase2ring_pow2<T, 1024>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
+      case 2048: phase2ring_pow2<T, 2048>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
+      case 4096: phase2ring_pow2<T, 4096>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
+      default: phase2ring_pow2<T, 8192>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
     }
   }
   for (int c = int(gp.pb_M.size()) - 1; c >= 0; --c) {
     if (gp.pb_count[c] == 0) continue;
     switch (gp.pb_M[c]) {
-      case 1024: phase2ring_blue<T, 1024>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs); break;
-      case 2048: phase2ring_blue<T, 2048>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs); break;
-      case 4096: phase2ring_blue<T, 4096>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs); break;
-      default: phase2ring_blue<T, 8192>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs); break;
+      case 1024: phase2ring_blue<T, 1024>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
+      case 2048: phase2ring_blue<T, 2048>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
+      case 4096: phase2ring_blue<T, 4096>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
+      default: phase2ring_blue<T, 8192>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
     }
   }
   for (int c = int(gp.po_M.size()) - 1; c >= 0; --c)
-    odd_rings<T, true>(job, gp, c, map_lo, maps_dev, nmapptr, const_cast<double2 *>(phase), ncm, rs);
-  short_rings<T, true>(job, gp, map_lo, maps_dev, nmapptr, const_cast<double2 *>(phase), ncm, rs);
+    odd_rings<T, true>(job, gp, c, map_lo, maps_dev, nmapptr, const_cast<double2 *>(phase), ncm, st);
+  short_rings<T, true>(job, gp, map_lo, maps_dev, nmapptr, const_cast<double2 *>(phase), ncm, st);
 }
 
 template <typename T>
 void ring2phase_pow2_classes(const JobDesc &job, const GeomPlan &gp, long long map_lo,
                              const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
-                             RingStream &rs) {
+                             cudaStream_t st) {
   for (int c = int(gp.pw_N.size()) - 1; c >= 0; --c) {
     if (gp.pw_count[c] == 0) continue;
     switch (gp.pw_N[c]) {
-      case 1024: ring2phase_pow2<T, 1024>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs); break;
-      case 2048: ring2phase_pow2<T, 2048>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs); break;
-      case 4096: ring2phase_pow2<T, 4096>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs); break;
-      default: ring2phase_pow2<T, 8192>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs); break;
+      case 1024: ring2phase_pow2<T, 1024>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
+      case 2048: ring2phase_pow2<T, 2048>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
+      case 4096: ring2phase_pow2<T, 4096>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
+      default: ring2phase_pow2<T, 8192>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
     }
   }
   for (int c = int(gp.pb_M.size()) - 1; c >= 0; --c) {
     if (gp.pb_count[c] == 0) continue;
     switch (gp.pb_M[c]) {
-      case 1024: ring2phase_blue<T, 1024>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs); break;
-      case 2048: ring2phase_blue<T, 2048>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs); break;
-      case 4096: ring2phase_blue<T, 4096>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs); break;
-      default: ring2phase_blue<T, 8192>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs); break;
+      case 1024: ring2phase_blue<T, 1024>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
+      case 2048: ring2phase_blue<T, 2048>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
+      case 4096: ring2phase_blue<T, 4096>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
+      default: ring2phase_blue<T, 8192>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
     }
   }
   for (int c = int(gp.po_M.size()) - 1; c >= 0; --c)
-    odd_rings<T, false>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs);
-  short_rings<T, false>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, rs);
+    odd_rings<T, false>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+  short_rings<T, false>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, st);
 }
 
 }  // namespace
@@ -2532,11 +2491,10 @@ void launch_phase2ring(const JobDesc &job, const GeomPlan &gp, long long map_lo,
                        const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
                        cudaStream_t st) {
   ProfScope ps("ring_synth", st);
-  RingStream rs(gp, st);
   if (job.dp)
-    phase2ring_pow2_classes<double>(job, gp, map_lo, phase, ncm, maps_dev, nmapptr, rs);
+    phase2ring_pow2_classes<double>(job, gp, map_lo, phase, ncm, maps_dev, nmapptr, st);
   else
-    phase2ring_pow2_classes<float>(job, gp, map_lo, phase, ncm, maps_dev, nmapptr, rs);
+    phase2ring_pow2_classes<float>(job, gp, map_lo, phase, ncm, maps_dev, nmapptr, st);
   for (int cls = 0; cls < int(gp.cls_N.size()); ++cls) {
     if (gp.cls_count[cls] == 0) continue;
     if (job.dp)
@@ -2550,11 +2508,10 @@ void launch_ring2phase(const JobDesc &job, const GeomPlan &gp, long long map_lo,
                        const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
                        cudaStream_t st) {
   ProfScope ps("ring_anal", st);
-  RingStream rs(gp, st);
   if (job.dp)
-    ring2phase_pow2_classes<double>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, rs);
+    ring2phase_pow2_classes<double>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, st);
   else
-    ring2phase_pow2_classes<float>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, rs);
+    ring2phase_pow2_classes<float>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, st);
   for (int cls = 0; cls < int(gp.cls_N.size()); ++cls) {
     if (gp.cls_count[cls] == 0) continue;
     if (job.dp)

@@ -1,6 +1,9 @@
-"""Host side of the kernel launches: launch_overlapped takes only arguments that
-convert to the kernel's parameters by themselves, as a plain launch does."""
+"""The kernel launches, as far as the sources show it: launch_overlapped takes only
+arguments that convert to the kernel's parameters by themselves, as a plain launch
+does, and a kernel that may start early waits for its predecessor first of all."""
+import glob
 import os
+import re
 import shutil
 import subprocess
 
@@ -43,3 +46,16 @@ def test_matching_arguments_compile(args, tmp_path):
                                   "cd, d2, d", "n, d2, 1ll", "cd, d2"])
 def test_mismatched_arguments_do_not_compile(args, tmp_path):
     assert not _compiles(args, tmp_path)
+
+
+def test_early_kernels_wait_before_anything_else():
+    bodies = 0
+    for path in glob.glob(os.path.join(ROOT, "planck-levels_b200", "csrc", "*.cu")):
+        with open(path) as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        for call in re.finditer(r"grid_wait\(\)\s*;", text):
+            assert re.search(r"\)\s*\{\s*$", text[:call.start()]), (path, text[call.start() - 80:call.end()])
+            bodies += 1
+        for call in re.finditer(r"grid_release\w*\(\)\s*;", text):
+            assert re.search(r"grid_wait\(\)\s*;\s*$", text[:call.start()]), path
+    assert bodies >= 10
