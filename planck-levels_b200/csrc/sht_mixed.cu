@@ -38,7 +38,6 @@
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
-#include <vector>
 
 #include "sht_device.h"
 #include "sht_recurrence.cuh"
@@ -50,6 +49,22 @@ namespace {
 
 constexpr int kMC = 32;          // l-steps per chunk
 constexpr int kLP = kMC / 2;     // l-steps of one parity per chunk
+
+// Chunks of the orders below m, i.e. where the image of m begins: order k has
+// (lmax - max(k, spin)) / kMC + 1 (spin <= lmax, m <= lmax + 1).  In closed form,
+// so that no table has to be uploaded (one in pageable host memory would be gone
+// when a captured call is replayed).
+__host__ __device__ inline long long chunks_below(int m, int lmax, int spin) {
+  // sum over j = 0 .. n-1 of j / kMC + 1
+  auto sum = [](long long n) {
+    const long long q = n / kMC, r = n % kMC;
+    return kMC * (q * (q + 1) / 2) + r * (q + 1);
+  };
+  const long long low = m < spin ? m : spin;
+  long long n = low * ((lmax - spin) / kMC + 1);
+  if (m > spin) n += sum(lmax - spin + 1) - sum(lmax - m + 1);
+  return n;
+}
 constexpr int kKB = 4 * kLP;     // K bytes of one parity tile (64)
 constexpr int kRows = 128;       // ring pairs per row set (MMA M)
 constexpr int kRS = 2;           // row sets per CTA (256 ring pairs, 8 producer warps)
@@ -168,8 +183,8 @@ template <class S>
 __global__ void __launch_bounds__(256)
 mixed_image_kernel(int lmax, int spin, const long long *__restrict__ moff,
                    const double *__restrict__ ca, const double *__restrict__ cb,
-                   const double *__restrict__ cfac, const long long *__restrict__ ioff,
-                   const double2 *__restrict__ A, int ncA, int comp0,
+                   const double *__restrict__ cfac, const double2 *__restrict__ A, int ncA,
+                   int comp0,
                    unsigned char *__restrict__ img, double *__restrict__ epi) {
   constexpr int NCOL = S::NCOL, NCU = NCOL / 2;   // real columns, complex components
   constexpr int G = 256 / NCU;                    // l-groups of the scale pass
@@ -184,7 +199,7 @@ mixed_image_kernel(int lmax, int spin, const long long *__restrict__ moff,
   const long long mo = moff[m] - m;
   const int nch = (lmax - lbase + kMC) / kMC;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  unsigned char *base = img + ioff[m];
+  unsigned char *base = img + chunks_below(m, lmax, spin) * S::BLK;
   double *ep = epi + (long long)m * 3 * NCOL;
   auto bound = [&](int l) { return spin == 0 ? sqrt((2.0 * l + 1.0) / (4.0 * M_PI)) : 2.0; };
   // a_l * b_l of component c (both columns), zero where cfac is zero
@@ -373,9 +388,8 @@ mixed_synth_kernel(const int2 *__restrict__ items, const int *__restrict__ count
                    const double *__restrict__ cth, const double *__restrict__ sth,
                    const int *__restrict__ nph_ring, const double *__restrict__ pre_v,
                    const int *__restrict__ pre_e, int spin, const unsigned char *__restrict__ img,
-                   const long long *__restrict__ ioff, const double *__restrict__ epi, int lmax,
-                   double2 *__restrict__ phase, int ncm, int pcomp0, int ms,
-                   int *__restrict__ err) {
+                   const double *__restrict__ epi, int lmax, double2 *__restrict__ phase, int ncm,
+                   int pcomp0, int ms, int *__restrict__ err) {
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ uint64_t full_b[kSB], full_a[kSA], done[kSA];
   __shared__ uint32_t tslot;
@@ -386,7 +400,6 @@ mixed_synth_kernel(const int2 *__restrict__ items, const int *__restrict__ count
   const int mhi = max(m, spin);
   const int cnt = count[m];
   const int nch = mhi <= lmax ? (lmax - mhi + kMC) / kMC : 0;
-  const unsigned char *img_m = img + ioff[m];
   unsigned char *sB = sm;                         // kSB blocks
   unsigned char *sA = sm + kSB * S::BLK;          // kSA x kRS x ATILES tiles
 
@@ -410,6 +423,7 @@ mixed_synth_kernel(const int2 *__restrict__ items, const int *__restrict__ count
   if (warp == 4 * kRS) {
     // ---------------- loader / MMA issuer (lane 0 issues) ----------------
     if (nch > 0) {
+      const unsigned char *img_m = img + chunks_below(m, lmax, spin) * S::BLK;
       if (lane == 0) {
         const int npre = nch < kSB ? nch : kSB;
         for (int c = 0; c < npre; ++c) {
@@ -593,29 +607,17 @@ template <class S>
 void launch_shape(const JobDesc &job, const GeomPlan &gp, const CoefPlan &cp, const double2 *A,
                   int ncA, int t0, double2 *phase, int ncm, int *d_err, cudaStream_t st) {
   const int mmax = job.mmax, lmax = job.lmax, spin = job.spin;
-  std::vector<long long> ioff(mmax + 1);
-  long long tot = 0;
-  for (int m = 0; m <= mmax; ++m) {
-    ioff[m] = tot;
-    const int lbase = m > spin ? m : spin;
-    if (lbase <= lmax) tot += (long long)((lmax - lbase + kMC) / kMC) * S::BLK;
-  }
-  if (tot == 0) return;
+  const long long tot = chunks_below(mmax + 1, lmax, spin) * S::BLK;
   unsigned char *img = nullptr;
-  long long *d_ioff = nullptr;
   double *epi = nullptr;
   const size_t epi_bytes = sizeof(double) * 3 * S::NCOL * (mmax + 1);
   SHT_CUDA(::sht::ws_alloc(&img, size_t(tot), st));
-  SHT_CUDA(::sht::ws_alloc(&d_ioff, sizeof(long long) * (mmax + 1), st));
   SHT_CUDA(::sht::ws_alloc(&epi, epi_bytes, st));
-  SHT_CUDA(cudaMemcpyAsync(d_ioff, ioff.data(), sizeof(long long) * (mmax + 1),
-                           cudaMemcpyHostToDevice, st));
   SHT_CUDA(cudaMemsetAsync(epi, 0, epi_bytes, st));
   {
     ProfScope ps("mixed_image", st);
     mixed_image_kernel<S><<<mmax + 1, 256, 0, st>>>(lmax, spin, cp.d_moff, cp.alpha, cp.beta,
-                                                    cp.cfac, d_ioff, A, ncA, t0 * S::NCOMP, img,
-                                                    epi);
+                                                    cp.cfac, A, ncA, t0 * S::NCOMP, img, epi);
     SHT_CUDA(cudaGetLastError());
   }
   {
@@ -623,12 +625,11 @@ void launch_shape(const JobDesc &job, const GeomPlan &gp, const CoefPlan &cp, co
     auto k = mixed_synth_kernel<S>;
     SHT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
     k<<<int(gp.mixed_items.size()), kThreads, S::SMEM, st>>>(
-        gp.mitems, gp.count, gp.cth, gp.sth, gp.nph, cp.seed, cp.seed_exp, spin, img, d_ioff,
-        epi, lmax, phase, ncm, t0 * S::NCOMP, mmax + 1, d_err);
+        gp.mitems, gp.count, gp.cth, gp.sth, gp.nph, cp.seed, cp.seed_exp, spin, img, epi,
+        lmax, phase, ncm, t0 * S::NCOMP, mmax + 1, d_err);
     SHT_CUDA(cudaGetLastError());
   }
   SHT_CUDA(cudaFreeAsync(img, st));
-  SHT_CUDA(cudaFreeAsync(d_ioff, st));
   SHT_CUDA(cudaFreeAsync(epi, st));
 }
 
