@@ -84,3 +84,34 @@ def test_bitwise_as_alone(spin, flags):
         own = list(range(SETS))[t::2]
         for i, x in enumerate(results[t]):
             same(own[i % len(own)], x)
+
+
+@pytest.mark.parametrize("spin", [0, 2])
+def test_first_mixed_analyses_share_their_tables(spin):
+    # two geometries, one lmax: the batch runs them on two streams, and the first
+    # call after an emptied cache builds the coefficients that both use
+    import torch
+    lmax, flags = 500, sb.SHARP_DP | sb.SHARP_MIXED
+    ainfo = sb.AlmInfo.triangular(lmax)
+    geoms = [sb.Geometry.healpix(n) for n in (256, 128)]
+    rng = np.random.default_rng(spin)
+    nc = 1 if spin == 0 else 2
+    maps = [[torch.from_numpy(rng.uniform(-1, 1, g.npix())).cuda() for _ in range(nc)] for g in geoms]
+
+    def outputs():
+        return [[torch.zeros(2 * sb.nalm_triangular(lmax), dtype=torch.float64, device="cuda")
+                 for _ in range(nc)] for _ in geoms]
+
+    alone = outputs()
+    for g, m, a in zip(geoms, maps, alone):
+        sb.execute_device(sb.SHARP_MAP2ALM, spin, a, m, g, ainfo, 1, flags)
+        torch.cuda.synchronize()
+    for _ in range(5):
+        got = outputs()
+        torch.cuda.synchronize()
+        sb._lib.sharp_b200_release_cache()
+        sb.execute_batch([(sb.SHARP_MAP2ALM, spin, a, m, g, ainfo, 1, flags)
+                          for g, m, a in zip(geoms, maps, got)], device=True)
+        torch.cuda.synchronize()
+        assert all(torch.equal(x, y) for p, q in zip(got, alone) for x, y in zip(p, q))
+    sb.check_device_errors()
