@@ -744,10 +744,10 @@ bool tuner_on(int flags, cudaStream_t st) {
   return cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
 }
 
-// run(w) enqueues every pass of the job with width w on st; reset() undoes
-// what the timing runs accumulated.  Returns the width to use.
+// run(w) enqueues every pass of the job with width w on st; passes overwrite their
+// outputs, so the timing runs leave nothing behind.  Returns the width to use.
 int tuned_width(const TuneKey &key, int wmax, int wdefault, const std::function<void(int)> &run,
-                const std::function<void()> &reset, cudaStream_t st) {
+                cudaStream_t st) {
   std::lock_guard<std::mutex> lk(g_tune_mutex);
   auto it = g_tuned.find(key);
   if (it != g_tuned.end()) return it->second;
@@ -767,7 +767,6 @@ int tuned_width(const TuneKey &key, int wmax, int wdefault, const std::function<
   }
   SHT_CUDA(cudaEventDestroy(e0));
   SHT_CUDA(cudaEventDestroy(e1));
-  reset();
   float tdef = 0.f;
   for (auto &t : times)
     if (t.first == wdefault) tdef = t.second;
@@ -937,9 +936,8 @@ void execute_impl(sharp_jobtype type_in, int spin, void *alm, void *map,
       };
       int width = ntmax_synth;
       if (ntrans >= 2 && tuner_on(flags, st))
-        // synthesis passes overwrite the phase rows, so the timing runs leave nothing behind
         width = tuned_width(TuneKey{gp->hash, job.lmax, mmax, spin, type, ntrans, 0},
-                            ntmax_synth, ntmax_synth, passes, [] {}, st);
+                            ntmax_synth, ntmax_synth, passes, st);
       passes(width);
     }
     if (no_fft)
@@ -972,9 +970,8 @@ void execute_impl(sharp_jobtype type_in, int spin, void *alm, void *map,
       int width = ntmax_anal;
       const int wmax = spin == 0 ? 4 : gp->npairs <= kAnalWidePairs ? 2 : 1;
       if (ntrans >= 2 && wmax > 1 && tuner_on(flags, st))
-        // analysis passes overwrite Aout likewise
         width = tuned_width(TuneKey{gp->hash, job.lmax, mmax, spin, type, ntrans, 1}, wmax,
-                            ntmax_anal, passes, [] {}, st);
+                            ntmax_anal, passes, st);
       passes(width);
     }
     launch_scatter_alm(job, *ap, alm_lo, *cp, norm, reinterpret_cast<double *>(work_A), ncA, alms,
