@@ -139,7 +139,6 @@ int alm2map_noalloc(const sharp_geom_info *g, const sharp_alm_info *a, const voi
   const size_t o_mfac = L.take<double>(mmax + 1);
   const size_t o_mvs = L.take<long long>(mmax + 1);
   const size_t o_norm = L.take<double>(lmax + 1);
-  const size_t o_ptr = L.take<void *>(2);
   const size_t o_pw = L.take<int>(2);
   const size_t o_A = L.take<double2>(off);
   const size_t o_phase = L.take<double2>(size_t(2) * (mmax + 1) * std::max(np, 1));
@@ -178,8 +177,6 @@ int alm2map_noalloc(const sharp_geom_info *g, const sharp_alm_info *a, const voi
   put(o_mfac, mfac.data(), sizeof(double) * (mmax + 1));
   put(o_mvs, mvstart.data(), sizeof(long long) * (mmax + 1));
   put(o_norm, norm.data(), sizeof(double) * (lmax + 1));
-  const void *ptrs[2] = {alm, map};
-  put(o_ptr, ptrs, sizeof(ptrs));
 
   // ---- non-owning plan views over the scratch array --------------------------
   GeomPlan gp;
