@@ -277,12 +277,13 @@ __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;
 __device__ __forceinline__ void grid_release() {
   asm volatile("griddepcontrol.launch_dependents;");
 }
+constexpr unsigned kSmCount = 148;   // of a B200
 // Only a grid of at most two CTAs per SM: the CTAs of the next kernel take
 // whatever room there is, and beside a larger grid they end up unevenly spread
 // (Gauss grid of 251 pairs, three spin-1 transforms both ways: 554 us with an
 // early release of every grid, 471 with this, 490 without overlap).
 __device__ __forceinline__ void grid_release_small() {
-  if (gridDim.x * gridDim.y <= 2 * 148) grid_release();
+  if (gridDim.x * gridDim.y <= 2 * kSmCount) grid_release();
 }
 #endif
 
