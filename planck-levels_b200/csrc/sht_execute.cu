@@ -572,7 +572,8 @@ CoefPlan *get_coef_plan(int lmax, int mmax, int spin, cudaStream_t st) {
       norm[l] = (l < spin) ? 0. : spinsign * 0.5 * std::sqrt((2 * l + 1) / (4 * M_PI));
     if (spin == 1)
       for (int l = 0; l <= lmax; ++l)
-        norm[lmax + 1 + l] = (l < 1) ? 0. : 0.5 * std::sqrt(l * (l + 1.) * (2 * l + 1.) / (4 * M_PI));
+        norm[lmax + 1 + l] =
+            (l < 1) ? 0. : 0.5 * std::sqrt(l * (l + 1.) * (2 * l + 1.) / (4 * M_PI));
     cp->norm = dev_upload(norm, st);
   } else {
     std::vector<double> mfac(mmax + 1);

@@ -48,7 +48,8 @@ namespace {
 __device__ __forceinline__ double2 warp_reduce16(const double (&v)[16], double2 *buf) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int c = 0; c < 8; ++c) buf[lane * 8 + (c ^ (lane & 7))] = make_double2(v[2 * c], v[2 * c + 1]);
+  for (int c = 0; c < 8; ++c)
+    buf[lane * 8 + (c ^ (lane & 7))] = make_double2(v[2 * c], v[2 * c + 1]);
   __syncwarp();
   const int q = lane >> 3, c = lane & 7;
   double2 w[8];
@@ -607,24 +608,26 @@ synth_spin_kernel(const int2 *__restrict__ items, const int *__restrict__ count,
 }
 
 // ---------------------------------------------------------------------------
-// Analysis.  One CTA of W warps per m loops over tiles of 32*W*R ring pairs.  Per l-block (LB steps, LB*VPL == 32 values) every lane accumulates
-// its R rings' contributions; a warp transpose-reduction leaves one sum per
-// lane, kept in a per-warp shared array for the whole chunk.  After the next
-// chunk's barrier (the same one that publishes staged coefficients) the warps
-// share out the sub-blocks, add the warps' sums in a fixed order and store
-// them (first tile) or add them (later tiles; the same thread owns an entry
-// in every tile) to Aout, which this CTA owns: bitwise repeatable,
-// one barrier per kAChunk l-steps.  Every row l in [m, lmax] is written.
+// Analysis.  One CTA of W warps per m loops over tiles of 32*W*R ring pairs.
+// Per l-block (LB steps, LB*VPL == 16 values) every lane accumulates its R
+// rings' contributions; the sums over the warp (two each in lanes 0 .. 7) go to
+// a per-warp shared array for the whole chunk.  After the next chunk's barrier
+// (the same one that publishes staged coefficients) the warps share out the
+// sub-blocks, add the warps' sums in a fixed order and store them (first tile)
+// or add them (later tiles; the same thread owns an entry in every tile) to
+// Aout, which this CTA owns: bitwise repeatable, one barrier per kAChunk l-steps.
+// Every row l in [m, lmax] is written.
 //
-// The reduction through shared memory takes 42 instructions per 16 values;
-// recursive halving with shuffles took 107, more than half of them selects, and
-// left the FP64 pipe at 40%.  With it and the loops free of tests, Nside 1024 /
-// lmax 2048: spin 2 4.72 ms, spin 0 1.70 (before: 6.11 and 1.99); Nside 2048 /
-// lmax 4096: 32.9 and 11.8 (44.8 and 14.1).  Overlapping the reduction with the
-// next values' loop (WarpSums) is worth 1.5 ms of that at spin 2 (R = 3; R = 4
-// without it 34.4, with it 34.1).  Rings of a thread spread over the
-// tile (equal work for the warps between two barriers), with loops compiled for
-// each number of active ones: 5.1-5.3 and 1.94 ms, so a warp's rings stay
+// The reduction through shared memory takes 8 stores, 8 loads, 18 additions and
+// 8 shuffles per 16 values (warp_reduce16); recursive halving with shuffles took
+// 31 exchanges of a double per 32 values, each with two selects, two shuffles and
+// an addition, and left the FP64 pipe at 40%.  With the former and the loops free
+// of tests, Nside 1024 / lmax 2048: spin 2 4.72 ms, spin 0 1.70 (before: 6.11 and
+// 1.99); Nside 2048 / lmax 4096: 32.9 and 11.8 (44.8 and 14.1).  Overlapping the
+// reduction with the next values' loop (WarpSums) is worth 1.5 ms of that at spin
+// 2 (R = 3; R = 4 without it 34.4, with it 34.1).  Rings of a thread spread over
+// the tile (equal work for the warps between two barriers), with loops compiled
+// for each number of active ones: 5.1-5.3 and 1.94 ms, so a warp's rings stay
 // consecutive.  The contraction on the FP64 tensor instructions fills 4 (spin s)
 // or 2 (spin 0) of the 8 columns of an m8n8k4 with one transform: no gain.
 // ---------------------------------------------------------------------------
@@ -770,8 +773,8 @@ anal_spin0_kernel(const int *__restrict__ count, const double *__restrict__ cth,
       __syncthreads();
       stage(ch + 2);
       if (ch > 0)
-        flush_chunk<VPL, W>(wred[(ch - 1) & 1][0], nwarps, tb == 0, m + (ch - 1) * kAChunk, lmax, mo,
-                         ncA, comp0, Aout);
+        flush_chunk<VPL, W>(wred[(ch - 1) & 1][0], nwarps, tb == 0, m + (ch - 1) * kAChunk, lmax,
+                            mo, ncA, comp0, Aout);
       if (warp >= nwarps) continue;
       WarpSums ws{red[warp], nullptr};
       const double2 *ca = reinterpret_cast<const double2 *>(s_al[ch % 3]);
@@ -851,8 +854,8 @@ anal_spin0_kernel(const int *__restrict__ count, const double *__restrict__ cth,
     }
     __pipeline_wait_prior(0);
     __syncthreads();
-    flush_chunk<VPL, W>(wred[(nchunks - 1) & 1][0], nwarps, tb == 0, m + (nchunks - 1) * kAChunk, lmax,
-                     mo, ncA, comp0, Aout);
+    flush_chunk<VPL, W>(wred[(nchunks - 1) & 1][0], nwarps, tb == 0, m + (nchunks - 1) * kAChunk,
+                        lmax, mo, ncA, comp0, Aout);
     __syncthreads();
   }
 }
@@ -957,8 +960,8 @@ anal_spin_kernel(const int *__restrict__ count, const double *__restrict__ cth,
       __syncthreads();
       stage(ch + 2);
       if (ch > 0)
-        flush_chunk<VPL, W>(wred[(ch - 1) & 1][0], nwarps, tb == 0, mhi + (ch - 1) * kAChunk, lmax, mo,
-                         ncA, comp0, Aout);
+        flush_chunk<VPL, W>(wred[(ch - 1) & 1][0], nwarps, tb == 0, mhi + (ch - 1) * kAChunk, lmax,
+                            mo, ncA, comp0, Aout);
       if (warp >= nwarps) continue;
       WarpSums ws{red[warp], nullptr};
       const double2 *cab = s_ab[ch % 3];
@@ -985,15 +988,17 @@ anal_spin_kernel(const int *__restrict__ count, const double *__restrict__ cth,
 #pragma unroll
                   for (int k = 0; k < 4; ++k) {
                     // odd: +h3, -h2, -h1, +h0
-                    const double f = (i & 1) ? ((k == 1 || k == 2) ? -h[r][j][3 - k] : h[r][j][3 - k])
-                                             : h[r][j][k];
+                    const double f = !(i & 1)             ? h[r][j][k]
+                                     : (k == 1 || k == 2) ? -h[r][j][3 - k]
+                                                          : h[r][j][3 - k];
                     o[k] = r == 0 ? ep * f : fma(ep, f, o[k]);
                   }
 #pragma unroll
                   for (int k = 0; k < 4; ++k) {
                     // odd: -g3, +g2, +g1, -g0
-                    const double f = (i & 1) ? ((k == 1 || k == 2) ? g[r][j][3 - k] : -g[r][j][3 - k])
-                                             : g[r][j][k];
+                    const double f = !(i & 1)             ? g[r][j][k]
+                                     : (k == 1 || k == 2) ? g[r][j][3 - k]
+                                                          : -g[r][j][3 - k];
                     o[k] = fma(em, f, o[k]);
                   }
                 }
@@ -1055,7 +1060,7 @@ anal_spin_kernel(const int *__restrict__ count, const double *__restrict__ cth,
     __pipeline_wait_prior(0);
     __syncthreads();
     flush_chunk<VPL, W>(wred[(nchunks - 1) & 1][0], nwarps, tb == 0, mhi + (nchunks - 1) * kAChunk,
-                     lmax, mo, ncA, comp0, Aout);
+                        lmax, mo, ncA, comp0, Aout);
     __syncthreads();
   }
 }

@@ -505,19 +505,17 @@ __device__ __forceinline__ double2 shift_of(const double2 *lo, const double2 *hi
 // phase -> ring (synthesis).  Grid: (pairs of one size class, components).
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(1024) phase2ring_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
-                                  const int *__restrict__ nph, const long long *__restrict__ ofs,
-                                  const int *__restrict__ stride, const double *__restrict__ phi0,
-                       const double2 *__restrict__ shift, int sw,
-                                  const double *__restrict__ weight, const int *__restrict__ fftidx,
-                                  const FftDesc *__restrict__ fdesc,
-                                  const double2 *__restrict__ twiddle,
-                                  const double2 *__restrict__ wpow2, int P,
-                                  const double2 *__restrict__ bhat,
-                                  const double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                                  int nbufA, int nbufB, int twcap, const __grid_constant__ PtrList maps,
-                                  long long map_lo, double2 *__restrict__ gbuf, int npc,
-                                  int nitems) {
+__global__ void __launch_bounds__(1024)
+phase2ring_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
+                  const int *__restrict__ nph, const long long *__restrict__ ofs,
+                  const int *__restrict__ stride, const double *__restrict__ phi0,
+                  const double2 *__restrict__ shift, int sw, const double *__restrict__ weight,
+                  const int *__restrict__ fftidx, const FftDesc *__restrict__ fdesc,
+                  const double2 *__restrict__ twiddle, const double2 *__restrict__ wpow2, int P,
+                  const double2 *__restrict__ bhat, const double2 *__restrict__ phase, int ncm,
+                  int mmax, int flags, int nbufA, int nbufB, int twcap,
+                  const __grid_constant__ PtrList maps, long long map_lo,
+                  double2 *__restrict__ gbuf, int npc, int nitems) {
   extern __shared__ double2 smem[];
   const int ms = mmax + 1;
   // SHARP_SUBTRACT: the negated result is added (negation is exact)
@@ -556,8 +554,8 @@ __global__ void __launch_bounds__(1024) phase2ring_kernel(const int *__restrict_
     const Buf C{bufB}, Ab{bufA};
     const double2 *src = phase + ((long long)(p * ncm + c) * 2 + h) * ms;
     if (rot)
-      load_shift(slo, shi, mm, ph, false, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
-                 blockDim.x);
+      load_shift(slo, shi, mm, ph, false, shift ? shift + size_t(ring) * sw : nullptr,
+                 threadIdx.x, blockDim.x);
     load_twshared(twlo, twhi, twiddle + d.tw, n);
     __syncthreads();
     // fold phase_m * wgt * e^{i m phi0} into bins 0..half (sharp.c:265-300);
@@ -623,18 +621,17 @@ __global__ void __launch_bounds__(1024) phase2ring_kernel(const int *__restrict_
 // ring -> phase (analysis)
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(1024) ring2phase_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
-                                  const int *__restrict__ nph, const long long *__restrict__ ofs,
-                                  const int *__restrict__ stride, const double *__restrict__ phi0,
-                       const double2 *__restrict__ shift, int sw,
-                                  const double *__restrict__ weight, const int *__restrict__ fftidx,
-                                  const FftDesc *__restrict__ fdesc,
-                                  const double2 *__restrict__ twiddle,
-                                  const double2 *__restrict__ wpow2, int P,
-                                  const double2 *__restrict__ bhat, double2 *__restrict__ phase,
-                                  int ncm, int mmax, int flags, int nbufA, int nbufB, int twcap,
-                                  const __grid_constant__ PtrList maps, long long map_lo,
-                                  double2 *__restrict__ gbuf, int npc, int nitems) {
+__global__ void __launch_bounds__(1024)
+ring2phase_kernel(const int *__restrict__ pairs, const int *__restrict__ mlim,
+                  const int *__restrict__ nph, const long long *__restrict__ ofs,
+                  const int *__restrict__ stride, const double *__restrict__ phi0,
+                  const double2 *__restrict__ shift, int sw, const double *__restrict__ weight,
+                  const int *__restrict__ fftidx, const FftDesc *__restrict__ fdesc,
+                  const double2 *__restrict__ twiddle, const double2 *__restrict__ wpow2, int P,
+                  const double2 *__restrict__ bhat, double2 *__restrict__ phase, int ncm,
+                  int mmax, int flags, int nbufA, int nbufB, int twcap,
+                  const __grid_constant__ PtrList maps, long long map_lo,
+                  double2 *__restrict__ gbuf, int npc, int nitems) {
   extern __shared__ double2 smem[];
   const int ms = mmax + 1;
   const double wscale = (flags & SHARP_REAL_HARMONICS) ? kSqrtTwo : 1.0;
@@ -667,8 +664,8 @@ __global__ void __launch_bounds__(1024) ring2phase_kernel(const int *__restrict_
     const long long o = ofs[ring] - map_lo;
     const long long st = stride[ring];
     if (rot)
-      load_shift(slo, shi, mm, ph, true, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
-                 blockDim.x);
+      load_shift(slo, shi, mm, ph, true, shift ? shift + size_t(ring) * sw : nullptr,
+                 threadIdx.x, blockDim.x);
     load_twshared(twlo, twhi, twiddle + d.tw, n);
     const Buf Ab{bufA};
     if ((n & 1) == 0) {
@@ -823,7 +820,8 @@ __device__ __forceinline__ void mul_powers(double2 (&v)[16], double2 w1) {
 // is the entry at base + s i (s = len/16, base = (u/s) len + k0, k0 = u mod s).
 template <int N, bool INV>
 __device__ __forceinline__ void pw_pass16_regs(double2 (&v)[16], double2 *buf, int len,
-                                               const double2 *__restrict__ W, int tl, int u = threadIdx.x) {
+                                               const double2 *__restrict__ W, int tl,
+                                               int u = threadIdx.x) {
   const int s = len >> 4;
   const int k0 = u & (s - 1);
   const int base = (u / s) * len + k0;
@@ -858,7 +856,9 @@ __device__ __forceinline__ void pw_pass16(double2 *buf, int len, const double2 *
 }
 
 // Lanes 0 .. n-1 of a warp.
-__device__ __forceinline__ unsigned sub_warp(int n) { return n >= 32 ? 0xffffffffu : (1u << n) - 1; }
+__device__ __forceinline__ unsigned sub_warp(int n) {
+  return n >= 32 ? 0xffffffffu : (1u << n) - 1;
+}
 // Barrier between passes: of the CTA, or of the THREADS first lanes of a warp.
 template <bool WARP, int THREADS>
 __device__ __forceinline__ void pw_sync() {
@@ -884,7 +884,8 @@ __device__ __forceinline__ void pw_pass_last(double2 *buf, int u = threadIdx.x) 
 // The passes of pw_fft after the first (which the caller ran from registers
 // with pw_pass16_regs and a __syncthreads).
 template <int N, bool INV, bool WARP = false>
-__device__ void pw_fft_rest(double2 *buf, const double2 *__restrict__ W, int tl, int u = threadIdx.x) {
+__device__ void pw_fft_rest(double2 *buf, const double2 *__restrict__ W, int tl,
+                            int u = threadIdx.x) {
   int len = N >> 4;
 #pragma unroll
   for (int q = 1; q < pw_passes16(N); ++q) {
@@ -923,7 +924,8 @@ __device__ void pw_fft(double2 *buf, const double2 *__restrict__ W, int tl) {
 // i >= NOUT are not stored.
 template <int N, int NOUT = 16>
 __device__ __forceinline__ void pw_pass16_back(double2 *buf, int len,
-                                               const double2 *__restrict__ W, int tl, int u = threadIdx.x) {
+                                               const double2 *__restrict__ W, int tl,
+                                               int u = threadIdx.x) {
   const int s = len >> 4;
   const int k0 = u & (s - 1);
   const int base = (u / s) * len + k0;
@@ -1010,8 +1012,8 @@ phase2ring_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
   }
   if constexpr (kSlices) load_twshared(twl, twh, W, N);   // W: the table of 2N entries
   if (rot)
-      load_shift(slo, shi, mm, ph, false, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
-                 blockDim.x);
+    load_shift(slo, shi, mm, ph, false, shift ? shift + size_t(ring) * sw : nullptr,
+               threadIdx.x, blockDim.x);
   // a copy that did not complete within the bounded wait is redone by the
   // threads from global memory (the same values, so a late bulk write
   // changes nothing)
@@ -1093,8 +1095,8 @@ ring2phase_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
   const double2 *W = twiddle + fdesc[fftidx[ring]].tw;
   const T *map = static_cast<const T *>(maps.p[c]) + (ofs[ring] - map_lo);
   if (rot)
-      load_shift(slo, shi, mm, ph, true, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
-                 blockDim.x);
+    load_shift(slo, shi, mm, ph, true, shift ? shift + size_t(ring) * sw : nullptr,
+               threadIdx.x, blockDim.x);
   load_twshared(twl, twh, W, N + 1);   // W: the table of 2N entries
   // pixels 2j, 2j+1 for j = tid + (N/16) s2: this thread's inputs of the
   // first pass, which runs from registers
@@ -1286,8 +1288,8 @@ phase2ring_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
     }
   }
   if (rot)
-      load_shift(slo, shi, mm, ph, false, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
-                 blockDim.x);
+    load_shift(slo, shi, mm, ph, false, shift ? shift + size_t(ring) * sw : nullptr,
+               threadIdx.x, blockDim.x);
   if (stage_row) {
     // a copy that did not complete within the bounded wait is redone by
     // the threads (the same values)
@@ -1381,8 +1383,8 @@ ring2phase_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
   const T *map = static_cast<const T *>(maps.p[c]) + (ofs[ring] - map_lo);
   const long long st = stride[ring];
   if (rot)
-      load_shift(slo, shi, mm, ph, true, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
-                 blockDim.x);
+    load_shift(slo, shi, mm, ph, true, shift ? shift + size_t(ring) * sw : nullptr,
+               threadIdx.x, blockDim.x);
   // x_j c_j, x_j = pixels 2j + i (2j+1), zero on [N, M): for j = tid + NT i
   // this thread's inputs of the first forward pass, run from registers
   double2 v[16];
@@ -1559,8 +1561,8 @@ phase2ring_short_kernel(const int *__restrict__ pairs, const int *__restrict__ m
   const long long st = stride[ring];
   const bool vec = px2_vec(map, st);
   if (rot) {
-    load_shift(slo, shi, mm, ph, false, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
-               32);
+    load_shift(slo, shi, mm, ph, false, shift ? shift + size_t(ring) * sw : nullptr,
+               threadIdx.x, 32);
     __syncwarp();
   }
   auto tm = [&](int m) {
@@ -1681,8 +1683,8 @@ ring2phase_short_kernel(const int *__restrict__ pairs, const int *__restrict__ m
   const bool vec = px2_vec(map, st);
   double2 *dst = phase + ((long long)(p * ncm + c) * 2 + h) * ms;
   if (rot)
-    load_shift(slo, shi, mm, ph, true, shift ? shift + size_t(ring) * sw : nullptr, threadIdx.x,
-               32);
+    load_shift(slo, shi, mm, ph, true, shift ? shift + size_t(ring) * sw : nullptr,
+               threadIdx.x, 32);
   // phase_m = X_{m mod n} (conjugated above N) wgt e^{-i m phi0}, m <= mm
   auto write = [&](const auto &x_at) {
     for (int m = threadIdx.x; m <= mm; m += 32) {
@@ -2294,11 +2296,10 @@ void phase2ring_class(const JobDesc &job, const GeomPlan &gp, int cls, long long
   auto k = phase2ring_kernel<T>;
   allow_smem(k, L.smem);
   k<<<L.grid, L.thr, L.smem, st>>>(gp.cls_pairs + gp.cls_start[cls], gp.mlim, gp.nph, gp.ofs,
-                                   gp.stride, gp.phi0, gp.shift, gp.shift_width, gp.weight, gp.fft, gp.fdesc, gp.twiddle,
-                                   gp.wpow2, gp.P, gp.bhat, phase, ncm, job.mmax, job.flags,
-                                   gp.cls_bufA[cls], gp.cls_bufB[cls], fft_twcap(gp),
-                                   maps_dev, map_lo, L.gbuf, L.npc,
-                                   L.nitems);
+                                   gp.stride, gp.phi0, gp.shift, gp.shift_width, gp.weight,
+                                   gp.fft, gp.fdesc, gp.twiddle, gp.wpow2, gp.P, gp.bhat, phase,
+                                   ncm, job.mmax, job.flags, gp.cls_bufA[cls], gp.cls_bufB[cls],
+                                   fft_twcap(gp), maps_dev, map_lo, L.gbuf, L.npc, L.nitems);
   SHT_CUDA(cudaGetLastError());
   if (L.gbuf) SHT_CUDA(cudaFreeAsync(L.gbuf, st));
 }
@@ -2311,11 +2312,10 @@ void ring2phase_class(const JobDesc &job, const GeomPlan &gp, int cls, long long
   auto k = ring2phase_kernel<T>;
   allow_smem(k, L.smem);
   k<<<L.grid, L.thr, L.smem, st>>>(gp.cls_pairs + gp.cls_start[cls], gp.mlim, gp.nph, gp.ofs,
-                                   gp.stride, gp.phi0, gp.shift, gp.shift_width, gp.weight, gp.fft, gp.fdesc, gp.twiddle,
-                                   gp.wpow2, gp.P, gp.bhat, phase, ncm, job.mmax, job.flags,
-                                   gp.cls_bufA[cls], gp.cls_bufB[cls], fft_twcap(gp),
-                                   maps_dev, map_lo, L.gbuf,
-                                   L.npc, L.nitems);
+                                   gp.stride, gp.phi0, gp.shift, gp.shift_width, gp.weight,
+                                   gp.fft, gp.fdesc, gp.twiddle, gp.wpow2, gp.P, gp.bhat, phase,
+                                   ncm, job.mmax, job.flags, gp.cls_bufA[cls], gp.cls_bufB[cls],
+                                   fft_twcap(gp), maps_dev, map_lo, L.gbuf, L.npc, L.nitems);
   SHT_CUDA(cudaGetLastError());
   if (L.gbuf) SHT_CUDA(cudaFreeAsync(L.gbuf, st));
 }
@@ -2438,23 +2438,38 @@ void phase2ring_pow2_classes(const JobDesc &job, const GeomPlan &gp, long long m
   for (int c = int(gp.pw_N.size()) - 1; c >= 0; --c) {
     if (gp.pw_count[c] == 0) continue;
     switch (gp.pw_N[c]) {
-      case 1024: phase2ring_pow2<T, 1024>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
-      case 2048: phase2ring_pow2<T, 2048>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
-      case 4096: phase2ring_pow2<T, 4096>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
-      default: phase2ring_pow2<T, 8192>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
+      case 1024:
+        phase2ring_pow2<T, 1024>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        break;
+      case 2048:
+        phase2ring_pow2<T, 2048>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        break;
+      case 4096:
+        phase2ring_pow2<T, 4096>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        break;
+      default:
+        phase2ring_pow2<T, 8192>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
     }
   }
   for (int c = int(gp.pb_M.size()) - 1; c >= 0; --c) {
     if (gp.pb_count[c] == 0) continue;
     switch (gp.pb_M[c]) {
-      case 1024: phase2ring_blue<T, 1024>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
-      case 2048: phase2ring_blue<T, 2048>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
-      case 4096: phase2ring_blue<T, 4096>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
-      default: phase2ring_blue<T, 8192>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st); break;
+      case 1024:
+        phase2ring_blue<T, 1024>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        break;
+      case 2048:
+        phase2ring_blue<T, 2048>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        break;
+      case 4096:
+        phase2ring_blue<T, 4096>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        break;
+      default:
+        phase2ring_blue<T, 8192>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
     }
   }
   for (int c = int(gp.po_M.size()) - 1; c >= 0; --c)
-    odd_rings<T, true>(job, gp, c, map_lo, maps_dev, nmapptr, const_cast<double2 *>(phase), ncm, st);
+    odd_rings<T, true>(job, gp, c, map_lo, maps_dev, nmapptr, const_cast<double2 *>(phase), ncm,
+                       st);
   short_rings<T, true>(job, gp, map_lo, maps_dev, nmapptr, const_cast<double2 *>(phase), ncm, st);
 }
 
@@ -2465,19 +2480,33 @@ void ring2phase_pow2_classes(const JobDesc &job, const GeomPlan &gp, long long m
   for (int c = int(gp.pw_N.size()) - 1; c >= 0; --c) {
     if (gp.pw_count[c] == 0) continue;
     switch (gp.pw_N[c]) {
-      case 1024: ring2phase_pow2<T, 1024>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
-      case 2048: ring2phase_pow2<T, 2048>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
-      case 4096: ring2phase_pow2<T, 4096>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
-      default: ring2phase_pow2<T, 8192>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
+      case 1024:
+        ring2phase_pow2<T, 1024>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        break;
+      case 2048:
+        ring2phase_pow2<T, 2048>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        break;
+      case 4096:
+        ring2phase_pow2<T, 4096>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        break;
+      default:
+        ring2phase_pow2<T, 8192>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
     }
   }
   for (int c = int(gp.pb_M.size()) - 1; c >= 0; --c) {
     if (gp.pb_count[c] == 0) continue;
     switch (gp.pb_M[c]) {
-      case 1024: ring2phase_blue<T, 1024>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
-      case 2048: ring2phase_blue<T, 2048>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
-      case 4096: ring2phase_blue<T, 4096>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
-      default: ring2phase_blue<T, 8192>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st); break;
+      case 1024:
+        ring2phase_blue<T, 1024>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        break;
+      case 2048:
+        ring2phase_blue<T, 2048>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        break;
+      case 4096:
+        ring2phase_blue<T, 4096>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        break;
+      default:
+        ring2phase_blue<T, 8192>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
     }
   }
   for (int c = int(gp.po_M.size()) - 1; c >= 0; --c)
