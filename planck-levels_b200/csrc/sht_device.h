@@ -96,13 +96,37 @@ inline int pow2_ring_length(int nph, int stride, int mm) {
 // folding) whose complex length either calls for a Bluestein convolution by
 // the cost model of the size classes or exceeds 1024 (there the size-class
 // kernel, one 1024-thread CTA per SM, ran the mixed-radix Stockham passes
-// about twice as slowly per ring as the register convolution); with all set,
-// every ring that has such an M.
+// about twice as slowly per ring as the register convolution); with all set
+// (every plan but that of the allocation-free synthesis) every ring that has
+// such an M, but see smooth_ring_length.
 constexpr int kRegBluesteinMinN = 1024;
 inline int blue_ring_length(int nph, const FftDesc &d, bool all) {
   if (nph <= 0 || (nph & 1)) return 0;
   if (!all && !d.blue && d.N <= kRegBluesteinMinN) return 0;
   return (d.M == 1024 || d.M == 2048 || d.M == 4096 || d.M == 8192) ? d.M : 0;
+}
+// Whether an even ring has a complex length N in (512, 1024] without factors
+// above 5, whose direct passes in the size classes take less than the
+// convolution of length 2048.  Ring FFTs of a Gauss grid of nph pixels per ring,
+// 6 components, us, direct and convolution (synthesis / analysis):
+//   nph 1000: 58 / 56  50 / 42    1080: 66 / 65  93 / 85    1200: 73 / 72  105 / 95
+//       1536: 95 / 93  139 / 123  1800: 134 / 131  179 / 149
+//       2000: 144 / 140  203 / 166
+// With a factor 7 the convolution takes less (1120: 90 / 88, 97 / 88; 1400: 150
+// / 147, 125 / 111) and with larger ones half or a quarter.  In a geometry that
+// has at least as many other rings with that convolution they share its launch
+// (convolution_takes_smooth): HEALPix Nside 512, 3 components: 165 / 143 us with
+// its smooth rings in the size classes, 145 / 122 without.
+inline bool smooth_ring_length(int nph) {
+  if (nph <= 0 || (nph & 1)) return false;
+  int N = nph / 2;
+  if (N <= 512 || N > 1024) return false;
+  for (int p : {2, 3, 5})
+    while (N % p == 0) N /= p;
+  return N == 1;
+}
+inline bool convolution_takes_smooth(size_t smooth_pairs, size_t other_pairs) {
+  return other_pairs >= smooth_pairs;
 }
 // How the short-ring kernels run an even ring of complex length N, or kNone:
 // directly (N <= 32), by the passes of length L = N (64 .. 512, a power of two),

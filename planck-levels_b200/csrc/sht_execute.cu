@@ -303,6 +303,7 @@ GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin,
   // length); a length whose buffer and phi0 slices exceed the shared memory
   // of a CTA stays in the size classes
   std::map<int, std::vector<int>> pw_lists, pb_lists, po_lists;
+  std::vector<int> smooth;   // pairs of smooth_ring_length that have a convolution
   // 1: power-of-two pair, 2: pair with a register Bluestein convolution
   std::vector<char> is_pw(np, 0);
   auto fits = [&](int len) {
@@ -311,7 +312,7 @@ GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin,
   for (int p = 0; p < np; ++p) {
     const int mm = std::min(mmax, h.mlim_sorted[p]);
     int N = -1, M = -1;
-    bool is_short = registers, sblue = false;
+    bool is_short = registers, sblue = false, is_smooth = registers;
     for (int hh = 0; hh < 2; ++hh) {
       const int i = 2 * p + hh;
       if (h.nph[i] <= 0) continue;
@@ -320,6 +321,7 @@ GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin,
       is_short = is_short && !(h.nph[i] & 1) &&
                  short_ring_kind(h.nph[i] / 2, &len, &blue) != ShortKind::kNone;
       if (is_short && h.nph[i] > 64 && blue) sblue = true;
+      is_smooth = is_smooth && smooth_ring_length(h.nph[i]);
       const int n = pow2_ring_length(h.nph[i], h.stride[i], mm);
       N = (N < 0 || N == n) ? n : 0;
       const int b = blue_ring_length(h.nph[i], h.descs[h.fft[i]], registers);
@@ -336,8 +338,20 @@ GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin,
       pw_lists[N].push_back(p);
       is_pw[p] = 1;
     } else if (M > 0 && fits(M)) {
-      pb_lists[M].push_back(p);
-      is_pw[p] = 2;
+      if (is_smooth) {
+        smooth.push_back(p);
+      } else {
+        pb_lists[M].push_back(p);
+        is_pw[p] = 2;
+      }
+    }
+  }
+  if (!smooth.empty()) {
+    std::vector<int> &other = pb_lists[2048];   // the M of all of them
+    if (convolution_takes_smooth(smooth.size(), other.size())) {
+      for (int p : smooth) is_pw[p] = 2;
+      other.insert(other.end(), smooth.begin(), smooth.end());
+      std::sort(other.begin(), other.end());
     }
   }
   for (auto &kv : pw_lists) {
