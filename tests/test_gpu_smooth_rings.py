@@ -44,7 +44,8 @@ def _kernels(geom, lmax, npix):
         torch.cuda.synchronize()
     both()
     with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        both()
+        for _ in range(5):   # the trace may lack the first kernels
+            both()
     names = [e.key for e in prof.key_averages()]
     if not any("legendre" in n or "spin0" in n for n in names):
         pytest.skip("no kernel trace on this machine")
