@@ -312,9 +312,26 @@ __device__ __forceinline__ void grid_release_small() {
 #endif
 
 // Kernel launchers (sht_legendre.cu)
-// Ring pairs up to which the spin analysis takes two transforms per pass (above,
-// three rings per thread leave no registers for a second one).
-constexpr int kAnalWidePairs = 512;
+// Whether the analysis runs CTAs of eight warps with two ring pairs per thread
+// (tiles of 512 pairs), 257 .. 512 pairs: one tile, whose sums over rings end early
+// for few l.  For many l the sums cost more than the shorter chain gives and four
+// warps with more rings per thread take less, at spin s as long as one tile of
+// theirs (384 pairs) holds all.  Whole analyses, us, eight warps and four (R4 at
+// spin 0, R3 at spin 2), pairs / lmax = mmax:
+//   spin 0  257/700: 83, 96   384/500: 62, 71   512/500: 67, 78   512/700: 107, 107
+//           320/1000: 158, 139  512/1000: 189, 164  512/2000: 673, 529
+//   spin 2  512/500: 146, 201  384/700: 217, 181  512/2000: 1603, 1629
+//           257/1000: 340, 290  384/1000: 401, 318  384/2000: 1451, 1117
+// (mmax 300, spin 0: 257/1000 112, 128  290/1000 123, 117  512/2000 312, 256.)
+inline bool anal_eight_warps(int spin, int npairs, int lmax) {
+  if (npairs <= 256 || npairs > 512) return false;
+  return lmax <= 750 || (spin == 0 ? npairs <= 288 : npairs > 384);
+}
+// Whether the spin analysis takes two transforms per pass (three rings per thread
+// leave no registers for a second one).
+inline bool anal_spin_wide(int spin, int npairs, int lmax) {
+  return npairs <= 256 || anal_eight_warps(spin, npairs, lmax);
+}
 void launch_coef_tables(CoefPlan &cp, cudaStream_t st);
 void launch_legendre_synth(const JobDesc &job, const GeomPlan &gp, const CoefPlan &cp,
                            const double2 *A, int ncA, int comp0, int nt,

@@ -728,7 +728,7 @@ double wall_now() {
 // Pass-width tuner, the counterpart of the reference's nv oracle
 // (libsharp/sharp.c:890-965, which times its SIMD vector counts on first
 // use): the FP64 Legendre kernels take 1, 2 or 4 transforms per pass (spin s
-// and deriv1: 1 or 2); wider passes share one recurrence, narrower ones keep
+// and deriv1: 1 or 2; spin analysis only where anal_spin_wide); wider passes share one recurrence, narrower ones keep
 // more CTAs per SM, and which wins depends on the geometry, lmax and spin.
 // The first job of a shape with several transforms times each width once on
 // its own buffers (after one untimed run of it; one host synchronisation per
@@ -921,10 +921,9 @@ void execute_impl(sharp_jobtype type_in, int spin, void *alm, void *map,
   double2 *phase = d_work.as<double2>();
   double2 *work_A = reinterpret_cast<double2 *>(d_work.as<char>() + a_at);
   const int ntmax_synth = (spin == 0 && !deriv) ? 4 : 2;
-  // FP64 analysis: one transform per launch is fastest per transform (the
-  // per-thread phase factors of several transforms cost occupancy): at Nside
-  // 2048 / lmax 4096, spin 0 takes 14.1 ms at 1, 15.2 ms each at 4; spin 2
-  // takes 44.9 ms at 1, 54.1 ms each at 2.
+  // FP64 analysis: one transform per launch is the default (the per-thread phase
+  // factors of several transforms cost occupancy); where a wider pass takes less,
+  // the tuner finds it
   const int ntmax_anal = 1;
   auto group = [&](int left, int ntmax) {
     int nt = 1;
@@ -983,7 +982,7 @@ void execute_impl(sharp_jobtype type_in, int spin, void *alm, void *map,
         }
       };
       int width = ntmax_anal;
-      const int wmax = spin == 0 ? 4 : gp->npairs <= kAnalWidePairs ? 2 : 1;
+      const int wmax = spin == 0 ? 4 : anal_spin_wide(spin, gp->npairs, job.lmax) ? 2 : 1;
       if (ntrans >= 2 && wmax > 1 && tuner_on(flags, st))
         width = tuned_width(TuneKey{gp->hash, job.lmax, mmax, spin, type, ntrans, 1}, wmax,
                             ntmax_anal, passes, st);

@@ -1163,7 +1163,7 @@ void launch_legendre_anal(const JobDesc &job, const GeomPlan &gp, const CoefPlan
   auto shape = [&](auto n, auto f) {
     if (gp.npairs <= 128) f(n, c1, c4);
     else if (gp.npairs <= 256) f(n, c2, c4);
-    else if (gp.npairs <= kAnalWidePairs) f(n, c2, c8);
+    else if (anal_eight_warps(job.spin, gp.npairs, job.lmax)) f(n, c2, c8);
     else if (job.spin == 0) f(n, c4, c4);
     else f(n, c3, c4);
   };
@@ -1174,7 +1174,7 @@ void launch_legendre_anal(const JobDesc &job, const GeomPlan &gp, const CoefPlan
   } else if (nt == 1) {
     shape(c1, spins);
   } else {
-    SHT_REQUIRE(gp.npairs <= kAnalWidePairs, "analysis pass too wide");
+    SHT_REQUIRE(anal_spin_wide(job.spin, gp.npairs, job.lmax), "analysis pass too wide");
     if (gp.npairs <= 128) spins(c2, c1, c4);
     else if (gp.npairs <= 256) spins(c2, c2, c4);
     else spins(c2, c2, c8);
