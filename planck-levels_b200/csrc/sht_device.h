@@ -284,8 +284,8 @@ inline void allow_smem(K kernel, size_t bytes);
 // Launch with programmatic stream serialisation: the kernel may become resident
 // while its predecessor in the stream runs out (once all its CTAs have called
 // grid_release or ended), which hides the launch latency, 1 to 2 us a kernel
-// (Nside 64: a synthesis of three kernels takes 18.0 us, 23.4 without; an
-// analysis 20.6 and 26.6).  Every kernel launched like this calls grid_wait
+// (Nside 64: a synthesis of three kernels takes 19.6 us, 23.8 without; an
+// analysis 20.5 and 26.6).  Every kernel launched like this calls grid_wait
 // first of all: only past it are the writes of earlier kernels sure to be
 // visible, and a kernel that ended before its predecessor would release its own
 // successors too soon.  (Letting the ring kernels of one direction start on the
@@ -304,8 +304,8 @@ __device__ __forceinline__ void grid_release() {
 constexpr unsigned kSmCount = 148;   // of a B200
 // Only a grid of at most two CTAs per SM: the CTAs of the next kernel take
 // whatever room there is, and beside a larger grid they end up unevenly spread
-// (Gauss grid of 251 pairs, three spin-1 transforms both ways: 554 us with an
-// early release of every grid, 471 with this, 490 without overlap).
+// (Gauss grid of 251 pairs, three spin-1 transforms both ways: 559 us with an
+// early release of every grid, 477 with this, 495 without overlap).
 __device__ __forceinline__ void grid_release_small() {
   if (gridDim.x * gridDim.y <= 2 * kSmCount) grid_release();
 }

@@ -728,15 +728,16 @@ double wall_now() {
 // Pass-width tuner, the counterpart of the reference's nv oracle
 // (libsharp/sharp.c:890-965, which times its SIMD vector counts on first
 // use): the FP64 Legendre kernels take 1, 2 or 4 transforms per pass (spin s
-// and deriv1: 1 or 2; spin analysis only where anal_spin_wide); wider passes share one recurrence, narrower ones keep
-// more CTAs per SM, and which wins depends on the geometry, lmax and spin.
-// The first job of a shape with several transforms times each width once on
-// its own buffers (after one untimed run of it; one host synchronisation per
-// width) and the fastest is kept for the process, the default width unless
-// another is more than 3% faster.  Jobs whose flags carry a vector-count hint (the low bits,
-// SHARP_NVMAX, as the reference's nv), jobs on a stream that is being
-// captured, and all jobs when SHARP_B200_TUNE=0 keep the default widths;
-// SHARP_B200_TUNE_LOG prints each decision with its timings to stderr.
+// and deriv1: 1 or 2; spin analysis 2 only where anal_spin_wide); wider passes
+// share one recurrence, narrower ones keep more CTAs per SM, and which wins
+// depends on the geometry, lmax and spin.  The first job of a shape with several
+// transforms times each width once on its own buffers (after one untimed run of
+// it; one host synchronisation per width) and the fastest is kept for the
+// process, the default width unless another is more than 3% faster.  Jobs whose
+// flags carry a vector-count hint (the low bits, SHARP_NVMAX, as the reference's
+// nv), jobs on a stream that is being captured, and all jobs when
+// SHARP_B200_TUNE=0 keep the default widths; SHARP_B200_TUNE_LOG prints each
+// decision with its timings to stderr.
 // ---------------------------------------------------------------------------
 struct TuneKey {
   uint64_t geom;

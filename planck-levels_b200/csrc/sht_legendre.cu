@@ -1151,7 +1151,8 @@ void launch_legendre_anal(const JobDesc &job, const GeomPlan &gp, const CoefPlan
   // Shape (R rings per thread, W warps).  More rings per thread share a
   // reduction and more warps a tile; but one warp walks all l of its m alone, so
   // with few ring pairs that chain is the kernel's time and smaller R is faster.
-  // Measured with one transform, us, spin 0 / spin 2 (Nside: pairs):
+  // Measured with one transform, us, spin 0 / spin 2 (Nside: pairs; lmax = 2 Nside,
+  // see anal_eight_warps for other lmax):
   //   Nside 64 (128):    R1 W4 8.8 / 15.0   R2 W4 10.7 / 21.1   R4 W4 15.7 / 33.9
   //   Nside 128 (256):   R1 W4 29.0 / 53.6  R2 W4 19.9 / 38.5   R4 W4 28.5 / 61.7
   //   Nside 256 (512):   R2 W4 79.9 / 177   R2 W8 56.9 / 142    R4 W4 66.3 / 145

@@ -18,10 +18,10 @@
 //    launch (phase2ring_short_kernel / ring2phase_short_kernel);
 //  * odd rings: the two of a pair as one complex Bluestein convolution
 //    (phase2ring_odd_kernel / ring2phase_odd_kernel);
-//  * the rest (pairs of unequal odd lengths, single pixels, rings too long for
-//    shared memory, and the allocation-free synthesis, whose tables share a
-//    fixed scratch) in size classes (phase2ring_kernel / ring2phase_kernel),
-//    described here.
+//  * the rest (grids of even rings that smooth_ring_length names, pairs of unequal
+//    odd lengths, single pixels, rings too long for shared memory, and the
+//    allocation-free synthesis, whose tables share a fixed scratch) in size
+//    classes (phase2ring_kernel / ring2phase_kernel), described here.
 //
 // Size classes: one CTA owns one (ring pair, component) and runs both
 // hemispheres.  The FFT
@@ -1786,13 +1786,13 @@ ring2phase_short_kernel(const int *__restrict__ pairs, const int *__restrict__ m
 // length M >= 2n - 1.  The rounding error of either is relative to the larger of
 // the two, so the ring weights are applied where it can tell them apart: to the
 // pixels before the transform in the analysis (a ring of weight 0 contributes
-// zeros, whatever its pixels hold; the two rings' terms are added right after),
-// and to the pixels after it in the synthesis (the unweighted rings are of one
-// size, being the sum and difference of the same two partial sums).
-// One CTA of M/16 threads per pair and component.  A Gauss
-// grid of 251 pairs of 1001 = 7 11 13 pixels, 6 components of floats: 55 us
-// (synthesis) and 49 us (analysis), against 238 and 236 us with generic radix-7,
-// 11 and 13 passes in the size classes, one ring after the other.
+// zeros, whatever finite values its pixels hold; the two rings' terms are added
+// right after), and to the pixels after it in the synthesis (the unweighted rings
+// are of one size, being the sum and difference of the same two partial sums).
+// One CTA of M/16 threads per pair and component.  A Gauss grid of 251 pairs of
+// 1001 = 7 11 13 pixels, 6 components of floats: 59 us (synthesis) and 53 us
+// (analysis), against 242 and 241 us with generic radix-7, 11 and 13 passes in the
+// size classes, one ring after the other.
 // ---------------------------------------------------------------------------
 template <typename T, int M>
 __global__ void __launch_bounds__(M / 16, blue_min_blocks(M))
