@@ -113,10 +113,11 @@ inline int blue_ring_length(int nph, const FftDesc &d, bool all) {
 //       1536: 95 / 93  139 / 123  1800: 134 / 131  179 / 149
 //       2000: 144 / 140  203 / 166
 // With a factor 7 the convolution takes less (1120: 90 / 88, 97 / 88; 1400: 150
-// / 147, 125 / 111) and with larger ones half or a quarter.  In a geometry that
-// has at least as many other rings with that convolution they share its launch
-// (convolution_takes_smooth): HEALPix Nside 512, 3 components: 165 / 143 us with
-// its smooth rings in the size classes, 145 / 122 without.
+// / 147, 125 / 111) and with larger ones half or a quarter.  In a geometry with
+// other rings of that convolution they share its launch, which takes less than one
+// of their own (HEALPix, 3 components: Nside 512 145 / 122 us, 165 / 143 with the
+// smooth rings in the size classes; Nside 300, whose equatorial rings are smooth,
+// 104 / 93 and 113 / 100).
 inline bool smooth_ring_length(int nph) {
   if (nph <= 0 || (nph & 1)) return false;
   int N = nph / 2;
@@ -124,9 +125,6 @@ inline bool smooth_ring_length(int nph) {
   for (int p : {2, 3, 5})
     while (N % p == 0) N /= p;
   return N == 1;
-}
-inline bool convolution_takes_smooth(size_t smooth_pairs, size_t other_pairs) {
-  return other_pairs >= smooth_pairs;
 }
 // How the short-ring kernels run an even ring of complex length N, or kNone:
 // directly (N <= 32), by the passes of length L = N (64 .. 512, a power of two),

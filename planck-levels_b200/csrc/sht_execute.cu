@@ -346,13 +346,11 @@ GeomHost build_geom_host(const sharp_geom_info *g, int lmax, int mmax, int spin,
       }
     }
   }
-  if (!smooth.empty()) {
-    std::vector<int> &other = pb_lists[2048];   // the M of all of them
-    if (convolution_takes_smooth(smooth.size(), other.size())) {
-      for (int p : smooth) is_pw[p] = 2;
-      other.insert(other.end(), smooth.begin(), smooth.end());
-      std::sort(other.begin(), other.end());
-    }
+  const auto other = pb_lists.find(2048);   // the M of smooth rings
+  if (other != pb_lists.end()) {
+    for (int p : smooth) is_pw[p] = 2;
+    other->second.insert(other->second.end(), smooth.begin(), smooth.end());
+    std::sort(other->second.begin(), other->second.end());
   }
   for (auto &kv : pw_lists) {
     h.pw_N.push_back(kv.first);

@@ -1,7 +1,7 @@
 """Rings whose complex length has no factor above 5, between 513 and 1024: on a grid of
 such rings alone they take the direct passes (the convolution of the register
-kernels was up to 1.5 times as long there), among at least as many others, as on a
-HEALPix grid, the convolution.  Which kernels ran is read from a trace; the results
+kernels was up to 1.5 times as long there), among others, as on a HEALPix grid, the
+convolution.  Which kernels ran is read from a trace; the results
 are compared with the oracle at 1e-12, the FP64 bar of the parity tests."""
 import os
 import subprocess
@@ -66,9 +66,11 @@ def test_route_of_a_grid_of_one_length(nphi, want):
 
 
 @pytest.mark.gpu
-def test_route_on_healpix():
-    nside = 512   # 1080, 1200, 1280 ... pixels among the other polar rings
-    assert _kernels(sb.Geometry.healpix(nside), 64, 12 * nside**2) == CONVOLUTION
+@pytest.mark.parametrize("nside,lmax", [(512, 64), (300, 600), (512, 1100)])
+def test_route_on_healpix(nside, lmax):
+    # 1080, 1200, 1280 ... pixels among the other polar rings; equatorial rings of 1200
+    # or (folded) 2048 pixels, more than there are others
+    assert _kernels(sb.Geometry.healpix(nside), lmax, 12 * nside**2) == CONVOLUTION
 
 
 @pytest.mark.gpu
