@@ -286,7 +286,10 @@ inline void allow_smem(K kernel, size_t bytes);
 // analysis 20.5 and 26.6).  Every kernel launched like this calls grid_wait
 // first of all: only past it are the writes of earlier kernels sure to be
 // visible, and a kernel that ended before its predecessor would release its own
-// successors too soon.  (Letting the ring kernels of one direction start on the
+// successors too soon.  What an earlier kernel wrote comes through plain pointers:
+// a const __restrict__ one tells the compiler that the data stays as it is while
+// the kernel runs, which begins before the wait, so that it might be loaded early
+// or through the read-only path.  (Letting the ring kernels of one direction start on the
 // phase rows or maps before that, because the first of them had waited, was
 // worth 2.6% of the chi-square gradient at Nside 512 and 3.3% of three Jacobi
 // sweeps at Nside 1024, but rested on an ordering that the instruction does not

@@ -277,7 +277,7 @@ synth_spin0_kernel(const int2 *__restrict__ items, const int *__restrict__ count
                    const double *__restrict__ cth, const double *__restrict__ sth,
                    const int *__restrict__ nph_ring, const long long *__restrict__ moff,
                    const double *__restrict__ alpha, const double *__restrict__ mfac,
-                   const double2 *__restrict__ A, int ncA, int comp0, int lmax,
+                   const double2 *A, int ncA, int comp0, int lmax,
                    double2 *__restrict__ phase, int ncm, int pcomp0, int ms) {
   grid_wait();
   grid_release_small();
@@ -426,7 +426,7 @@ synth_spin_kernel(const int2 *__restrict__ items, const int *__restrict__ count,
                   const int *__restrict__ nph_ring, const long long *__restrict__ moff,
                   const double *__restrict__ ca, const double *__restrict__ cb,
                   const double *__restrict__ pre_v, const int *__restrict__ pre_e, int s,
-                  const double2 *__restrict__ A, int ncA, int comp0, int lmax,
+                  const double2 *A, int ncA, int comp0, int lmax,
                   double2 *__restrict__ phase, int ncm, int pcomp0, int ms) {
   grid_wait();
   grid_release_small();
@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(32 * W, anal_min_blocks(0, NT, R, W))
 anal_spin0_kernel(const int *__restrict__ count, const double *__restrict__ cth,
                   const double *__restrict__ sth, const int *__restrict__ nph_ring,
                   const long long *__restrict__ moff, const double *__restrict__ alpha,
-                  const double *__restrict__ mfac, const double2 *__restrict__ phase, int ncm,
+                  const double *__restrict__ mfac, const double2 *phase, int ncm,
                   int pcomp0, int lmax, int ms, double *__restrict__ Aout, int ncA,
                   int comp0) {
   grid_wait();
@@ -873,7 +873,7 @@ anal_spin_kernel(const int *__restrict__ count, const double *__restrict__ cth,
                  const double *__restrict__ sth, const int *__restrict__ nph_ring,
                  const long long *__restrict__ moff, const double *__restrict__ ca,
                  const double *__restrict__ cb, const double *__restrict__ pre_v,
-                 const int *__restrict__ pre_e, int s, const double2 *__restrict__ phase,
+                 const int *__restrict__ pre_e, int s, const double2 *phase,
                  int ncm, int pcomp0, int lmax, int ms, double *__restrict__ Aout, int ncA,
                  int comp0) {
   grid_wait();

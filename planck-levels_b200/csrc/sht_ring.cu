@@ -970,7 +970,7 @@ phase2ring_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const double *__restrict__ phi0, const double2 *__restrict__ shift, int sw,
                        const double *__restrict__ weight,
                        const int *__restrict__ fftidx, const FftDesc *__restrict__ fdesc,
-                       const double2 *__restrict__ twiddle, const double2 *__restrict__ phase,
+                       const double2 *__restrict__ twiddle, const double2 *phase,
                        int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
                        long long map_lo) {
   grid_wait();
@@ -1245,7 +1245,7 @@ phase2ring_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const FftDesc *__restrict__ fdesc, const double2 *__restrict__ twiddle,
                        const double2 *__restrict__ wpow2, int P,
                        const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
-                       const double2 *__restrict__ phase, int ncm, int mmax, int flags,
+                       const double2 *phase, int ncm, int mmax, int flags,
                        const __grid_constant__ PtrList maps, long long map_lo, int stage_row) {
   grid_wait();
   grid_release_small();
@@ -1536,7 +1536,7 @@ phase2ring_short_kernel(const int *__restrict__ pairs, const int *__restrict__ m
                         const FftDesc *__restrict__ fdesc, const double2 *__restrict__ twiddle,
                         const double2 *__restrict__ wpow2, int P,
                         const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
-                        const double2 *__restrict__ phase, int ncm, int mmax, int flags,
+                        const double2 *phase, int ncm, int mmax, int flags,
                         const __grid_constant__ PtrList maps, long long map_lo) {
   grid_wait();
   grid_release_small();
@@ -1803,7 +1803,7 @@ phase2ring_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mli
                       const double *__restrict__ weight, const int *__restrict__ fftidx,
                       const FftDesc *__restrict__ fdesc, const double2 *__restrict__ wpow2,
                       int P, const double2 *__restrict__ bhat,
-                      const double2 *__restrict__ chirp, const double2 *__restrict__ phase,
+                      const double2 *__restrict__ chirp, const double2 *phase,
                       int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
                       long long map_lo) {
   grid_wait();
@@ -2024,7 +2024,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 stage_alm_kernel(int lmax, int nalmptr, const long long *__restrict__ mvstart,
                  long long astride, bool packed, long long alm_lo,
-                 const long long *__restrict__ moff, const double *__restrict__ cfac,
+                 const long long *__restrict__ moff, const double *cfac,
                  const double *__restrict__ norm_l, bool use_norm, double norm_m0,
                  const __grid_constant__ PtrList alm, double2 *__restrict__ A, int ncA, int lgtl,
                  bool pm) {
@@ -2082,7 +2082,7 @@ scatter_alm_kernel(int lmax, int nalmptr, const long long *__restrict__ mvstart,
                    long long astride, bool packed, long long alm_lo,
                    const long long *__restrict__ moff, const double *__restrict__ cfac,
                    const double *__restrict__ norm_l, bool use_norm, double norm_m0, double sgn,
-                   bool add, const double *__restrict__ Aout, int ncA,
+                   bool add, const double *Aout, int ncA,
                    const __grid_constant__ PtrList alm, int lgtl) {
   grid_wait();
   grid_release_small();

@@ -59,3 +59,25 @@ def test_early_kernels_wait_before_anything_else():
         for call in re.finditer(r"grid_release\w*\(\)\s*;", text):
             assert re.search(r"grid_wait\(\)\s*;\s*$", text[:call.start()]), path
     assert bodies >= 10
+
+
+# pointer parameters of the kernels launched early to what an earlier kernel of the
+# stream wrote (the coefficients of the staging: by the allocation-free synthesis)
+WRITTEN_BEFORE = {"synth_spin0_kernel": "A", "synth_spin_kernel": "A", "anal_spin0_kernel": "phase",
+                  "anal_spin_kernel": "phase", "phase2ring_pow2_kernel": "phase",
+                  "phase2ring_blue_kernel": "phase", "phase2ring_short_kernel": "phase",
+                  "phase2ring_odd_kernel": "phase", "stage_alm_kernel": "cfac",
+                  "scatter_alm_kernel": "Aout"}
+
+
+def test_early_kernels_take_earlier_results_through_plain_pointers():
+    text = ""
+    for path in glob.glob(os.path.join(ROOT, "planck-levels_b200", "csrc", "*.cu")):
+        with open(path) as f:
+            text += re.sub(r"//[^\n]*", "", f.read())
+    early = re.findall(r"\n(\w+)\(([^{};]*)\)\s*\{\s*grid_wait\(\)", text)
+    assert len(early) >= 14
+    for name, params in early:
+        read = re.findall(r"const double2? \*(__restrict__ )?(A|Aout|phase|cfac)\b", params)
+        assert not [p for r, p in read if r and WRITTEN_BEFORE.get(name) == p], name
+    assert set(WRITTEN_BEFORE) <= {name for name, _ in early}
