@@ -205,6 +205,10 @@ struct GeomPlan {
   // e^{i m phi0} per ring as two slices (see shift_table_kernel), or null
   double2 *shift = nullptr;
   int shift_width = 0;
+  // kChainFlags flags of the ring kernels' chains (ChainLink), or null; the epoch
+  // of the last chain (changed under the lock of the plans)
+  unsigned long long *chain = nullptr;
+  mutable unsigned long long chain_epoch = 0;
   long long map_lo = 0, map_hi = 0;  // pixel index extent [lo, hi)
   bool map_covered = false;          // rings tile [lo,hi) exactly
   GeomPlan() = default;
@@ -284,16 +288,12 @@ inline void allow_smem(K kernel, size_t bytes);
 // grid_release or ended), which hides the launch latency, 1 to 2 us a kernel
 // (Nside 64: a synthesis of three kernels takes 19.6 us, 23.8 without; an
 // analysis 20.5 and 26.6).  Every kernel launched like this calls grid_wait
-// first of all: only past it are the writes of earlier kernels sure to be
-// visible, and a kernel that ended before its predecessor would release its own
-// successors too soon.  What an earlier kernel wrote comes through plain pointers:
-// a const __restrict__ one tells the compiler that the data stays as it is while
-// the kernel runs, which begins before the wait, so that it might be loaded early
-// or through the read-only path.  (Letting the ring kernels of one direction start on the
-// phase rows or maps before that, because the first of them had waited, was
-// worth 2.6% of the chi-square gradient at Nside 512 and 3.3% of three Jacobi
-// sweeps at Nside 1024, but rested on an ordering that the instruction does not
-// promise.)
+// first of all (or is one of a chain, see GridChain): only past it are the writes
+// of earlier kernels sure to be visible, and a kernel that ended before its
+// predecessor would release its own successors too soon.  What an earlier kernel
+// wrote comes through plain pointers: a const __restrict__ one tells the compiler
+// that the data stays as it is while the kernel runs, which begins before the
+// wait, so that it might be loaded early or through the read-only path.
 template <class... P, class... A>
 inline void launch_overlapped(void (*kernel)(P...), dim3 grid, int threads, size_t smem,
                               cudaStream_t st, A &&...args);
@@ -310,6 +310,62 @@ constexpr unsigned kSmCount = 148;   // of a B200
 __device__ __forceinline__ void grid_release_small() {
   if (gridDim.x * gridDim.y <= 2 * kSmCount) grid_release();
 }
+#endif
+
+// The register ring kernels of one direction read the same phase rows or maps and
+// write disjoint ones, so each may run while its predecessor's last CTAs do.  What
+// it reads was written before the first of them, which waits (grid_wait) and then
+// publishes the call's epoch in a flag of the plan by a release; a later one
+// acquires that epoch before it reads or writes anything, or, should the flag
+// not hold it yet, waits like every other kernel.  It ends only after its
+// predecessor has (grid_wait), so that what follows the last one finds all of
+// them done.  The first and the later ones let their successor start as soon as
+// all their CTAs have started, the last one as grid_release_small does.  Without a
+// flag (a single kernel, a captured stream, whose replays would find the epoch
+// of the one before, and the allocation-free synthesis) every kernel waits first.
+// T synthesis, Nside 450 / lmax 450: 102 us, 125 if every kernel waits; chi-square
+// gradient at Nside 512: 2420 and 2480 us; three Jacobi sweeps at Nside 1024: 11.68
+// and 12.06 ms.
+struct ChainLink {
+  unsigned long long *flag = nullptr;
+  unsigned long long epoch = 0;
+  bool first = true, last = true;
+};
+constexpr int kChainFlags = 64;   // calls of a plan in flight that have a flag of their own
+#ifdef __CUDACC__
+class GridChain {
+ public:
+  __device__ __forceinline__ explicit GridChain(const ChainLink &l) {
+    if (l.flag == nullptr || l.first) {
+      grid_wait();
+      if (l.flag != nullptr && (threadIdx.x | blockIdx.x | blockIdx.y) == 0)
+        asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(l.flag), "l"(l.epoch) : "memory");
+    } else {
+      // the barrier hands the acquire of thread 0 on to the others
+      waited_ = __syncthreads_or(threadIdx.x == 0 && !published(l));
+      if (waited_) grid_wait();
+      // for the bulk copies of phase rows, which thread 0 issues
+      if (threadIdx.x == 0) asm volatile("fence.proxy.async.global;" ::: "memory");
+    }
+    if (l.flag == nullptr || l.last) grid_release_small();
+    else grid_release();
+  }
+  __device__ __forceinline__ ~GridChain() {
+    if (!waited_) grid_wait();
+  }
+
+ private:
+  // a few tries: usually the epoch is there before the kernel starts
+  static __device__ __forceinline__ bool published(const ChainLink &l) {
+    for (int i = 0; i < 32; ++i) {
+      unsigned long long v;
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(l.flag) : "memory");
+      if (v == l.epoch) return true;
+    }
+    return false;
+  }
+  bool waited_ = true;
+};
 #endif
 
 // Kernel launchers (sht_legendre.cu)

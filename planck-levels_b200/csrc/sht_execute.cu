@@ -506,6 +506,8 @@ std::unique_ptr<GeomPlan> build_geom_plan(const sharp_geom_info *g, int lmax, in
   SHT_CUDA(cudaMalloc(&gp->shift, sizeof(double2) * std::max<size_t>(2 * size_t(h.npairs), 1) *
                                       gp->shift_width));
   launch_shift_table(*gp, st);
+  SHT_CUDA(cudaMalloc(&gp->chain, sizeof(unsigned long long) * kChainFlags));
+  SHT_CUDA(cudaMemsetAsync(gp->chain, 0, sizeof(unsigned long long) * kChainFlags, st));
   SHT_CUDA(cudaStreamSynchronize(st));
   return gp;
 }
@@ -1475,6 +1477,7 @@ GeomPlan::~GeomPlan() {
   dev_free(phi0); dev_free(weight); dev_free(ofs); dev_free(nph); dev_free(stride);
   dev_free(fft); dev_free(fdesc); dev_free(twiddle); dev_free(cls_pairs); dev_free(pw_pairs);
   dev_free(pb_pairs); dev_free(ps_pairs); dev_free(po_pairs); dev_free(shift);
+  dev_free(chain);
   dev_free(bhat); dev_free(wpow2); dev_free(chirp);
 }
 CoefPlan::~CoefPlan() {

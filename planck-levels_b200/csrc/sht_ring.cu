@@ -972,9 +972,8 @@ phase2ring_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const int *__restrict__ fftidx, const FftDesc *__restrict__ fdesc,
                        const double2 *__restrict__ twiddle, const double2 *phase,
                        int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
-                       long long map_lo) {
-  grid_wait();
-  grid_release_small();
+                       long long map_lo, const ChainLink link) {
+  const GridChain chain(link);
   extern __shared__ double2 smem[];
   __shared__ uint64_t row_full;
   double2 *buf = smem;
@@ -1074,9 +1073,8 @@ ring2phase_pow2_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const int *__restrict__ fftidx, const FftDesc *__restrict__ fdesc,
                        const double2 *__restrict__ twiddle, double2 *__restrict__ phase,
                        int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
-                       long long map_lo) {
-  grid_wait();
-  grid_release_small();
+                       long long map_lo, const ChainLink link) {
+  const GridChain chain(link);
   extern __shared__ double2 smem[];
   double2 *buf = smem;
   double2 *slo = smem + pw_entries(N);
@@ -1246,9 +1244,9 @@ phase2ring_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const double2 *__restrict__ wpow2, int P,
                        const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                        const double2 *phase, int ncm, int mmax, int flags,
-                       const __grid_constant__ PtrList maps, long long map_lo, int stage_row) {
-  grid_wait();
-  grid_release_small();
+                       const __grid_constant__ PtrList maps, long long map_lo, int stage_row,
+                       const ChainLink link) {
+  const GridChain chain(link);
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   __shared__ uint64_t row_full;
@@ -1357,9 +1355,9 @@ ring2phase_blue_kernel(const int *__restrict__ pairs, const int *__restrict__ ml
                        const double2 *__restrict__ wpow2, int P,
                        const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                        double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                       const __grid_constant__ PtrList maps, long long map_lo) {
-  grid_wait();
-  grid_release_small();
+                       const __grid_constant__ PtrList maps, long long map_lo,
+                       const ChainLink link) {
+  const GridChain chain(link);
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   double2 *buf = smem;
@@ -1537,9 +1535,9 @@ phase2ring_short_kernel(const int *__restrict__ pairs, const int *__restrict__ m
                         const double2 *__restrict__ wpow2, int P,
                         const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                         const double2 *phase, int ncm, int mmax, int flags,
-                        const __grid_constant__ PtrList maps, long long map_lo) {
-  grid_wait();
-  grid_release_small();
+                        const __grid_constant__ PtrList maps, long long map_lo,
+                        const ChainLink link) {
+  const GridChain chain(link);
   extern __shared__ double2 smem[];
   double2 *buf = smem, *slo = buf + kShortEntries, *shi = slo + kShiftLo;
   const int p = pairs[blockIdx.x >> 1], h = blockIdx.x & 1, c = blockIdx.y;
@@ -1661,9 +1659,9 @@ ring2phase_short_kernel(const int *__restrict__ pairs, const int *__restrict__ m
                         const double2 *__restrict__ wpow2, int P,
                         const double2 *__restrict__ bhat, const double2 *__restrict__ chirp,
                         double2 *__restrict__ phase, int ncm, int mmax, int flags,
-                        const __grid_constant__ PtrList maps, long long map_lo) {
-  grid_wait();
-  grid_release_small();
+                        const __grid_constant__ PtrList maps, long long map_lo,
+                        const ChainLink link) {
+  const GridChain chain(link);
   extern __shared__ double2 smem[];
   double2 *buf = smem, *slo = buf + kShortEntries, *shi = slo + kShiftLo;
   const int p = pairs[blockIdx.x >> 1], h = blockIdx.x & 1, c = blockIdx.y;
@@ -1805,9 +1803,8 @@ phase2ring_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mli
                       int P, const double2 *__restrict__ bhat,
                       const double2 *__restrict__ chirp, const double2 *phase,
                       int ncm, int mmax, int flags, const __grid_constant__ PtrList maps,
-                      long long map_lo) {
-  grid_wait();
-  grid_release_small();
+                      long long map_lo, const ChainLink link) {
+  const GridChain chain(link);
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   double2 *buf = smem;
@@ -1888,9 +1885,8 @@ ring2phase_odd_kernel(const int *__restrict__ pairs, const int *__restrict__ mli
                       int P, const double2 *__restrict__ bhat,
                       const double2 *__restrict__ chirp, double2 *__restrict__ phase, int ncm,
                       int mmax, int flags, const __grid_constant__ PtrList maps,
-                      long long map_lo) {
-  grid_wait();
-  grid_release_small();
+                      long long map_lo, const ChainLink link) {
+  const GridChain chain(link);
   constexpr int NT = M / 16;
   extern __shared__ double2 smem[];
   double2 *buf = smem;
@@ -2324,6 +2320,32 @@ void ring2phase_class(const JobDesc &job, const GeomPlan &gp, int cls, long long
 
 namespace {
 
+// Launches the register ring kernels of one direction (ChainLink).
+class RingStream {
+ public:
+  RingStream(const GeomPlan &gp, cudaStream_t st) : st_(st), left_(gp.ps_count > 0 ? 1 : 0) {
+    for (const auto *v : {&gp.pw_count, &gp.pb_count, &gp.po_count})
+      for (int n : *v) left_ += n > 0;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (left_ > 1 && gp.chain && cudaStreamIsCapturing(st, &cs) == cudaSuccess &&
+        cs == cudaStreamCaptureStatusNone) {
+      link_.epoch = ++gp.chain_epoch;
+      link_.flag = gp.chain + link_.epoch % kChainFlags;
+    }
+  }
+  template <class... P, class... A>
+  void launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, A &&...args) {
+    link_.last = --left_ == 0;
+    launch_overlapped(kernel, grid, threads, smem, st_, std::forward<A>(args)..., link_);
+    link_.first = false;
+  }
+
+ private:
+  cudaStream_t st_;
+  int left_;   // kernels to come
+  ChainLink link_;
+};
+
 size_t pow2_smem(int N, int mmax) {
   return sizeof(double2) * (size_t(pw_entries(N)) + kShiftLo + mmax / kShiftLo + 2);
 }
@@ -2331,11 +2353,11 @@ size_t pow2_smem(int N, int mmax) {
 template <typename T, int N>
 void phase2ring_pow2(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
                      const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
-                     cudaStream_t st) {
+                     RingStream &rs) {
   auto k = phase2ring_pow2_kernel<T, N>;
   const size_t smem = pow2_smem(N, job.mmax);
   allow_smem(k, smem);
-  launch_overlapped(k, dim3(2 * gp.pw_count[cls], nmapptr), N / 16, smem, st,
+  rs.launch(k, dim3(2 * gp.pw_count[cls], nmapptr), N / 16, smem,
       gp.pw_pairs + gp.pw_start[cls], gp.mlim, gp.nph, gp.ofs, gp.phi0, gp.shift,
       gp.shift_width, gp.weight, gp.fft,
       gp.fdesc, gp.twiddle, phase, ncm, job.mmax, job.flags,
@@ -2345,12 +2367,12 @@ void phase2ring_pow2(const JobDesc &job, const GeomPlan &gp, int cls, long long 
 template <typename T, int N>
 void ring2phase_pow2(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
                      const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
-                     cudaStream_t st) {
+                     RingStream &rs) {
   auto k = ring2phase_pow2_kernel<T, N>;
   // plus the twiddle slices of the unpacking
   const size_t smem = pow2_smem(N, job.mmax) + sizeof(double2) * (kTwLo + N / kTwLo + 1);
   allow_smem(k, smem);
-  launch_overlapped(k, dim3(2 * gp.pw_count[cls], nmapptr), N / 16, smem, st,
+  rs.launch(k, dim3(2 * gp.pw_count[cls], nmapptr), N / 16, smem,
       gp.pw_pairs + gp.pw_start[cls], gp.mlim, gp.nph, gp.ofs, gp.phi0, gp.shift,
       gp.shift_width, gp.weight, gp.fft,
       gp.fdesc, gp.twiddle, phase, ncm, job.mmax, job.flags,
@@ -2360,7 +2382,7 @@ void ring2phase_pow2(const JobDesc &job, const GeomPlan &gp, int cls, long long 
 template <typename T, int M>
 void phase2ring_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
                      const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
-                     cudaStream_t st) {
+                     RingStream &rs) {
   auto k = phase2ring_blue_kernel<T, M>;
   // the phase row is staged in shared memory where that keeps the CTAs per
   // SM (M = 8192: one CTA per SM either way) and fits
@@ -2369,7 +2391,7 @@ void phase2ring_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long 
   const int stage_row = (M == 8192 && with_row + 1024 <= 227 * 1024) ? 1 : 0;
   const size_t smem = stage_row ? with_row : base;
   allow_smem(k, smem);
-  launch_overlapped(k, dim3(2 * gp.pb_count[cls], nmapptr), M / 16, smem, st,
+  rs.launch(k, dim3(2 * gp.pb_count[cls], nmapptr), M / 16, smem,
       gp.pb_pairs + gp.pb_start[cls], gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.shift,
       gp.shift_width, gp.weight,
       gp.fft, gp.fdesc, gp.twiddle, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase, ncm, job.mmax,
@@ -2379,11 +2401,11 @@ void phase2ring_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long 
 template <typename T, int M>
 void ring2phase_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
                      const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
-                     cudaStream_t st) {
+                     RingStream &rs) {
   auto k = ring2phase_blue_kernel<T, M>;
   const size_t smem = pow2_smem(M, job.mmax);
   allow_smem(k, smem);
-  launch_overlapped(k, dim3(2 * gp.pb_count[cls], nmapptr), M / 16, smem, st,
+  rs.launch(k, dim3(2 * gp.pb_count[cls], nmapptr), M / 16, smem,
       gp.pb_pairs + gp.pb_start[cls], gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.shift,
       gp.shift_width, gp.weight,
       gp.fft, gp.fdesc, gp.twiddle, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase, ncm, job.mmax,
@@ -2392,13 +2414,13 @@ void ring2phase_blue(const JobDesc &job, const GeomPlan &gp, int cls, long long 
 
 template <typename T, bool SYNTH>
 void odd_rings(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo,
-               const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm, cudaStream_t st) {
+               const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm, RingStream &rs) {
   auto length = [&](auto len) {
     constexpr int M = decltype(len)::value;
     const size_t smem = sizeof(double2) * odd_ring_smem_entries(M, job.mmax);
     auto go = [&](auto kernel) {
       allow_smem(kernel, smem);
-      launch_overlapped(kernel, dim3(gp.po_count[cls], nmapptr), M / 16, smem, st,
+      rs.launch(kernel, dim3(gp.po_count[cls], nmapptr), M / 16, smem,
           gp.po_pairs + gp.po_start[cls], gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.shift,
           gp.shift_width, gp.weight, gp.fft, gp.fdesc, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase,
           ncm, job.mmax, job.flags, maps_dev, map_lo);
@@ -2418,11 +2440,11 @@ void odd_rings(const JobDesc &job, const GeomPlan &gp, int cls, long long map_lo
 
 template <typename T, bool SYNTH>
 void short_rings(const JobDesc &job, const GeomPlan &gp, long long map_lo, const PtrList &maps_dev,
-                 int nmapptr, double2 *phase, int ncm, cudaStream_t st) {
+                 int nmapptr, double2 *phase, int ncm, RingStream &rs) {
   if (gp.ps_count == 0) return;
   const size_t smem = short_smem(job.mmax);
   auto go = [&](auto kernel) {
-    launch_overlapped(kernel, dim3(2 * gp.ps_count, nmapptr), 32, smem, st,
+    rs.launch(kernel, dim3(2 * gp.ps_count, nmapptr), 32, smem,
         gp.ps_pairs, gp.mlim, gp.nph, gp.ofs, gp.stride, gp.phi0, gp.shift, gp.shift_width,
         gp.weight, gp.fft, gp.fdesc, gp.twiddle, gp.wpow2, gp.P, gp.bhat, gp.chirp, phase, ncm,
         job.mmax, job.flags, maps_dev, map_lo);
@@ -2434,84 +2456,84 @@ void short_rings(const JobDesc &job, const GeomPlan &gp, long long map_lo, const
 template <typename T>
 void phase2ring_pow2_classes(const JobDesc &job, const GeomPlan &gp, long long map_lo,
                              const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
-                             cudaStream_t st) {
+                             RingStream &rs) {
   for (int c = int(gp.pw_N.size()) - 1; c >= 0; --c) {
     if (gp.pw_count[c] == 0) continue;
     switch (gp.pw_N[c]) {
       case 1024:
-        phase2ring_pow2<T, 1024>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        phase2ring_pow2<T, 1024>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs);
         break;
       case 2048:
-        phase2ring_pow2<T, 2048>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        phase2ring_pow2<T, 2048>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs);
         break;
       case 4096:
-        phase2ring_pow2<T, 4096>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        phase2ring_pow2<T, 4096>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs);
         break;
       default:
-        phase2ring_pow2<T, 8192>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        phase2ring_pow2<T, 8192>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs);
     }
   }
   for (int c = int(gp.pb_M.size()) - 1; c >= 0; --c) {
     if (gp.pb_count[c] == 0) continue;
     switch (gp.pb_M[c]) {
       case 1024:
-        phase2ring_blue<T, 1024>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        phase2ring_blue<T, 1024>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs);
         break;
       case 2048:
-        phase2ring_blue<T, 2048>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        phase2ring_blue<T, 2048>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs);
         break;
       case 4096:
-        phase2ring_blue<T, 4096>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        phase2ring_blue<T, 4096>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs);
         break;
       default:
-        phase2ring_blue<T, 8192>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, st);
+        phase2ring_blue<T, 8192>(job, gp, c, map_lo, phase, ncm, maps_dev, nmapptr, rs);
     }
   }
   for (int c = int(gp.po_M.size()) - 1; c >= 0; --c)
     odd_rings<T, true>(job, gp, c, map_lo, maps_dev, nmapptr, const_cast<double2 *>(phase), ncm,
-                       st);
-  short_rings<T, true>(job, gp, map_lo, maps_dev, nmapptr, const_cast<double2 *>(phase), ncm, st);
+                       rs);
+  short_rings<T, true>(job, gp, map_lo, maps_dev, nmapptr, const_cast<double2 *>(phase), ncm, rs);
 }
 
 template <typename T>
 void ring2phase_pow2_classes(const JobDesc &job, const GeomPlan &gp, long long map_lo,
                              const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
-                             cudaStream_t st) {
+                             RingStream &rs) {
   for (int c = int(gp.pw_N.size()) - 1; c >= 0; --c) {
     if (gp.pw_count[c] == 0) continue;
     switch (gp.pw_N[c]) {
       case 1024:
-        ring2phase_pow2<T, 1024>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        ring2phase_pow2<T, 1024>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs);
         break;
       case 2048:
-        ring2phase_pow2<T, 2048>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        ring2phase_pow2<T, 2048>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs);
         break;
       case 4096:
-        ring2phase_pow2<T, 4096>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        ring2phase_pow2<T, 4096>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs);
         break;
       default:
-        ring2phase_pow2<T, 8192>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        ring2phase_pow2<T, 8192>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs);
     }
   }
   for (int c = int(gp.pb_M.size()) - 1; c >= 0; --c) {
     if (gp.pb_count[c] == 0) continue;
     switch (gp.pb_M[c]) {
       case 1024:
-        ring2phase_blue<T, 1024>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        ring2phase_blue<T, 1024>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs);
         break;
       case 2048:
-        ring2phase_blue<T, 2048>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        ring2phase_blue<T, 2048>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs);
         break;
       case 4096:
-        ring2phase_blue<T, 4096>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        ring2phase_blue<T, 4096>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs);
         break;
       default:
-        ring2phase_blue<T, 8192>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
+        ring2phase_blue<T, 8192>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs);
     }
   }
   for (int c = int(gp.po_M.size()) - 1; c >= 0; --c)
-    odd_rings<T, false>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, st);
-  short_rings<T, false>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, st);
+    odd_rings<T, false>(job, gp, c, map_lo, maps_dev, nmapptr, phase, ncm, rs);
+  short_rings<T, false>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, rs);
 }
 
 }  // namespace
@@ -2520,10 +2542,11 @@ void launch_phase2ring(const JobDesc &job, const GeomPlan &gp, long long map_lo,
                        const double2 *phase, int ncm, const PtrList &maps_dev, int nmapptr,
                        cudaStream_t st) {
   ProfScope ps("ring_synth", st);
+  RingStream rs(gp, st);
   if (job.dp)
-    phase2ring_pow2_classes<double>(job, gp, map_lo, phase, ncm, maps_dev, nmapptr, st);
+    phase2ring_pow2_classes<double>(job, gp, map_lo, phase, ncm, maps_dev, nmapptr, rs);
   else
-    phase2ring_pow2_classes<float>(job, gp, map_lo, phase, ncm, maps_dev, nmapptr, st);
+    phase2ring_pow2_classes<float>(job, gp, map_lo, phase, ncm, maps_dev, nmapptr, rs);
   for (int cls = 0; cls < int(gp.cls_N.size()); ++cls) {
     if (gp.cls_count[cls] == 0) continue;
     if (job.dp)
@@ -2537,10 +2560,11 @@ void launch_ring2phase(const JobDesc &job, const GeomPlan &gp, long long map_lo,
                        const PtrList &maps_dev, int nmapptr, double2 *phase, int ncm,
                        cudaStream_t st) {
   ProfScope ps("ring_anal", st);
+  RingStream rs(gp, st);
   if (job.dp)
-    ring2phase_pow2_classes<double>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, st);
+    ring2phase_pow2_classes<double>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, rs);
   else
-    ring2phase_pow2_classes<float>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, st);
+    ring2phase_pow2_classes<float>(job, gp, map_lo, maps_dev, nmapptr, phase, ncm, rs);
   for (int cls = 0; cls < int(gp.cls_N.size()); ++cls) {
     if (gp.cls_count[cls] == 0) continue;
     if (job.dp)

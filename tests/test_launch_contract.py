@@ -48,17 +48,37 @@ def test_mismatched_arguments_do_not_compile(args, tmp_path):
     assert not _compiles(args, tmp_path)
 
 
+# what a kernel that may start early does first: wait for its predecessor, or, if it is
+# one of a chain, what GridChain does
+START = r"(?:grid_wait\(\)|const GridChain chain\(link\))\s*;"
+
+
 def test_early_kernels_wait_before_anything_else():
     bodies = 0
     for path in glob.glob(os.path.join(ROOT, "planck-levels_b200", "csrc", "*.cu")):
         with open(path) as f:
             text = re.sub(r"//[^\n]*", "", f.read())
-        for call in re.finditer(r"grid_wait\(\)\s*;", text):
+        for call in re.finditer(START, text):
             assert re.search(r"\)\s*\{\s*$", text[:call.start()]), (path, text[call.start() - 80:call.end()])
             bodies += 1
         for call in re.finditer(r"grid_release\w*\(\)\s*;", text):
             assert re.search(r"grid_wait\(\)\s*;\s*$", text[:call.start()]), path
-    assert bodies >= 10
+    assert bodies >= 14
+
+
+def test_kernels_of_a_chain_acquire_or_wait_and_end_after_their_predecessor():
+    with open(os.path.join(ROOT, "planck-levels_b200", "csrc", "sht_device.h")) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    chain = re.sub(r"\s+", " ", text[text.index("class GridChain"):])
+    chain = chain[:chain.index("bool waited_ = true;")]
+    first, later = chain[chain.index("{", 20):chain.index("~GridChain")].split("} else {")
+    assert first.index("grid_wait();") < first.index("st.release.gpu")
+    assert "if (l.flag == nullptr || l.first)" in first
+    steps = ["waited_ = __syncthreads_or(threadIdx.x == 0 && !published(l));",
+             "if (waited_) grid_wait();", "fence.proxy.async.global", "grid_release"]
+    assert [later.index(x) for x in steps] == sorted(later.index(x) for x in steps)
+    assert "~GridChain() { if (!waited_) grid_wait(); }" in chain
+    assert "ld.acquire.gpu" in chain
 
 
 # pointer parameters of the kernels launched early to what an earlier kernel of the
@@ -75,7 +95,7 @@ def test_early_kernels_take_earlier_results_through_plain_pointers():
     for path in glob.glob(os.path.join(ROOT, "planck-levels_b200", "csrc", "*.cu")):
         with open(path) as f:
             text += re.sub(r"//[^\n]*", "", f.read())
-    early = re.findall(r"\n(\w+)\(([^{};]*)\)\s*\{\s*grid_wait\(\)", text)
+    early = re.findall(r"\n(\w+)\(([^{};]*)\)\s*\{\s*" + START, text)
     assert len(early) >= 14
     for name, params in early:
         read = re.findall(r"const double2? \*(__restrict__ )?(A|Aout|phase|cfac)\b", params)
